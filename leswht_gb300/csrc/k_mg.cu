@@ -26,8 +26,7 @@
 // Tables (pmat :55-94, mwavenumber :97-113, coefmg :643-798, the LU factors
 // of poisinit :18-52) are built on the host in the reference's arithmetic
 // order and uploaded once.
-#include "k_fft.cuh"
-#include <cooperative_groups.h>
+#include "k_mgl.cuh"
 #include <new>
 #include <math.h>
 #include <stdlib.h>
@@ -45,7 +44,7 @@ namespace lg {
 // push out of L1
 constexpr int kMgThreads = 256;
 constexpr int kMC = 8;            // rows per lane: y lines of up to 32 * kMC = 256 cells
-constexpr int kMaxLev = 20;
+constexpr int kMaxLev = kMgMaxLev;
 
 int mg_cluster_cap();
 
@@ -87,6 +86,14 @@ struct MgTables {
     MgSet<float> f;             // their FP32 copies (mixed form)
     long long *iters;           // per mode, last solve
     long long pc_plane, gg_plane;
+    // the cycles with the modes resident in their clusters' shared memory
+    // (k_mgl.cuh), used wherever a mode fits
+    int resident, prd;
+    MgLineArgs *dargs;          // device copies: one per substep, one for the autotuner's timing
+    double *ltab_d, *llc_d, *lact, *lasl, *lanl;
+    float *ltab_f, *llc_f;
+    size_t smem, lbt_size;      // a block's dynamic shared memory; lbt's elements
+    double *lbt;                // right-hand sides of modes whose b does not fit beside the rest
 };
 
 struct MgArgs {
@@ -1172,6 +1179,60 @@ __global__ void k_mg_begin(DScal *S, int slot, int nfft, int nmodes, double fac)
     S->mg_test = nfft == 1 ? S->test1 : S->test1 / (double)nmodes * (double)nfft * fac;
 }
 
+// ------------------------------------------- tables of the resident cycles
+// Half a warp per line of a mode: the solve table of k_mgl.cuh from the LU
+// factors (bet, gam, i fastest), formed in FP64.
+template <int R, class T>
+__global__ void k_mgl_tables(const double *as, const double *bet, const double *gam, int nld, int n2m, long long nlines, T *tab) {
+    const int lane = threadIdx.x & 15;
+    constexpr int W = 16 / (int)sizeof(T);
+    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4; w < nlines;
+         w += ((long long)gridDim.x * blockDim.x) >> 4) {
+        const unsigned half = 0xffffu << (threadIdx.x & 16);
+        const long long kv = w / nld, i = w % nld;
+        const size_t cb = (size_t)nld * n2m * kv + i;
+        T *to = tab + (size_t)w * mgl_tab_len<R, T>();
+        auto put = [&](int e, double v) { to[(e / W) * (16 * W) + lane * W + e % W] = (T)v; };
+        double P = 1.0, G = 1.0;
+        for (int q = 0; q < R; q++) {
+            const int j = lane * R + q, jb = lane * R + R - 1 - q;      // 0-based rows
+            const double b = j < n2m ? bet[cb + (size_t)nld * j] : 0.0;
+            const double p = j < n2m ? -as[j + 1] * b : 0.0;
+            const double g = jb + 1 < n2m ? -gam[cb + (size_t)nld * (jb + 1)] : 0.0;
+            P *= p;
+            G *= g;
+            put(q, b);
+            put(R + q, p);
+            put(2 * R + R - 1 - q, g);
+            if (mgl_cum<R>()) {
+                put(3 * R + 8 + q, P);
+                put(4 * R + 8 + R - 1 - q, G);
+            }
+        }
+        for (int s = 0; s < 4; s++) {
+            const int d = 1 << s;
+            put(3 * R + s, lane >= d ? P : 0.0);
+            put(3 * R + 4 + s, lane + d < 16 ? G : 0.0);
+            const double Po = __shfl_up_sync(half, P, d, 16), Go = __shfl_down_sync(half, G, d, 16);
+            if (lane >= d) P *= Po;
+            if (lane + d < 16) G *= Go;
+        }
+    }
+}
+
+// the top lines' diagonal, rows in solve order
+template <int R>
+__global__ void k_mgl_diag(const double *ac, int nl, int nld, int n2m, int nmodes, double *act) {
+    constexpr int LS = R * 16;
+    const long long n = (long long)nmodes * nl * LS;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        const int j = (int)(t % LS);
+        const long long l = t / LS;
+        act[l * LS + mgl_row_at<R>(j % R, j / R)] =
+            j < n2m ? ac[(size_t)nld * n2m * (l / nl) + (size_t)nld * j + l % nl] : 0.0;
+    }
+}
+
 // ---------------------------------------------------------------- host side
 // The semi-coarsened axis of a solve, in the reference's Fortran indexing:
 // x for poiss_z_ft, z for poiss_x_ft.
@@ -1336,6 +1397,75 @@ static int set_up_tables(lesgpu_case *c, MgTables &T) {
         if (cudaMalloc((void **)&dst, sizeof(T0) * v.size()) != cudaSuccess) { ok = false; return; }
         cudaMemcpy(dst, v.data(), sizeof(T0) * v.size(), cudaMemcpyHostToDevice);
     };
+    if (T.resident) {
+        // line coefficients (k_mgl.cuh): aw, ae; the coarse line's source
+        // weights (cor1, cor2 on the two top lines, -cor1 aw and -cor1 ae on
+        // the even neighbours of the finer odd line below); the weights of
+        // the three coarse lines a prolongation puts into an odd line's
+        // right-hand side (the last coarse line's coi2 only in x_ft)
+        std::vector<double> lcv((size_t)n1md * kLcN, 0.0);
+        for (int ilev = nlev; ilev >= 0; ilev--) {
+            const int ibg = iimg[ilev][0], nln = iimg[ilev][2];
+            for (int l = 0; l < nln; l++) {
+                double *q = &lcv[(size_t)(ibg - 1 + l) * kLcN];
+                const int i = ibg + l;
+                q[0] = aw[i];
+                q[1] = ae[i];
+                if (ilev < nlev) {
+                    const int f = iimg[ilev + 1][0] + 2 * l;
+                    q[2] = ilev == nlev - 1 ? cor1[i] : -cor1[i] * aw[f];
+                    q[3] = ilev == nlev - 1 ? cor2[i] : -cor1[i] * ae[f];
+                }
+                if (ilev >= 1 && (l & 1) == 0) {
+                    const int cb = iimg[ilev - 1][0], cn = iimg[ilev - 1][2], cc = l / 2;
+                    auto w2 = [&](int c0) { return (c0 < cn - 1 || xft) ? coi2[cb + c0] : 0.0; };
+                    const int cm = cc > 0 ? cc - 1 : A.prdic ? cn - 1 : -1;
+                    q[4] = cm >= 0 ? -aw[i] * coi1[cb + cm] : 0.0;
+                    q[5] = -((cm >= 0 ? aw[i] * w2(cm) : 0.0) + ae[i] * coi1[cb + cc]);
+                    q[6] = -ae[i] * w2(cc);
+                }
+            }
+        }
+        up(T.llc_d, lcv);
+        if (T.mixed) {
+            std::vector<float> h(lcv.begin(), lcv.end());
+            up(T.llc_f, h);
+        }
+        double *das = nullptr, *dac = nullptr, *dbet = nullptr, *dgam = nullptr;
+        up(das, as); up(dac, ac); up(dbet, bet); up(dgam, gam);
+        const long long nlines = (long long)n1md * nmodes;
+        auto build = [&](auto m) {
+            constexpr int R = decltype(m)::value, ls = 16 * R;
+            std::vector<double> asl(ls, 0.0), anl(ls, 0.0);
+            for (int j = 0; j < n2m; j++) {
+                asl[mgl_row_at<R>(j % R, j / R)] = j > 0 ? as[j + 1] : 0.0;
+                anl[mgl_row_at<R>(j % R, j / R)] = j + 1 < n2m ? an[j + 1] : 0.0;
+            }
+            up(T.lasl, asl); up(T.lanl, anl);
+            if ((T.mixed ? cudaMalloc(&T.ltab_f, sizeof(float) * nlines * mgl_tab_len<R, float>())
+                         : cudaMalloc(&T.ltab_d, sizeof(double) * nlines * mgl_tab_len<R, double>())) != cudaSuccess ||
+                cudaMalloc(&T.lact, sizeof(double) * (size_t)nmodes * n1m * ls) != cudaSuccess)
+                ok = false;
+            if (!ok) return;
+            if (T.mixed) k_mgl_tables<R, float><<<blocks_for(nlines * 16), kThreads>>>(das, dbet, dgam, n1md, n2m, nlines, T.ltab_f);
+            else k_mgl_tables<R, double><<<blocks_for(nlines * 16), kThreads>>>(das, dbet, dgam, n1md, n2m, nlines, T.ltab_d);
+            k_mgl_diag<R><<<blocks_for((long long)nmodes * n1m * ls), kThreads>>>(dac, n1m, n1md, n2m, nmodes, T.lact);
+        };
+        switch (mgl_r(n2m)) {
+        case 2: build(std::integral_constant<int, 2>{}); break;
+        case 3: build(std::integral_constant<int, 3>{}); break;
+        case 4: build(std::integral_constant<int, 4>{}); break;
+        case 6: build(std::integral_constant<int, 6>{}); break;
+        case 8: build(std::integral_constant<int, 8>{}); break;
+        case 12: build(std::integral_constant<int, 12>{}); break;
+        default: build(std::integral_constant<int, 16>{}); break;
+        }
+        if (ok) {
+            if (cudaDeviceSynchronize() != cudaSuccess) ok = false;
+        }
+        cudaFree(das); cudaFree(dac); cudaFree(dbet); cudaFree(dgam);
+        return ok ? 0 : LESGPU_ERR_OOM;
+    }
     up(T.d.aw, aw); up(T.d.ae, ae); up(T.d.as, as); up(T.d.an, an);
     up(T.d.coi1, coi1); up(T.d.coi2, coi2); up(T.d.cor1, cor1); up(T.d.cor2, cor2);
     up(T.ipm, ipm); up(T.imm, imm); up(T.d.ac, ac); up(T.d.bet, bet); up(T.d.gam, gam);
@@ -1360,6 +1490,50 @@ static bool cs_splits(const MgTables &T, int cs) {
     return true;
 }
 
+// How a cluster of cs blocks holds a mode (k_mgl.cuh): the pairs of lines of
+// every level per block, and the dynamic shared memory of a block; false if
+// it does not fit.  The levels of at most kMglSolo lines stay on block 0:
+// spreading one more level adds two cluster barriers per direction and takes
+// line solves off block 0.  Measured (us a solve): mixed 128x96 with 16 blocks
+// 754 at 16 lines, 770 at 8; FP64 64x48, whose solves are three times as long,
+// 1428 at 16, 1352 at 8.
+constexpr size_t kMglSmem = 222 * 1024;
+constexpr int kMglSoloMixed = 16, kMglSoloFp64 = 8;
+constexpr int kMglTuneCycles = 12;
+static bool mgl_plan(const MgTables &T, int n2m, int cs, MgLineArgs &a, size_t &smem) {
+    const int ls = 32 * mgl_r(n2m);
+    const size_t v = T.mixed ? sizeof(float) : sizeof(double);
+    for (int solo = T.mixed ? kMglSoloMixed : kMglSoloFp64; solo >= 1; solo >>= 1) {
+        int lines = 0;
+        for (int l = T.nlev; l >= 0; l--) {
+            MgLevel &L = a.lev[l];
+            L.n = T.nl >> (T.nlev - l);
+            L.np = (L.n + 1) / 2;
+            L.solo = cs == 1 || l == 0 || (l < T.nlev && L.n <= solo);
+            L.pp = L.solo ? L.np : (L.np + cs - 1) / cs;
+            L.inv = L.pp > 1 ? 0xFFFFFFFFu / (unsigned)L.pp + 1u : 0u;
+            L.off = lines;
+            lines += 2 * L.pp;
+        }
+        // levels run from the top down to block 0's: below a level of its own, none is spread
+        for (int l = 1; l < T.nlev; l++)
+            if (a.lev[l].solo && !a.lev[l - 1].solo) return false;
+        a.lines = lines;
+        a.top2 = 2 * a.lev[T.nlev].pp;
+        // tasks (mgl_schedule): the top's three halves and the pinned mode's
+        // shifts, four halves of a level, level 0's source and three halves
+        a.ndesc = 4 * a.lev[T.nlev].pp + a.lev[0].n + 3 * a.lev[0].pp;
+        for (int l = 1; l < T.nlev; l++) a.ndesc += 4 * a.lev[l].pp;
+        for (a.bshared = 1; a.bshared >= 0; a.bshared--) {
+            smem = (size_t)a.top2 * ls * sizeof(double) * (1 + a.bshared) + ls * sizeof(double) + mgl_fixed_bytes(ls / 32, T.mixed != 0) +
+                   a.ndesc * (T.mixed ? mgl_task_bytes<float>() : mgl_task_bytes<double>()) + ((size_t)lines + a.lev[0].n) * ls * v;
+            if (smem <= kMglSmem) return true;
+        }
+        if (cs == 1) return false;
+    }
+    return false;
+}
+
 static void cluster_cfg(cudaLaunchConfig_t &lc, cudaLaunchAttribute (&at)[1], int nmodes, int cs) {
     lc = {};
     lc.gridDim = dim3(nmodes * cs);
@@ -1368,6 +1542,121 @@ static void cluster_cfg(cudaLaunchConfig_t &lc, cudaLaunchAttribute (&at)[1], in
     at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     lc.attrs = at;
     lc.numAttrs = 1;
+}
+
+static MglKernel mgl_kernel(const MgTables &T, int n2m) {
+    return T.mixed ? mgl_kernel_mixed(mgl_r(n2m)) : mgl_kernel_fp64(mgl_r(n2m));
+}
+
+static void mgl_cfg(const MgTables &T, cudaLaunchConfig_t &lc, cudaLaunchAttribute (&at)[1], int nmodes, int cs, size_t smem) {
+    cluster_cfg(lc, at, nmodes, cs);
+    lc.blockDim = dim3(kMglThreads);
+    lc.dynamicSmemBytes = smem;
+}
+
+// clusters of cs blocks the device holds at once; 0 if a mode does not fit one
+static int mgl_active(const lesgpu_case *c, int cs) {
+    const MgTables &T = *c->pois.mg;
+    MgLineArgs a;
+    size_t sm;
+    if (!mgl_plan(T, c->kp.g.n2m, cs, a, sm)) return 0;
+    cudaLaunchConfig_t lc;
+    cudaLaunchAttribute at[1];
+    mgl_cfg(T, lc, at, T.nmodes, cs, sm);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, mgl_kernel(T, c->kp.g.n2m), &lc) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return n;
+}
+
+static bool mgl_args(const lesgpu_case *c, int cs, int slot, bool timing, MgLineArgs &a, size_t &smem) {
+    const lesgpu_config &cf = c->cfg;
+    const MgTables &T = *c->pois.mg;
+    memset(&a, 0, sizeof(a));
+    a.nl = T.nl; a.n2m = c->kp.g.n2m; a.nld = T.nld; a.nlev = T.nlev; a.nbli = (int)cf.nbli;
+    a.mgitr = timing ? kMglTuneCycles : (int)cf.mgitr;
+    a.xft = T.xft; a.prd = T.prd; a.cs = cs;
+    a.tab_d = T.ltab_d; a.lc_d = T.llc_d; a.act = T.lact; a.asl = T.lasl; a.anl = T.lanl;
+    a.tab_f = T.ltab_f; a.lc_f = T.llc_f;
+    a.ccap = c->pois.ccap; a.bt = T.lbt;
+    a.iters = T.iters; a.S = c->S; a.slot = slot; a.timing = timing;
+    if (!mgl_plan(T, a.n2m, cs, a, smem)) return false;
+    for (int l = 0; l <= T.nlev; l++) a.lev[l].ibg = T.iimg[l][0];
+    return true;
+}
+
+// The device copies of the arguments for clusters of cs blocks: what a graph
+// captured afterwards reads.  Ordered before the case's work by the wait.
+static int mgl_set_cluster(lesgpu_case *c, int cs) {
+    MgTables *T = c->pois.mg;
+    MgLineArgs a[4];
+    size_t sm = 0;
+    for (int q = 0; q < 4; q++)
+        if (!mgl_args(c, cs, q < 3 ? q : 0, q == 3, a[q], sm)) return LESGPU_ERR_CONFIG;
+    const size_t nb = a[0].bshared ? 0 : (size_t)T->nmodes * cs * a[0].top2 * 32 * mgl_r(c->kp.g.n2m);
+    if (nb > T->lbt_size) {
+        cudaStreamSynchronize(c->stream);
+        cudaFree(T->lbt);
+        T->lbt = nullptr;
+        T->lbt_size = 0;
+        if (cudaMalloc(&T->lbt, nb * sizeof(double)) != cudaSuccess) return LESGPU_ERR_OOM;
+        T->lbt_size = nb;
+    }
+    for (int q = 0; q < 4; q++) a[q].bt = T->lbt;
+    T->cs = cs;
+    T->smem = sm;
+    if (cudaMemcpyAsync(T->dargs, a, sizeof(a), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess)
+        return LESGPU_ERR_CUDA;
+    return 0;
+}
+
+// slot 0..2: a substep's solve; 3: the timing run
+static void mgl_launch(lesgpu_case *c, int slot) {
+    const MgTables &T = *c->pois.mg;
+    cudaLaunchConfig_t lc;
+    cudaLaunchAttribute at[1];
+    mgl_cfg(T, lc, at, T.nmodes, T.cs, T.smem);
+    lc.stream = c->stream;
+    cudaLaunchKernelEx(&lc, mgl_kernel(T, c->kp.g.n2m), (const MgLineArgs *)T.dargs + slot, T.nmodes);
+}
+
+static int mgl_init(lesgpu_case *c) {
+    const DGrid &g = c->kp.g;
+    DPois &P = c->pois;
+    MgTables *T = P.mg;
+    const size_t nm = (size_t)T->nmodes;
+    if (cudaMalloc(&T->iters, sizeof(long long) * nm) != cudaSuccess ||
+        cudaMalloc(&T->dargs, sizeof(MgLineArgs) * 4) != cudaSuccess ||
+        cudaMalloc(&P.ccap, sizeof(double2) * (size_t)T->nl * g.n2m * nm) != cudaSuccess)
+        return LESGPU_ERR_OOM;
+    cudaMemset(T->iters, 0, sizeof(long long) * nm);
+    if (T->xft) {
+        if (cudaFuncSetAttribute(k_fft_xr_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kFftSmemMax) != cudaSuccess ||
+            cudaFuncSetAttribute(k_fft_xr_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, kFftSmemMax) != cudaSuccess)
+            return LESGPU_ERR_CUDA;
+    } else {
+        if (fft_smem64(kFftSmemMax)) return LESGPU_ERR_CUDA;
+    }
+    const MglKernel k = mgl_kernel(*T, g.n2m);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMglSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        return LESGPU_ERR_CUDA;
+    int cap = mg_cluster_cap();
+    const char *env = getenv("LESGPU_MG_CLUSTER_MAX");
+    if (env && atoi(env) >= 1) cap = atoi(env);
+    T->cap = cap;
+    // until the autotuner times them: fewest waves per block of a mode, the
+    // smaller cluster among equals; above the cap only if no smaller one holds a mode
+    int pick = 0;
+    double best = 1e300;
+    for (int cs = 1; cs <= 16; cs <<= 1) {
+        const int n = mgl_active(c, cs);
+        if (n < 1 || (cap >= 1 && cs > cap && pick)) continue;
+        const double cost = (double)((T->nmodes + n - 1) / n) / cs;
+        if (cost < best - 1e-12) { best = cost; pick = cs; }
+    }
+    if (!pick) return LESGPU_ERR_CUDA;
+    return mgl_set_cluster(c, pick);
 }
 
 int mg2d_init(lesgpu_case *c) {
@@ -1395,8 +1684,17 @@ int mg2d_init(lesgpu_case *c) {
     // correction (LESGPU_MG_FP64=1 keeps them in FP64)
     const char *mg64 = getenv("LESGPU_MG_FP64");
     T->mixed = cf.precision == LESGPU_PREC_MIXED && !(mg64 && mg64[0] == '1');
+    T->prd = (xft ? cf.zprdic : cf.xprdic) == 1;
+    {   // resident cycles wherever some cluster holds a mode (and no mode runs SOR)
+        MgLineArgs a;
+        size_t sm;
+        const bool ok = nmodes <= cf.imgsor && 4 * nlev + 2 * cf.nbli + 8 <= kMglMaxPhase;
+        for (int cs = 1; cs <= 16 && ok; cs <<= 1)
+            if (mgl_plan(*T, g.n2m, cs, a, sm)) T->resident = 1;
+    }
     rc = set_up_tables(c, *T);
     if (rc) return rc;
+    if (T->resident) return mgl_init(c);
     const int ldp = nl + 2, ldg = T->nld + 1;
     T->pc_plane = (long long)ldp * (g.n2m + 2);
     T->gg_plane = (long long)ldg * (g.n2m + 2);
@@ -1493,7 +1791,8 @@ void mg2d_free(lesgpu_case *c) {
     void *ptrs[] = {T->d.aw, T->d.ae, T->d.as, T->d.an, T->d.coi1, T->d.coi2, T->d.cor1, T->d.cor2, T->ipm, T->imm,
                     T->d.ac, T->d.bet, T->d.gam, T->d.pc, T->d.gg, T->d.rs, T->d.rd, T->d.gu, T->d.gb, T->iters,
                     T->f.aw, T->f.ae, T->f.as, T->f.an, T->f.coi1, T->f.coi2, T->f.cor1, T->f.cor2,
-                    T->f.ac, T->f.bet, T->f.gam, T->f.pc, T->f.gg, T->f.rs, T->f.rd, T->f.gu, T->f.gb};
+                    T->f.ac, T->f.bet, T->f.gam, T->f.pc, T->f.gg, T->f.rs, T->f.rd, T->f.gu, T->f.gb,
+                    T->dargs, T->ltab_d, T->llc_d, T->lact, T->lasl, T->lanl, T->ltab_f, T->llc_f, T->lbt};
     for (void *q : ptrs) cudaFree(q);
     delete T;
     c->pois.mg = nullptr;
@@ -1588,7 +1887,8 @@ void launch_mg2d(lesgpu_case *c, int msub) {
     const int slot = (msub >= 1 && msub <= 3) ? msub - 1 : 0;
     inst_begin(c, LESGPU_K_POISSON);
     mg2d_pre(c, slot);
-    launch_modes(c, mg_args(c, slot, 0), T->cs);
+    if (T->resident) mgl_launch(c, slot);
+    else launch_modes(c, mg_args(c, slot, 0), T->cs);
     mg2d_post(c);
     inst_end(c, LESGPU_K_POISSON);
 }
@@ -1597,16 +1897,29 @@ void launch_mg2d(lesgpu_case *c, int msub) {
 // the mode solves of several cases of one shape in one launch
 void mg2d_launch_pre(lesgpu_case *c, int msub) { mg2d_pre(c, (msub >= 1 && msub <= 3) ? msub - 1 : 0); }
 void mg2d_launch_post(lesgpu_case *c) { mg2d_post(c); }
-int mg2d_batch_size(const lesgpu_case *) { return (int)sizeof(MgArgs); }
+int mg2d_batch_size(const lesgpu_case *c) { return (int)(c->pois.mg->resident ? sizeof(MgLineArgs) : sizeof(MgArgs)); }
 void mg2d_batch_args(lesgpu_case *c, int msub, void *out) {
+    if (c->pois.mg->resident) {
+        MgLineArgs l;
+        size_t sm;
+        mgl_args(c, c->pois.mg->cs, (msub >= 1 && msub <= 3) ? msub - 1 : 0, false, l, sm);
+        memcpy(out, &l, sizeof(l));
+        return;
+    }
     const MgArgs a = mg_args(c, (msub >= 1 && msub <= 3) ? msub - 1 : 0, 0);
     memcpy(out, &a, sizeof(MgArgs));
 }
-// d_args: n MgArgs of cases with equal mg2d_batch_key
+// d_args: n arguments (mg2d_batch_args) of cases with equal mg2d_batch_key
 void mg2d_launch_batch(const lesgpu_case *c0, const void *d_args, int n, cudaStream_t st) {
     const MgTables *T = c0->pois.mg;
     cudaLaunchConfig_t lc;
     cudaLaunchAttribute at[1];
+    if (T->resident) {
+        mgl_cfg(*T, lc, at, T->nmodes * n, T->cs, T->smem);
+        lc.stream = st;
+        cudaLaunchKernelEx(&lc, mgl_kernel(*T, c0->kp.g.n2m), (const MgLineArgs *)d_args, T->nmodes);
+        return;
+    }
     cluster_cfg(lc, at, T->nmodes * n, T->cs);
     lc.stream = st;
     cudaLaunchKernelEx(&lc, zft_batch_kernel(c0->kp.g.n2m), (const MgArgs *)d_args, T->nmodes);
@@ -1616,7 +1929,7 @@ void mg2d_launch_batch(const lesgpu_case *c0, const void *d_args, int n, cudaStr
 long long mg2d_batch_key(const lesgpu_case *c) {
     const MgTables *T = c->pois.mg;
     if (!T) return 0;
-    return (((long long)T->cs * 64 + T->nlev) * 64 + T->lc) * 4096 + T->nmodes;
+    return ((((long long)T->resident * 64 + T->cs) * 64 + T->nlev) * 64 + T->lc) * 4096 + T->nmodes;
 }
 
 // ---- autotuner: cluster size per mode.  A solve lasts as long as its
@@ -1627,6 +1940,47 @@ long long mg2d_batch_key(const lesgpu_case *c) {
 static std::map<std::array<int, 7>, int> g_zft_cs;
 static std::mutex g_zft_mu;
 
+// A seeded noise right-hand side of every mode for the timing runs.
+__global__ void k_mgl_noise(double2 *ccap, long long n) {
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        unsigned long long z = ((unsigned long long)t + 1ULL) * 0x9E3779B97F4A7C15ULL;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+        ccap[t] = make_double2((double)(int)(z >> 32) * 4.6e-10, (double)(int)z * 4.6e-10);
+    }
+}
+
+// Resident cycles: every cluster size that holds a mode is timed on solves of
+// all the modes.  More blocks shorten a mode's phases, but a cluster takes
+// its SMs whole: where the modes' clusters no longer run at once, the smaller
+// one wins (48x48 duct modes, 33 of them: DUCT4 us with 4 blocks, DUCT8 with 8).
+static int mgl_autotune(lesgpu_case *c) {
+    MgTables *T = c->pois.mg;
+    const long long n = (long long)T->nl * c->kp.g.n2m * T->nmodes;
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    int best = T->cs;
+    float best_ms = 3.0e38f;
+    bool any = false;
+    for (int cs = 1; cs <= 16; cs <<= 1) {
+        if ((T->cap >= 1 && cs > T->cap && any) || mgl_active(c, cs) < 1) continue;
+        any = true;
+        if (mgl_set_cluster(c, cs)) break;
+        for (int r = 0; r < 3; r++) {           // the first is the warm-up
+            k_mgl_noise<<<blocks_for(n), kThreads, 0, c->stream>>>(c->pois.ccap, n);
+            cudaEventRecord(e0, c->stream);
+            mgl_launch(c, 3);
+            cudaEventRecord(e1, c->stream);
+            float ms = 0.0f;
+            if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) break;
+            if (r > 0 && ms < best_ms) { best_ms = ms; best = cs; }
+        }
+    }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    return mgl_set_cluster(c, best);
+}
+
 int mg2d_autotune(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     MgTables *T = c->pois.mg;
@@ -1635,7 +1989,18 @@ int mg2d_autotune(lesgpu_case *c) {
     {
         std::lock_guard<std::mutex> lk(g_zft_mu);
         auto it = g_zft_cs.find(key);
-        if (it != g_zft_cs.end()) { T->cs = it->second; return 0; }
+        if (it != g_zft_cs.end()) {
+            if (T->resident) return it->second != T->cs ? mgl_set_cluster(c, it->second) : 0;
+            T->cs = it->second;
+            return 0;
+        }
+    }
+    if (T->resident) {
+        const int rc = mgl_autotune(c);
+        if (rc) return rc;
+        std::lock_guard<std::mutex> lk(g_zft_mu);
+        g_zft_cs[key] = T->cs;
+        return 0;
     }
     const MgArgs a = mg_args(c, 0, 3);
     cudaEvent_t e0, e1;
