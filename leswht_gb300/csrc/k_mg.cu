@@ -1180,43 +1180,15 @@ __global__ void k_mg_begin(DScal *S, int slot, int nfft, int nmodes, double fac)
 }
 
 // ------------------------------------------- tables of the resident cycles
-// Half a warp per line of a mode: the solve table of k_mgl.cuh from the LU
-// factors (bet, gam, i fastest), formed in FP64.
+// Half a warp per line of a mode: the solve table of k_mgl.cuh.
 template <int R, class T>
 __global__ void k_mgl_tables(const double *as, const double *bet, const double *gam, int nld, int n2m, long long nlines, T *tab) {
     const int lane = threadIdx.x & 15;
-    constexpr int W = 16 / (int)sizeof(T);
+    const unsigned half = 0xffffu << (threadIdx.x & 16);
     for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4; w < nlines;
          w += ((long long)gridDim.x * blockDim.x) >> 4) {
-        const unsigned half = 0xffffu << (threadIdx.x & 16);
-        const long long kv = w / nld, i = w % nld;
-        const size_t cb = (size_t)nld * n2m * kv + i;
-        T *to = tab + (size_t)w * mgl_tab_len<R, T>();
-        auto put = [&](int e, double v) { to[(e / W) * (16 * W) + lane * W + e % W] = (T)v; };
-        double P = 1.0, G = 1.0;
-        for (int q = 0; q < R; q++) {
-            const int j = lane * R + q, jb = lane * R + R - 1 - q;      // 0-based rows
-            const double b = j < n2m ? bet[cb + (size_t)nld * j] : 0.0;
-            const double p = j < n2m ? -as[j + 1] * b : 0.0;
-            const double g = jb + 1 < n2m ? -gam[cb + (size_t)nld * (jb + 1)] : 0.0;
-            P *= p;
-            G *= g;
-            put(q, b);
-            put(R + q, p);
-            put(2 * R + R - 1 - q, g);
-            if (mgl_cum<R>()) {
-                put(3 * R + 8 + q, P);
-                put(4 * R + 8 + R - 1 - q, G);
-            }
-        }
-        for (int s = 0; s < 4; s++) {
-            const int d = 1 << s;
-            put(3 * R + s, lane >= d ? P : 0.0);
-            put(3 * R + 4 + s, lane + d < 16 ? G : 0.0);
-            const double Po = __shfl_up_sync(half, P, d, 16), Go = __shfl_down_sync(half, G, d, 16);
-            if (lane >= d) P *= Po;
-            if (lane + d < 16) G *= Go;
-        }
+        const size_t cb = (size_t)nld * n2m * (w / nld) + w % nld;
+        mgl_table<R, T>(as, bet + cb, gam + cb, nld, n2m, lane, half, tab + (size_t)w * mgl_tab_len<R, T>());
     }
 }
 
@@ -1952,7 +1924,7 @@ __global__ void k_mgl_noise(double2 *ccap, long long n) {
 // Resident cycles: every cluster size that holds a mode is timed on solves of
 // all the modes.  More blocks shorten a mode's phases, but a cluster takes
 // its SMs whole: where the modes' clusters no longer run at once, the smaller
-// one wins (48x48 duct modes, 33 of them: DUCT4 us with 4 blocks, DUCT8 with 8).
+// one wins (33 modes of 48x48: 381 us a solve with 4 blocks a mode, 780 with 8).
 static int mgl_autotune(lesgpu_case *c) {
     MgTables *T = c->pois.mg;
     const long long n = (long long)T->nl * c->kp.g.n2m * T->nmodes;

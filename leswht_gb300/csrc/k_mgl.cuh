@@ -309,6 +309,18 @@ struct MglOp {
         }
         __syncwarp();
     }
+    // straight from global memory
+    __device__ __forceinline__ void fetch(const T *tab, int lane) {
+        using Q = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+        const Q *q = reinterpret_cast<const Q *>(tab) + (lane & 15);
+#pragma unroll
+        for (int r = 0; r < N; r++) {
+            const Q x = __ldg(q + r * 16);
+            e[W * r] = x.x;
+            e[W * r + 1] = x.y;
+            if constexpr (W == 4) { e[W * r + 2] = x.z; e[W * r + 3] = x.w; }
+        }
+    }
     __device__ __forceinline__ T bt(int r) const { return e[r]; }
     __device__ __forceinline__ T p(int r) const { return e[R + r]; }
     __device__ __forceinline__ T g(int r) const { return e[2 * R + r]; }
@@ -317,6 +329,38 @@ struct MglOp {
     __device__ __forceinline__ T cp(int r) const { return e[3 * R + 8 + r]; }
     __device__ __forceinline__ T cg(int r) const { return e[4 * R + 8 + r]; }
 };
+
+// One line's table from its LU factors: rows sj apart in bet and gam, as
+// 1-based; by the 16 lanes of `half`, formed in FP64.
+template <int R, class T>
+__device__ void mgl_table(const double *as, const double *bet, const double *gam, int sj, int n2m, int lane, unsigned half, T *tab) {
+    constexpr int W = 16 / (int)sizeof(T);
+    auto put = [&](int e, double v) { tab[(e / W) * (16 * W) + lane * W + e % W] = (T)v; };
+    double P = 1.0, G = 1.0;
+    for (int q = 0; q < R; q++) {
+        const int j = lane * R + q, jb = lane * R + R - 1 - q;      // 0-based rows
+        const double b = j < n2m ? bet[(size_t)sj * j] : 0.0;
+        const double p = j < n2m ? -as[j + 1] * b : 0.0;
+        const double g = jb + 1 < n2m ? -gam[(size_t)sj * (jb + 1)] : 0.0;
+        P *= p;
+        G *= g;
+        put(q, b);
+        put(R + q, p);
+        put(2 * R + R - 1 - q, g);
+        if (mgl_cum<R>()) {
+            put(3 * R + 8 + q, P);
+            put(4 * R + 8 + R - 1 - q, G);
+        }
+    }
+    for (int s = 0; s < 4; s++) {
+        const int d = 1 << s;
+        put(3 * R + s, lane >= d ? P : 0.0);
+        put(3 * R + 4 + s, lane + d < 16 ? G : 0.0);
+        const double Po = __shfl_up_sync(half, P, d, 16), Go = __shfl_down_sync(half, G, d, 16);
+        if (lane >= d) P *= Po;
+        if (lane + d < 16) G *= Go;
+    }
+}
 
 // start the copy of a line's table into the warp's stage
 template <int R, class T>

@@ -18,17 +18,29 @@
 // (iimg / kkmg ranges), so a neighbour or transfer index outside the level
 // reads zero -- it always carries a zero coefficient or weight.
 //
-// Fusions (exact: the fused operands are disjoint): the right-hand side of a
-// zebra half-sweep is formed in the same pass as the forward elimination;
-// the finest residual and its restriction (toplevel) are one pass, and so
-// are rescal and godown (every fine point belongs to one coarse point); the
-// closing toplevel's residual, which mg3d discards, is not computed.
+// Fusions: the right-hand side of a zebra half-sweep is formed in the same
+// pass as its line solves; a level's residual and its restriction are one
+// pass (toplevel, rescal + godown: every fine point belongs to one coarse
+// point); the closing toplevel's residual, which mg3d discards, is not
+// computed.  The residual after a relaxation without an initial guess is
+// known: zero on the lines solved last, minus the off-line neighbours' sum on
+// the others (their own rows cancel), so two of a coarse point's four fine
+// residuals vanish and the other two take four products each.
+//
+// What bounded the solve was the latency of its phases: one thread per y line
+// walked 2 n2m dependent rows with an L2 access in each.  A line is now solved by half a warp, its rows loaded
+// at once, with the table-driven scan of k_mgl.cuh, and the levels of at most
+// kMgrdSoloLines lines run on block 0 between two grid barriers (a block
+// barrier instead of a grid barrier per phase).  A solve, before and after, on
+// one GB300: 16x24x16 4.3 and 0.95 ms, 32^3 9.6 and 1.6, 64^3 21.1 and 3.2,
+// 128^3 58.7 and 10.9.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
-#include "k_fft.cuh"
+#include "k_mgl.cuh"
 #include "lesgpu_internal.cuh"
 
 namespace cg = cooperative_groups;
@@ -38,6 +50,9 @@ namespace lg {
 constexpr int kMgrdThreads = 256;
 constexpr int kMgrdMaxLev = 20;
 constexpr int kMgrdSlots = 8;   // partial-sum slots per block
+// levels of at most this many lines run on block 0: its eight warps solve a
+// colour of 64 lines in two rounds, less than the grid barrier it saves
+constexpr int kMgrdSoloLines = 64;
 
 struct MgrdLevel {
     int ibg, iend, nx, kbg, kend, nz;
@@ -51,21 +66,24 @@ struct MgrdTables {
     double *aw, *ae, *as, *an, *ab, *af, *fidw, *fkdw, *fiup, *fkup;
     int *imm, *ipm, *kmm, *kpm, *ih1, *ih2, *kh1, *kh2, *il1, *il2, *kl1, *kl2;
     double *bet, *gam, *gc, *rs;
+    double *tab;                  // solve tables of the lines (k_mgl.cuh); bet / gam serve longer lines
     double *p, *s, *y, *z, *v, *t, *res, *part;
 };
 
 struct MgrdArgs {
     int n1m, n2m, n3m, n2, nlev, nbli, mgitr, slot;
+    int solo;                     // levels 0 .. solo run on block 0 (-1: none)
     long long sx, sxy;
     const MgrdLevel *lev;
     const double *aw, *ae, *as, *an, *ab, *af, *fidw, *fkdw, *fiup, *fkup;
     const int *imm, *ipm, *kmm, *kpm, *ih1, *ih2, *kh1, *kh2, *il1, *il2, *kl1, *kl2;
-    const double *bet, *gam;
+    const double *bet, *gam, *tab;
     double *gc, *rs;
     double *p, *s, *y, *z, *v, *t, *res, *part;
     double *phi;
     const double *b;
     DScal *S;
+    IDiv d1, d2;                  // by n1m and n2m
 };
 
 // ------------------------------------------------------------ level access
@@ -92,12 +110,16 @@ struct LevelView {            // one level's storage, resolved once per phase
     }
 };
 
-// rhs - A gi at a point of a level (rescal / toplevel residual, :353-364, :414-421)
-__device__ __forceinline__ double mg_defect(const MgrdArgs &a, const LevelView &V, double rhs, int i, int j, int k) {
-    const double acc = -1.0 * (a.aw[i] + a.ae[i] + a.as[j] + a.an[j] + a.ab[k] + a.af[k]);
-    return rhs - acc * V.g[V.gi(i, j, k)] - a.aw[i] * V.get(a.imm[i], j, k) - a.ae[i] * V.get(a.ipm[i], j, k)
-           - a.as[j] * V.g[V.gi(i, j - 1, k)] - a.an[j] * V.g[V.gi(i, j + 1, k)]
-           - a.ab[k] * V.get(i, j, a.kmm[k]) - a.af[k] * V.get(i, j, a.kpm[k]);
+// colour 0 of a level: the lines its first half-sweep solves
+__device__ __forceinline__ bool mg_first(const MgrdArgs &a, const MgrdLevel &L, int i, int k) {
+    return (((i - L.ibg) ^ a.kpm[k]) & 1) == 0;
+}
+// The residual at a colour-0 point after a relaxation without an initial
+// guess (rescal / toplevel residual, :353-364, :414-421): its line's own rows
+// give the right-hand side back, the neighbouring lines' sum is left.
+__device__ __forceinline__ double mg_left(const MgrdArgs &a, const LevelView &V, int i, int j, int k) {
+    return -(a.aw[i] * V.get(a.imm[i], j, k) + a.ae[i] * V.get(a.ipm[i], j, k) + a.ab[k] * V.get(i, j, a.kmm[k])
+             + a.af[k] * V.get(i, j, a.kpm[k]));
 }
 
 // One zebra half-sweep of level l (relax :502-675 / toplevel :281-348): the y
@@ -105,7 +127,7 @@ __device__ __forceinline__ double mg_defect(const MgrdArgs &a, const LevelView &
 // take src - iold * (x and z neighbours) and are solved with the stored LU.
 // src is the full-layout right-hand side at the finest level, else resid.
 __device__ void mg_half(const MgrdArgs &a, double *sol, const double *src, int l, int color, double iold,
-                        long long tid, long long nthr) {
+                        int tid, int nthr) {
     const LevelView V(a, sol, l);
     const MgrdLevel &L = V.L;
     const int half = (L.nx + 1) >> 1;
@@ -150,63 +172,106 @@ __device__ void mg_half(const MgrdArgs &a, double *sol, const double *src, int l
     }
 }
 
-// toplevel's residual at the finest level restricted to level nlev-1
-// (:352-378), one coarse point per thread
-__device__ void mg_top_restrict(const MgrdArgs &a, double *sol, const double *rhs, long long tid, long long nthr) {
-    const LevelView F(a, sol, a.nlev);
-    const MgrdLevel C = a.lev[a.nlev - 1];
-    const long long n = (long long)C.nx * a.n2m * C.nz;
-    for (long long q = tid; q < n; q += nthr) {
-        const int ii = (int)(q % C.nx);
-        const long long r = q / C.nx;
-        const int j = 1 + (int)(r % a.n2m), kk = (int)(r / a.n2m);
-        const int ic = C.ibg + ii, kc = C.kbg + kk;
-        const int i1 = a.ih1[ic], i2 = a.ih2[ic], k1 = a.kh1[kc], k2 = a.kh2[kc];
-        const double fi = a.fidw[ic], fk = a.fkdw[kc];
-        const double r11 = mg_defect(a, F, rhs[i1 + a.sx * j + a.sxy * k1], i1, j, k1);
-        const double r21 = mg_defect(a, F, rhs[i2 + a.sx * j + a.sxy * k1], i2, j, k1);
-        const double r12 = mg_defect(a, F, rhs[i1 + a.sx * j + a.sxy * k2], i1, j, k2);
-        const double r22 = mg_defect(a, F, rhs[i2 + a.sx * j + a.sxy * k2], i2, j, k2);
-        a.rs[C.roff + q] = (1.0 - fi) * (1.0 - fk) * r11 + fi * (1.0 - fk) * r21 + (1.0 - fi) * fk * r12 + fi * fk * r22;
+// The same half-sweep with half a warp per line, its rows in the lanes'
+// registers (R each).  The last warps' idle halves run along on zeros.
+template <int R>
+__device__ __noinline__ void mg_half_scan(const MgrdArgs &a, double *sol, const double *src, int l, int color, double iold,
+                             int warp, int nwarp) {
+    const LevelView V(a, sol, l);
+    const MgrdLevel &L = V.L;
+    const int half = (L.nx + 1) >> 1, nlines = half * L.nz, n2m = a.n2m;
+    const int lane = threadIdx.x & 31, l16 = lane & 15;
+    for (int w = warp; 2 * w < nlines; w += nwarp) {
+        const int q = 2 * w + (lane >> 4), kk = q / half, hh = q - kk * half;
+        const int k = min(L.kbg + kk, L.kend);
+        const int i0 = L.ibg + (color == 0 ? (a.kpm[k] & 1) : (k & 1)) + 2 * hh;
+        const bool on = q < nlines && i0 <= L.iend;
+        const int i = min(i0, L.iend);
+        MglOp<R, double> o;
+        o.fetch(a.tab + (size_t)(L.loff / n2m + (i - L.ibg) + (long long)L.nx * (k - L.kbg)) * mgl_tab_len<R, double>(), lane);
+        const double *s0 = V.finest ? src + i + a.sxy * k : a.rs + L.roff + V.ri(a, i, 1, k) - L.nx;
+        const long long ss = V.finest ? a.sx : L.nx;
+        double v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int j = l16 * R + r + 1;
+            v[r] = on && j <= n2m ? s0[ss * j] : 0.0;
+        }
+        if (iold != 0.0) {
+            const int im = a.imm[i], ip = a.ipm[i], km = a.kmm[k], kp = a.kpm[k];
+            const double cw = -a.aw[i], ce = -a.ae[i], cb = -a.ab[k], cf = -a.af[k];
+            const double *gw = V.inside(im, k) ? V.g + V.gi(im, 0, k) : nullptr, *ge = V.inside(ip, k) ? V.g + V.gi(ip, 0, k) : nullptr;
+            const double *gb = V.inside(i, km) ? V.g + V.gi(i, 0, km) : nullptr, *gf = V.inside(i, kp) ? V.g + V.gi(i, 0, kp) : nullptr;
+            // the four neighbours' rows: all in flight together where the
+            // registers hold them
+            auto take = [&](const double *p, double (&x)[R]) {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const int j = l16 * R + r + 1;
+                    x[r] = on && p && j <= n2m ? p[V.sj * j] : 0.0;
+                }
+            };
+            auto add = [&](double c, const double (&x)[R]) {
+#pragma unroll
+                for (int r = 0; r < R; r++) v[r] += c * x[r];
+            };
+            if constexpr (R <= 6) {
+                double nw[R], ne[R], nb[R], nf[R];
+                take(gw, nw); take(ge, ne); take(gb, nb); take(gf, nf);
+                add(cw, nw); add(ce, ne); add(cb, nb); add(cf, nf);
+            } else {
+                double x[R];
+                take(gw, x); add(cw, x);
+                take(ge, x); add(ce, x);
+                take(gb, x); add(cb, x);
+                take(gf, x); add(cf, x);
+            }
+        }
+        mgl_solve<R, double>(v, o, lane);
+        double *g = V.g + V.gi(i, 0, k);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int j = l16 * R + r + 1;
+            if (on && j <= n2m) g[V.sj * j] = v[r];
+        }
     }
 }
 
-// rescal(l) (:403-425) then godown(l-1) (:455-476), one coarse point per
-// thread: the four level-l defects replace resid there and are restricted
-__device__ void mg_rescal_godown(const MgrdArgs &a, double *sol, int l, long long tid, long long nthr) {
+// The residual of level l restricted to level l - 1, one coarse point per
+// thread: toplevel's at the finest level (:352-378); below it rescal (:403-425)
+// and godown (:455-476), the residuals also replacing resid.
+__device__ void mg_restrict(const MgrdArgs &a, double *sol, int l, int tid, int nthr) {
     const LevelView F(a, sol, l);
     const MgrdLevel C = a.lev[l - 1];
-    const long long n = (long long)C.nx * a.n2m * C.nz;
-    for (long long q = tid; q < n; q += nthr) {
-        const int ii = (int)(q % C.nx);
-        const long long r = q / C.nx;
-        const int j = 1 + (int)(r % a.n2m), kk = (int)(r / a.n2m);
+    const int n = C.nx * a.n2m * C.nz;
+    for (int q = tid; q < n; q += nthr) {
+        const int r = q / C.nx, ii = q - r * C.nx, kk = r / a.n2m, j = 1 + r - kk * a.n2m;
         const int ic = C.ibg + ii, kc = C.kbg + kk;
         const int i1 = a.ih1[ic], i2 = a.ih2[ic], k1 = a.kh1[kc], k2 = a.kh2[kc];
         const double fi = a.fidw[ic], fk = a.fkdw[kc];
-        const long long q11 = F.L.roff + F.ri(a, i1, j, k1), q21 = F.L.roff + F.ri(a, i2, j, k1);
-        const long long q12 = F.L.roff + F.ri(a, i1, j, k2), q22 = F.L.roff + F.ri(a, i2, j, k2);
-        const double r11 = mg_defect(a, F, a.rs[q11], i1, j, k1);
-        const double r21 = mg_defect(a, F, a.rs[q21], i2, j, k1);
-        const double r12 = mg_defect(a, F, a.rs[q12], i1, j, k2);
-        const double r22 = mg_defect(a, F, a.rs[q22], i2, j, k2);
-        a.rs[q11] = r11; a.rs[q21] = r21; a.rs[q12] = r12; a.rs[q22] = r22;
-        a.rs[C.roff + q] = (1.0 - fi) * (1.0 - fk) * r11 + fi * (1.0 - fk) * r21 + (1.0 - fi) * fk * r12 + fi * fk * r22;
+        // colour 0 holds one diagonal of the four points, (i1, k1) and (i2, k2) or the other
+        const bool d = mg_first(a, F.L, i1, k1);
+        const int ia = d ? i1 : i2, ib = d ? i2 : i1;
+        const double ra = mg_left(a, F, ia, j, k1), rb = mg_left(a, F, ib, j, k2);
+        if (l < a.nlev) {
+            a.rs[F.L.roff + F.ri(a, ia, j, k1)] = ra;
+            a.rs[F.L.roff + F.ri(a, ib, j, k2)] = rb;
+            a.rs[F.L.roff + F.ri(a, ib, j, k1)] = 0.0;
+            a.rs[F.L.roff + F.ri(a, ia, j, k2)] = 0.0;
+        }
+        a.rs[C.roff + q] = (d ? 1.0 - fi : fi) * (1.0 - fk) * ra + (d ? fi : 1.0 - fi) * fk * rb;
     }
 }
 
 // goup(l) (:479-500): the points i = ibg + mod(k, 2) + 2q of level l gain
 // the interpolated correction of level l-1
-__device__ void mg_goup(const MgrdArgs &a, double *sol, int l, long long tid, long long nthr) {
+__device__ void mg_goup(const MgrdArgs &a, double *sol, int l, int tid, int nthr) {
     const LevelView F(a, sol, l), C(a, sol, l - 1);
     const MgrdLevel &L = F.L;
-    const int half = (L.nx + 1) >> 1;
-    const long long n = (long long)half * a.n2m * L.nz;
-    for (long long q = tid; q < n; q += nthr) {
-        const int hh = (int)(q % half);
-        const long long r = q / half;
-        const int j = 1 + (int)(r % a.n2m), k = L.kbg + (int)(r / a.n2m);
-        const int i = L.ibg + (k & 1) + 2 * hh;
+    const int half = (L.nx + 1) >> 1, n = half * a.n2m * L.nz;
+    for (int q = tid; q < n; q += nthr) {
+        const int r = q / half, hh = q - r * half, kk = r / a.n2m, j = 1 + r - kk * a.n2m;
+        const int k = L.kbg + kk, i = L.ibg + (k & 1) + 2 * hh;
         if (i > L.iend) continue;
         const double fi = a.fiup[i], fk = a.fkup[k];
         const int a1 = a.il1[i], a2 = a.il2[i], b1 = a.kl1[k], b2 = a.kl2[k];
@@ -218,33 +283,62 @@ __device__ void mg_goup(const MgrdArgs &a, double *sol, int l, long long tid, lo
 
 // mg3d (:227-268): one V-cycle, sol = M^-1 rhs.  The first half-sweep takes
 // no neighbours (IOLD = 0; with IOLD = 1 the reference reads its
-// uninitialised work array there, which is zero here).
-__device__ void mg3d(const MgrdArgs &a, cg::grid_group &grid, double *sol, const double *rhs, long long tid, long long nthr) {
+// uninitialised work array there, which is zero here).  Levels 0 .. solo run on
+// block 0.  R = 0: lines too long for the lanes' registers, a thread each.
+template <int R>
+__device__ void mg3d(const MgrdArgs &a, cg::grid_group &grid, double *sol, const double *rhs, int tid, int nthr) {
     const int nlev = a.nlev;
-    mg_half(a, sol, rhs, nlev, 0, 0.0, tid, nthr); grid.sync();
-    mg_half(a, sol, rhs, nlev, 1, 1.0, tid, nthr); grid.sync();
+    bool wide = true;                   // the phase's threads: the grid's, or block 0's
+    auto sync = [&]() {
+        if (wide) grid.sync();
+        else __syncthreads();
+    };
+    auto half = [&](int l, int color, double iold) {
+        const int t = wide ? tid : (int)threadIdx.x, n = wide ? nthr : (int)blockDim.x;
+        const double *src = l == nlev ? rhs : nullptr;
+        if constexpr (R > 0) mg_half_scan<R>(a, sol, src, l, color, iold, t >> 5, n >> 5);
+        else mg_half(a, sol, src, l, color, iold, t, n);
+        sync();
+    };
+    auto restrict_to = [&](int l) { mg_restrict(a, sol, l, wide ? tid : (int)threadIdx.x, wide ? nthr : (int)blockDim.x); sync(); };
+    auto goup = [&](int l) { mg_goup(a, sol, l, wide ? tid : (int)threadIdx.x, wide ? nthr : (int)blockDim.x); sync(); };
+    half(nlev, 0, 0.0);
+    half(nlev, 1, 1.0);
     if (nlev > 0) {
-        mg_top_restrict(a, sol, rhs, tid, nthr); grid.sync();
-        for (int l = nlev - 1; l >= 1; l--) {
-            mg_half(a, sol, nullptr, l, 0, 0.0, tid, nthr); grid.sync();
-            mg_half(a, sol, nullptr, l, 1, 1.0, tid, nthr); grid.sync();
-            mg_rescal_godown(a, sol, l, tid, nthr); grid.sync();
+        restrict_to(nlev);
+        for (int l = nlev - 1; l > a.solo && l >= 1; l--) {
+            half(l, 0, 0.0);
+            half(l, 1, 1.0);
+            restrict_to(l);
         }
-        mg_half(a, sol, nullptr, 0, 0, 0.0, tid, nthr); grid.sync();
-        mg_half(a, sol, nullptr, 0, 1, 1.0, tid, nthr); grid.sync();
-        for (int it = 1; it < a.nbli; it++) {
-            mg_half(a, sol, nullptr, 0, 0, 1.0, tid, nthr); grid.sync();
-            mg_half(a, sol, nullptr, 0, 1, 1.0, tid, nthr); grid.sync();
+        if (blockIdx.x == 0 || a.solo < 0) {
+            wide = a.solo < 0;
+            for (int l = min(a.solo, nlev - 1); l >= 1; l--) {
+                half(l, 0, 0.0);
+                half(l, 1, 1.0);
+                restrict_to(l);
+            }
+            for (int it = 0; it < a.nbli; it++) {
+                half(0, 0, it == 0 ? 0.0 : 1.0);
+                half(0, 1, 1.0);
+            }
+            for (int l = 1; l <= min(a.solo, nlev - 1); l++) {
+                goup(l);
+                half(l, 0, 1.0);
+                half(l, 1, 1.0);
+            }
+            wide = true;
         }
-        for (int l = 1; l <= nlev - 1; l++) {
-            mg_goup(a, sol, l, tid, nthr); grid.sync();
-            mg_half(a, sol, nullptr, l, 0, 1.0, tid, nthr); grid.sync();
-            mg_half(a, sol, nullptr, l, 1, 1.0, tid, nthr); grid.sync();
+        if (a.solo >= 0) grid.sync();
+        for (int l = max(a.solo, 0) + 1; l <= nlev - 1; l++) {
+            goup(l);
+            half(l, 0, 1.0);
+            half(l, 1, 1.0);
         }
-        mg_goup(a, sol, nlev, tid, nthr); grid.sync();
+        goup(nlev);
     }
-    mg_half(a, sol, rhs, nlev, 0, 1.0, tid, nthr); grid.sync();
-    mg_half(a, sol, rhs, nlev, 1, 1.0, tid, nthr); grid.sync();
+    half(nlev, 0, 1.0);
+    half(nlev, 1, 1.0);
 }
 
 // ------------------------------------------------------------ reductions
@@ -303,19 +397,27 @@ __device__ __forceinline__ double mg_apply(const MgrdArgs &a, const double *q, i
 // poisson (:25-224): phi = A^-1 divgsum to max|res| < test1, then
 // phi -= phi(1, n2m, 1).  IOLDV = 1 also starts from phi = 0 (solver.f90
 // zeroes phi before every call).
+template <int R>
 __global__ void __launch_bounds__(kMgrdThreads) k_mgrd_solve(MgrdArgs a) {
     cg::grid_group grid = cg::this_grid();
     __shared__ double sh[4 * 32];
-    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nthr = (long long)gridDim.x * blockDim.x;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
     const int n1m = a.n1m, n2m = a.n2m;
     const long long nin = (long long)n1m * n2m * a.n3m;
     const long long ntot = a.sxy * (a.n3m + 2);
+    const IDiv d1 = a.d1, d2 = a.d2;    // multiply-shift division (below 2^31 points)
     auto at = [&](long long q, int &i, int &j, int &k) {
-        i = 1 + (int)(q % n1m);
-        const long long r = q / n1m;
-        j = 1 + (int)(r % n2m);
-        k = 1 + (int)(r / n2m);
+        if (q < (1LL << 31)) {
+            const unsigned t = (unsigned)q, r = d1.div(t), kk = d2.div(r);
+            i = 1 + (int)(t - r * (unsigned)n1m);
+            j = 1 + (int)(r - kk * (unsigned)n2m);
+            k = 1 + (int)kk;
+        } else {
+            i = 1 + (int)(q % n1m);
+            const long long r = q / n1m;
+            j = 1 + (int)(r % n2m);
+            k = 1 + (int)(r / n2m);
+        }
         return i + a.sx * j + a.sxy * k;
     };
     for (long long q = tid; q < ntot; q += nthr) a.phi[q] = 0.0;
@@ -344,7 +446,7 @@ __global__ void __launch_bounds__(kMgrdThreads) k_mgrd_solve(MgrdArgs a) {
             a.p[c] = a.res[c] + bet * (a.p[c] - w * a.v[c]);
         }
         grid.sync();
-        mg3d(a, grid, a.y, a.p, tid, nthr);
+        mg3d<R>(a, grid, a.y, a.p, tid, nthr);
         double rv[1] = {0.0};
         for (long long q = tid; q < nin; q += nthr) {
             int i, j, k;
@@ -362,7 +464,7 @@ __global__ void __launch_bounds__(kMgrdThreads) k_mgrd_solve(MgrdArgs a) {
             a.s[c] = a.res[c] - alp * a.v[c];
         }
         grid.sync();
-        mg3d(a, grid, a.z, a.s, tid, nthr);
+        mg3d<R>(a, grid, a.z, a.s, tid, nthr);
         double ub[2] = {0.0, 0.0};
         const bool sum2[2] = {false, false};
         for (long long q = tid; q < nin; q += nthr) {
@@ -407,6 +509,33 @@ __global__ void __launch_bounds__(kMgrdThreads) k_mgrd_solve(MgrdArgs a) {
 }
 
 // ------------------------------------------------------------ host side
+// Half a warp per line: its solve table (k_mgl.cuh) from bet and gam, which hold
+// the lines of a level side by side.
+template <int R>
+__global__ void k_mgrd_tables(const double *as, const double *bet, const double *gam, int nx, int nz, int n2m, double *tab) {
+    const int lane = threadIdx.x & 15;
+    const unsigned half = 0xffffu << (threadIdx.x & 16);
+    const int nlines = nx * nz;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; w < nlines; w += (gridDim.x * blockDim.x) >> 4) {
+        const size_t cb = (size_t)(w % nx) + (size_t)nx * n2m * (w / nx);
+        mgl_table<R, double>(as, bet + cb, gam + cb, nx, n2m, lane, half, tab + (size_t)w * mgl_tab_len<R, double>());
+    }
+}
+
+typedef void (*MgrdKernel)(MgrdArgs);
+static MgrdKernel mgrd_kernel(int n2m) {
+    if (n2m > 256) return k_mgrd_solve<0>;
+    switch (mgl_r(n2m)) {
+    case 2: return k_mgrd_solve<2>;
+    case 3: return k_mgrd_solve<3>;
+    case 4: return k_mgrd_solve<4>;
+    case 6: return k_mgrd_solve<6>;
+    case 8: return k_mgrd_solve<8>;
+    case 12: return k_mgrd_solve<12>;
+    default: return k_mgrd_solve<16>;
+    }
+}
+
 // poisinit + mgcoef + tridcoef (:678-993)
 int mgrd_init(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
@@ -587,6 +716,31 @@ int mgrd_init(lesgpu_case *c) {
     std::vector<MgrdLevel> lev(T->h_lev, T->h_lev + nlev + 1);
     up(T->lev, lev);
     if (!ok) return LESGPU_ERR_OOM;
+    if (n2m <= 256) {                  // the lines' solve tables; they replace bet and gam
+        auto build = [&](auto m) {
+            constexpr int R = decltype(m)::value, len = mgl_tab_len<R, double>();
+            if (cudaMalloc(&T->tab, sizeof(double) * (size_t)(loff / n2m) * len) != cudaSuccess) { ok = false; return; }
+            for (int l = 0; l <= nlev; l++) {
+                const MgrdLevel &L = T->h_lev[l];
+                k_mgrd_tables<R><<<blocks_for((long long)L.nx * L.nz * 16), kThreads>>>(
+                    T->as, T->bet + L.loff, T->gam + L.loff, L.nx, L.nz, n2m, T->tab + (size_t)(L.loff / n2m) * len);
+            }
+            if (cudaDeviceSynchronize() != cudaSuccess) ok = false;
+        };
+        switch (mgl_r(n2m)) {
+        case 2: build(std::integral_constant<int, 2>{}); break;
+        case 3: build(std::integral_constant<int, 3>{}); break;
+        case 4: build(std::integral_constant<int, 4>{}); break;
+        case 6: build(std::integral_constant<int, 6>{}); break;
+        case 8: build(std::integral_constant<int, 8>{}); break;
+        case 12: build(std::integral_constant<int, 12>{}); break;
+        default: build(std::integral_constant<int, 16>{}); break;
+        }
+        cudaFree(T->bet);
+        cudaFree(T->gam);
+        T->bet = T->gam = nullptr;
+        if (!ok) return LESGPU_ERR_OOM;
+    }
     const size_t nt = (size_t)g.nt;
     double **vecs[7] = {&T->p, &T->s, &T->y, &T->z, &T->v, &T->t, &T->res};
     for (double **pv : vecs) {
@@ -598,13 +752,15 @@ int mgrd_init(lesgpu_case *c) {
         return LESGPU_ERR_OOM;
     cudaMemset(T->gc, 0, sizeof(double) * (size_t)(goff > 0 ? goff : 1));   // ghost rows j = 0, n2 stay zero
     // persistent grid: every block co-resident (a cooperative launch checks
-    // it); at most two blocks per SM keeps the barriers short
+    // it); at most two blocks per SM, and no more than the points fill, keep
+    // the barriers short
     int dev = 0, nsm = 0, occ = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mgrd_solve, kMgrdThreads, 0) != cudaSuccess || occ < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mgrd_kernel(n2m), kMgrdThreads, 0) != cudaSuccess || occ < 1)
         return LESGPU_ERR_CUDA;
     T->nblocks = nsm * (occ < 2 ? occ : 2);
+    T->nblocks = std::min(T->nblocks, std::max(32, blocks_for((long long)n1m * n2m * n3m, kMgrdThreads)));
     if (cudaMalloc(&T->part, sizeof(double) * kMgrdSlots * (size_t)T->nblocks) != cudaSuccess) return LESGPU_ERR_OOM;
     return cudaDeviceSynchronize() == cudaSuccess ? 0 : LESGPU_ERR_CUDA;
 }
@@ -614,7 +770,7 @@ void mgrd_free(lesgpu_case *c) {
     if (!T) return;
     void *ptrs[] = {T->lev, T->aw, T->ae, T->as, T->an, T->ab, T->af, T->fidw, T->fkdw, T->fiup, T->fkup,
                     T->imm, T->ipm, T->kmm, T->kpm, T->ih1, T->ih2, T->kh1, T->kh2, T->il1, T->il2, T->kl1, T->kl2,
-                    T->bet, T->gam, T->gc, T->rs, T->p, T->s, T->y, T->z, T->v, T->t, T->res, T->part};
+                    T->bet, T->gam, T->tab, T->gc, T->rs, T->p, T->s, T->y, T->z, T->v, T->t, T->res, T->part};
     for (void *q : ptrs) cudaFree(q);
     delete T;
     c->pois.mgrd = nullptr;
@@ -631,12 +787,16 @@ void launch_mgrd(lesgpu_case *c, int msub) {
     a.slot = (msub >= 1 && msub <= 3) ? msub - 1 : 0;
     a.sx = g.sx; a.sxy = g.sxy;
     a.lev = T->lev;
+    a.d1 = IDiv::make(g.n1m); a.d2 = IDiv::make(g.n2m);
+    a.solo = -1;
+    for (int l = 0; l < T->nlev; l++)
+        if ((long long)T->h_lev[l].nx * T->h_lev[l].nz <= kMgrdSoloLines) a.solo = l;
     a.aw = T->aw; a.ae = T->ae; a.as = T->as; a.an = T->an; a.ab = T->ab; a.af = T->af;
     a.fidw = T->fidw; a.fkdw = T->fkdw; a.fiup = T->fiup; a.fkup = T->fkup;
     a.imm = T->imm; a.ipm = T->ipm; a.kmm = T->kmm; a.kpm = T->kpm;
     a.ih1 = T->ih1; a.ih2 = T->ih2; a.kh1 = T->kh1; a.kh2 = T->kh2;
     a.il1 = T->il1; a.il2 = T->il2; a.kl1 = T->kl1; a.kl2 = T->kl2;
-    a.bet = T->bet; a.gam = T->gam; a.gc = T->gc; a.rs = T->rs;
+    a.bet = T->bet; a.gam = T->gam; a.tab = T->tab; a.gc = T->gc; a.rs = T->rs;
     a.p = T->p; a.s = T->s; a.y = T->y; a.z = T->z; a.v = T->v; a.t = T->t; a.res = T->res; a.part = T->part;
     a.phi = c->kp.f.phi; a.b = c->kp.f.divgsum; a.S = c->S;
     cudaLaunchConfig_t lc = {};
@@ -649,7 +809,7 @@ void launch_mgrd(lesgpu_case *c, int msub) {
     lc.attrs = at;
     lc.numAttrs = 1;
     inst_begin(c, LESGPU_K_POISSON);
-    cudaLaunchKernelEx(&lc, k_mgrd_solve, a);
+    cudaLaunchKernelEx(&lc, mgrd_kernel(g.n2m), a);
     inst_end(c, LESGPU_K_POISSON);
 }
 
