@@ -150,34 +150,11 @@ __device__ __forceinline__ void adi_chunk_coefs(const KP &p, int comp, int dir, 
     }
 }
 
-// Reciprocal of a pivot.  FP32: the division.  FP64: Newton-Raphson
-// iteration for 1/d, r <- r + r (1 - d r), from an FP32 reciprocal seed; each
-// step squares the relative error (2^-22 -> 2^-44 -> below the final
-// rounding), so the result is within 2 ulp of the quotient.  The seed's
-// FP64 <-> FP32 moves are done on the bit patterns with integer operations
-// (exponent rebias, mantissa truncated to 23 bits), not by conversions, which
-// on GB300 issue on the narrow FP64 pipe: the reciprocal then costs that pipe
-// four FMAs where a correctly rounded division takes more.  Pivots whose
-// binary exponent lies outside [-99, 99], where the FP32 seed or its
-// reciprocal would leave the normal FP32 range, take the division.
+// Reciprocal of a pivot: FP32 the division, FP64 rcp_fp64.
 template <class R>
 __device__ __forceinline__ R rcp_pivot(R d) {
     if (sizeof(R) == 4) return R(1.0) / d;
-    const unsigned long long bits = (unsigned long long)__double_as_longlong((double)d);
-    const unsigned hi = (unsigned)(bits >> 32);
-    const int ed = (int)((hi >> 20) & 0x7ffu);                // biased FP64 exponent
-    if ((unsigned)(ed - (1023 - 99)) > 198u) return R(1.0) / d;
-    const unsigned fs = (hi & 0x80000000u) | ((unsigned)(ed - 1023 + 127) << 23) | ((unsigned)(bits >> 29) & 0x7fffffu);
-    const unsigned rs = __float_as_uint(__frcp_rn(__uint_as_float(fs)));
-    const unsigned long long rb = ((unsigned long long)(rs & 0x80000000u) << 32)
-                                | ((unsigned long long)(((rs >> 23) & 0xffu) - 127u + 1023u) << 52)
-                                | ((unsigned long long)(rs & 0x7fffffu) << 29);
-    double r = __longlong_as_double((long long)rb);
-    double e = fma(-(double)d, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-(double)d, r, 1.0);
-    r = fma(r, e, r);
-    return R(r);
+    return R(rcp_fp64((double)d));
 }
 
 // Elements per chunk: a thread issues the loads of CH consecutive line

@@ -85,18 +85,32 @@ __device__ __forceinline__ void fft_stage(const V *in, V *out, int L, const Fast
             y[2] = csub(s02, s13);
             y[1] = cadd(d02, jd13);
             y[3] = csub(d02, jd13);
+        } else if constexpr (R == 3) {
+            // 12 operations instead of the 24 of the plain sums (Winograd,
+            // "On computing the discrete Fourier transform", Math. Comp. 32
+            // (1978)): a warp's FP64 operation takes 64 clocks on GB300
+            using T = decltype(V{}.x);
+            const T h = inv ? T(-0.86602540378443864676) : T(0.86602540378443864676);
+            const V t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+            const V m = V{v[0].x - T(0.5) * t.x, v[0].y - T(0.5) * t.y};
+            y[0] = cadd(v[0], t);
+            y[1] = V{m.x + h * d.y, m.y - h * d.x};
+            y[2] = V{m.x - h * d.y, m.y + h * d.x};
         } else {
-#pragma unroll
-            for (int m = 0; m < R; m++) {
-                V acc = v[0];
-#pragma unroll
-                for (int r = 1; r < R; r++) {
-                    V t = tw[((m * r) % R) * NR];
-                    if (inv) t.y = -t.y;
-                    acc = cadd(acc, cmul(v[r], t));
-                }
-                y[m] = acc;
-            }
+            // 36 operations instead of 80
+            using T = decltype(V{}.x);
+            const T c1 = T(0.30901699437494742410), c2 = T(-0.80901699437494742410);
+            const T s1 = inv ? T(-0.95105651629515357212) : T(0.95105651629515357212);
+            const T s2 = inv ? T(-0.58778525229247312917) : T(0.58778525229247312917);
+            const V a = cadd(v[1], v[4]), b = cadd(v[2], v[3]), e = csub(v[1], v[4]), f = csub(v[2], v[3]);
+            const V m1 = V{v[0].x + c1 * a.x + c2 * b.x, v[0].y + c1 * a.y + c2 * b.y};
+            const V m2 = V{v[0].x + c2 * a.x + c1 * b.x, v[0].y + c2 * a.y + c1 * b.y};
+            const V n1 = V{s1 * e.x + s2 * f.x, s1 * e.y + s2 * f.y}, n2 = V{s2 * e.x - s1 * f.x, s2 * e.y - s1 * f.y};
+            y[0] = V{v[0].x + a.x + b.x, v[0].y + a.y + b.y};
+            y[1] = V{m1.x + n1.y, m1.y - n1.x};
+            y[4] = V{m1.x - n1.y, m1.y + n1.x};
+            y[2] = V{m2.x + n2.y, m2.y - n2.x};
+            y[3] = V{m2.x - n2.y, m2.y + n2.x};
         }
         const int idxD = jq * Ns * R + jm;
 #pragma unroll
@@ -355,63 +369,102 @@ __device__ __forceinline__ void ycoef(const DGrid &g, const double *ak1, const d
 }
 
 // Elimination and substitution in one pass (the allocation-free entry point,
-// which keeps no per-case tables).
-__global__ void k_ytri_elim(KP p, double2 *ccap, const double *ak1, const double *ak3, double *gam) {
-    const DGrid &g = p.g;
-    const int n1m = g.n1m, n2m = g.n2m, n3mh = g.n3mh;
-    long long nl = (long long)n1m * n3mh;
-    const long long sj = (long long)n1m * n3mh;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nl; t += (long long)gridDim.x * blockDim.x) {
-        int i = 1 + (int)(t % n1m), k = 1 + (int)(t / n1m);
-        double2 *r = ccap + (i - 1) + (size_t)n1m * (k - 1);
-        double *gm = gam + (i - 1) + (size_t)n1m * (k - 1);
-        bool pin = (i == 1 && k == 1);
-        double am, ac, ap;
-        double ajcref = 0.0, ajmref = 0.0;
-        double2 crhsref = make_double2(0.0, 0.0);
-        if (pin) crhsref = r[(n2m - 1) * sj];
-        // forward
-        ycoef(g, ak1, ak3, i, k, 1, am, ac, ap);
-        if (pin && n2m == 1) { ajcref = ac; ajmref = am; ac = 1.0; am = 0.0; ap = 0.0; }
-        double bet = 1.0 / ac;
-        double2 x = r[0];
-        if (pin && n2m == 1) x = make_double2(0.0, 0.0);
-        x.x *= bet; x.y *= bet;
-        r[0] = x;
-        double cprev = ap;
-        for (int j = 2; j <= n2m; j++) {
-            ycoef(g, ak1, ak3, i, k, j, am, ac, ap);
-            double2 rj = r[(j - 1) * sj];
-            if (pin && j == n2m) {
-                ajcref = ac; ajmref = am;
-                ac = 1.0; am = 0.0; ap = 0.0;
-                rj = make_double2(0.0, 0.0);
-            }
-            double gj = cprev * bet;
-            bet = 1.0 / (ac - am * gj);
-            x = make_double2((rj.x - am * x.x) * bet, (rj.y - am * x.y) * bet);
-            gm[(j - 1) * sj] = gj;
-            r[(j - 1) * sj] = x;
-            cprev = ap;
+// which keeps no per-case tables).  A line's rows are eliminated from both ends
+// at once, by lane l of a half-warp upwards and lane l + 16 downwards, which
+// meet in a 2x2 system: half the dependent rows and twice the warps of the
+// one-ended sweep, which ran 128x125x120's 7808 modes as 244 warps of the
+// GPU's 608 sub-partitions.  A row costs 11 FP64 operations (64 clocks each
+// of a warp), 12 with the back substitution's two, from precomputed rows.
+// 128x125x120: 194 us one-ended, 55 this way.
+__global__ void __launch_bounds__(64) k_ytri_elim(int n1m, int n2m, int n3mh, double2 *ccap, const double *ak1, const double *ak3,
+                                                  const double4 *rows, double *gam) {
+    const long long nl = (long long)n1m * n3mh, sj = nl;
+    const int lane = threadIdx.x & 31, up = lane >> 4;      // up: the half that comes down from row n2m
+    const long long ngrp = (nl + 15) / 16;
+    constexpr int U = 4;
+    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ngrp;
+         w += ((long long)gridDim.x * blockDim.x) >> 5) {
+        const long long t0 = w * 16 + (lane & 15), t = t0 < nl ? t0 : nl - 1;
+        const bool on = t0 < nl;
+        const double akk = ak1[1 + (int)(t % n1m)] + ak3[1 + (int)(t / n1m)];
+        double2 *r = ccap + t;
+        double *gm = gam + t;
+        const bool pin = t == 0;
+        const int nb = (n2m + 1) / 2, n = up ? n2m - nb : nb;       // rows of this half
+        const int j0 = up ? n2m : 1, dj = up ? -1 : 1;
+        const double2 crhsref = pin ? r[(long long)(n2m - 1) * sj] : make_double2(0.0, 0.0);
+        // forward: g = (previous row's outer coefficient) bet, kept for the way back
+        double bet = 0.0, cprev = 0.0;
+        double2 x = make_double2(0.0, 0.0);
+        for (int q0 = 0; q0 < n; q0 += U) {
+            double2 rv[U];
+            double4 cf[U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (q0 + u < n) {
+                    const int j = j0 + dj * (q0 + u);
+                    rv[u] = r[(long long)(j - 1) * sj];
+                    cf[u] = rows[j];
+                }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (q0 + u < n) {
+                    const int j = j0 + dj * (q0 + u);
+                    double lo = up ? cf[u].y : cf[u].x, hi = up ? cf[u].x : cf[u].y, ac = cf[u].z - cf[u].w * akk;
+                    double2 rj = rv[u];
+                    if (pin && j == n2m) { ac = 1.0; lo = hi = 0.0; rj = make_double2(0.0, 0.0); }
+                    const double g = cprev * bet;
+                    bet = rcp_fp64(ac - lo * g);
+                    x = make_double2((rj.x - lo * x.x) * bet, (rj.y - lo * x.y) * bet);
+                    cprev = hi;
+                    if (on) {
+                        gm[(long long)(j - 1) * sj] = g;
+                        r[(long long)(j - 1) * sj] = x;
+                    }
+                }
         }
-        // backward
-        double2 xn = x;
-        for (int j = n2m - 1; j >= 1; j--) {
-            double2 xj = r[(j - 1) * sj];
-            double gn = gm[j * sj];
-            xj = make_double2(xj.x - gn * xn.x, xj.y - gn * xn.y);
-            r[(j - 1) * sj] = xj;
-            xn = xj;
+        // the two halves' last rows: x_b = y - G x_t and x_t = z - G' x_b
+        const double G = cprev * bet;
+        const double Go = __shfl_xor_sync(0xffffffffu, G, 16);
+        const double2 xo = make_double2(__shfl_xor_sync(0xffffffffu, x.x, 16), __shfl_xor_sync(0xffffffffu, x.y, 16));
+        const double det = rcp_fp64(1.0 - G * Go);
+        double2 xn = make_double2((x.x - G * xo.x) * det, (x.y - G * xo.y) * det);
+        if (on && n > 0) r[(long long)(j0 + dj * (n - 1) - 1) * sj] = xn;
+        // backward, outwards
+        for (int q0 = n - 2; q0 >= 0; q0 -= U) {
+            double2 xv[U];
+            double gv[U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (q0 - u >= 0) {
+                    const int j = j0 + dj * (q0 - u);
+                    xv[u] = r[(long long)(j - 1) * sj];
+                    gv[u] = gm[(long long)(j + dj - 1) * sj];
+                }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (q0 - u >= 0) {
+                    const int j = j0 + dj * (q0 - u);
+                    xn = make_double2(xv[u].x - gv[u] * xn.x, xv[u].y - gv[u] * xn.y);
+                    if (on) r[(long long)(j - 1) * sj] = xn;
+                }
         }
-        if (pin) {
-            // phref = (-ajmref*crhs(n2m-1,1) + crhsref)/ajcref; shift; crhs(n2m,1) = 0
-            double2 cm = n2m >= 2 ? r[(n2m - 2) * sj] : make_double2(0.0, 0.0);
-            double2 ph = make_double2((-ajmref * cm.x + crhsref.x) / ajcref, (-ajmref * cm.y + crhsref.y) / ajcref);
-            for (int j = 1; j <= n2m; j++) {
-                double2 v = r[(j - 1) * sj];
-                r[(j - 1) * sj] = make_double2(v.x - ph.x, v.y - ph.y);
+        // the pinned mode (poiss_ftft.f90:93-112): phref = (-ajmref*crhs(n2m-1,1)
+        // + crhsref)/ajcref; shift; crhs(n2m,1) = 0
+        if (w == 0) {
+            __syncwarp();
+            if (pin && on) {
+                const double4 last = rows[n2m];
+                const double2 cm = r[(long long)(n2m - 2) * sj];
+                const double ajc = last.z - last.w * akk;
+                const double2 ph = make_double2((-last.x * cm.x + crhsref.x) / ajc, (-last.x * cm.y + crhsref.y) / ajc);
+                __syncwarp(0x00010001u);            // both halves have read row n2m - 1
+                for (int q = 0; q < n; q++) {
+                    const long long at = (long long)(j0 + dj * q - 1) * sj;
+                    const double2 v = r[at];
+                    r[at] = j0 + dj * q == n2m ? make_double2(0.0, 0.0) : make_double2(v.x - ph.x, v.y - ph.y);
+                }
             }
-            r[(n2m - 1) * sj] = make_double2(0.0, 0.0);
         }
     }
 }

@@ -200,6 +200,30 @@ constexpr unsigned kMirVel = kMirU | kMirV | kMirW;
 // ------------------------------------------------------------------ helpers
 __device__ __forceinline__ double fixd(int v) { return (double)v; }
 
+// 1/d to within 2 ulp, from an FP32 reciprocal seed r (relative error
+// e = 1 - d r of about 2^-22) and one third-order step r + r (e + e^2), which
+// leaves e^3: three FMAs, one less than two Newton-Raphson steps.  (FP64
+// operations of a warp take 64 clocks on GB300; a correctly rounded division
+// takes more of them.)  The seed's FP64 <-> FP32 moves are done on the bit
+// patterns with integer operations (exponent rebias, mantissa truncated to 23
+// bits), not by conversions, which also issue on the FP64 pipe.  Operands
+// whose binary exponent lies outside [-99, 99], where the FP32 seed or its
+// reciprocal would leave the normal FP32 range, take the division.
+__device__ __forceinline__ double rcp_fp64(double d) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(d);
+    const unsigned hi = (unsigned)(bits >> 32);
+    const int ed = (int)((hi >> 20) & 0x7ffu);                // biased FP64 exponent
+    if ((unsigned)(ed - (1023 - 99)) > 198u) return 1.0 / d;
+    const unsigned fs = (hi & 0x80000000u) | ((unsigned)(ed - 1023 + 127) << 23) | ((unsigned)(bits >> 29) & 0x7fffffu);
+    const unsigned rs = __float_as_uint(__frcp_rn(__uint_as_float(fs)));
+    const unsigned long long rb = ((unsigned long long)(rs & 0x80000000u) << 32)
+                                | ((unsigned long long)(((rs >> 23) & 0xffu) - 127u + 1023u) << 52)
+                                | ((unsigned long long)(rs & 0x7fffffu) << 29);
+    const double r = __longlong_as_double((long long)rb);
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // Division of 0 <= n < 2^31 by an invariant d >= 1 as a multiply and a shift
 // (Granlund & Montgomery, "Division by invariant integers using
 // multiplication", PLDI 1994, theorem 4.2 with N = 31): l = ceil(log2 d),

@@ -37,6 +37,7 @@
 //     whose 1/dx or 1/dz varies by more than 1e-6 relative, is rejected with
 //     LESGPU_ERR_UNSUPPORTED.
 #include "k_fft.cuh"
+#include <algorithm>
 #include <math.h>
 #include <mutex>
 #include <string.h>
@@ -101,32 +102,55 @@ struct YTables {
 };
 
 struct TableDst {
-    double *ak1, *ak3, *f2fyi, *c2cyi;
-    int *jpv, *fixjl, *fixju;
+    double *ak1, *ak3;
+    double4 *rows;              // (am, ap, c0, w) of row j (k_ytri_elim)
     double2 *twx, *twz;
 };
 
 // poisinit of poiss_ftft.f90:164-204 on the device: the modified wavenumbers
 // ak1 = 2 (1 - cos(2 pi (i-1) / n1m)) / dx^2 (mirrored above n1mh) and
 // ak3 likewise over z, the twiddles exp(-2 pi i e / n) of both transforms,
-// and the y tables copied out of the parameter block.
-__global__ void k_noalloc_tables(YTables y, TableDst d, int n1m, int n2m, int n3m, double sdxis, double sdzis) {
-    const int n1mh = n1m / 2 + 1, n3mh = n3m / 2 + 1, n2 = n2m + 1;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < kMaxDir + 3; t += gridDim.x * blockDim.x) {
+// and the rows of the y systems from the parameter block's tables.
+// A block row per table (the transcendental functions are FP64-pipe bound, 64
+// clocks an operation of a warp: one warp should not walk through all four).
+__global__ void __launch_bounds__(64) k_noalloc_tables(YTables y, TableDst d, int n1m, int n2m, int n3m, double sdxis, double sdzis) {
+    const int n1mh = n1m / 2 + 1, n3mh = n3m / 2 + 1;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    double s, c;
+    switch (blockIdx.y) {
+    case 0:
         if (t <= n1m + 2) {
             double v = 0.0;
             const int i = (t >= n1mh + 1 && t <= n1m) ? n1m + 2 - t : t;
             if (t >= 1 && t <= n1m) v = 2.0 * (1.0 - cospi(2.0 * (double)(i - 1) / (double)n1m)) * sdxis * sdxis;
             d.ak1[t] = v;
         }
+        break;
+    case 1:
         if (t <= n3mh + 1)
             d.ak3[t] = (t >= 1 && t <= n3mh) ? 2.0 * (1.0 - cospi(2.0 * (double)(t - 1) / (double)n3m)) * sdzis * sdzis : 0.0;
-        if (t <= n2 + 1) { d.f2fyi[t] = y.f2fyi[t]; d.c2cyi[t] = y.c2cyi[t]; }
-        if (t <= n2m + 1) { d.jpv[t] = y.jpv[t]; d.fixjl[t] = y.fixjl[t]; d.fixju[t] = y.fixju[t]; }
-        double s, c;
+        break;
+    case 2:
         if (t < n1m) { sincospi(-2.0 * (double)t / (double)n1m, &s, &c); d.twx[t] = make_double2(c, s); }
+        break;
+    case 3:
         if (t < n3m) { sincospi(-2.0 * (double)t / (double)n3m, &s, &c); d.twz[t] = make_double2(c, s); }
+        break;
+    default:
+        if (t >= 1 && t <= n2m) {
+            const double fl = y.fixjl[t], fu = y.fixju[t], in = (1.0 - fl) * (1.0 - fu);
+            const double am = y.f2fyi[t] * y.c2cyi[t] * (1.0 - fl), ap = y.f2fyi[t] * y.c2cyi[y.jpv[t]] * (1.0 - fu);
+            d.rows[t] = make_double4(am, ap, -((am + ap) * in + y.f2fyi[1] * y.c2cyi[2] * fl + y.f2fyi[n2m] * y.c2cyi[n2m] * fu),
+                                     in + fl + fu);
+        }
     }
+}
+
+// lines a transform block takes: n points, count lines in each of `batch` groups
+int lines(int n, int count, int batch) {
+    int L = std::min(lg::fft_lines_per_block(n), 4);
+    while (L > 1 && (long long)((count + L - 1) / L) * batch < 2 * 152) L >>= 1;
+    return L;
 }
 
 // x and z must wrap (ipv(n1m) = 1, kpv(n3m) = 1) and be uniform: every 1/dx
@@ -167,11 +191,7 @@ extern "C" int lesgpu_poisson_ftft_noalloc(const lesgpu_grid *g, const double *d
     size_t off = 0;
     const size_t o_ak1 = off; off = align256(off + sizeof(double) * (n1 + 2));
     const size_t o_ak3 = off; off = align256(off + sizeof(double) * (n3mh + 2));
-    const size_t o_f2fyi = off; off = align256(off + sizeof(double) * (n2 + 2));
-    const size_t o_c2cyi = off; off = align256(off + sizeof(double) * (n2 + 2));
-    const size_t o_jpv = off; off = align256(off + sizeof(int) * (n2m + 2));
-    const size_t o_fixjl = off; off = align256(off + sizeof(int) * (n2m + 2));
-    const size_t o_fixju = off; off = align256(off + sizeof(int) * (n2m + 2));
+    const size_t o_rows = off; off = align256(off + sizeof(double4) * (n2m + 1));
     const size_t o_twx = off; off = align256(off + sizeof(double2) * n1m);
     const size_t o_twz = off; off = align256(off + sizeof(double2) * n3m);
     const size_t o_ccap = off; off = align256(off + sizeof(double2) * nspec);
@@ -204,25 +224,16 @@ extern "C" int lesgpu_poisson_ftft_noalloc(const lesgpu_grid *g, const double *d
     TableDst d;
     d.ak1 = (double *)(base + o_ak1);
     d.ak3 = (double *)(base + o_ak3);
-    d.f2fyi = (double *)(base + o_f2fyi);
-    d.c2cyi = (double *)(base + o_c2cyi);
-    d.jpv = (int *)(base + o_jpv);
-    d.fixjl = (int *)(base + o_fixjl);
-    d.fixju = (int *)(base + o_fixju);
+    d.rows = (double4 *)(base + o_rows);
     d.twx = (double2 *)(base + o_twx);
     d.twz = (double2 *)(base + o_twz);
-    k_noalloc_tables<<<(kMaxDir + 3 + 255) / 256, 256, 0, st>>>(y, d, n1m, n2m, n3m, g->f2fxi[1], g->f2fzi[1]);
+    k_noalloc_tables<<<dim3((std::max(n1m, std::max(n2m, n3m)) + 3 + 63) / 64, 5), 64, 0, st>>>(y, d, n1m, n2m, n3m, g->f2fxi[1], g->f2fzi[1]);
 
     lg::KP p;
     memset(&p, 0, sizeof(p));
     p.g.n1 = n1; p.g.n2 = n2; p.g.n3 = n3m + 1;
     p.g.n1m = n1m; p.g.n2m = n2m; p.g.n3m = n3m; p.g.n1mh = n1mh; p.g.n3mh = n3mh;
     p.g.sx = n1 + 1; p.g.sxy = p.g.sx * (n2 + 1); p.g.nt = p.g.sxy * (n3m + 2);
-    p.g.f2fyi = d.f2fyi;
-    p.g.c2cyi = d.c2cyi;
-    p.g.jpv = d.jpv;
-    p.g.fixjl = d.fixjl;
-    p.g.fixju = d.fixju;
     p.f.divgsum = (double *)d_divgsum;
     p.f.phi = d_phi;
     px.tw = d.twx;
@@ -233,7 +244,12 @@ extern "C" int lesgpu_poisson_ftft_noalloc(const lesgpu_grid *g, const double *d
     double *gam = (double *)(base + o_gam);
 
     // the same launch sequence as the case-based solve (k_fft.cu launch_poisson)
-    int Lz = lg::fft_lines_per_block(n3m), Lx = lg::fft_lines_per_block(n1m);
+    // Lines per block: four keep a block's shared memory small enough for
+    // several blocks an SM, so their transfers and FP64 stages overlap
+    // (128x125x120: 398 us with two, 361 with four, 367 with eight, 403 with
+    // sixteen, 490 with what fills the shared memory); fewer where that leaves
+    // SMs without a block.
+    const int Lz = lines(n3m, (n1m + 1) / 2, n2m), Lx = lines(n1m, n3mh * n2m, 1);
     size_t smz = (size_t)2 * n3m * Lz * sizeof(double2), smx = (size_t)2 * n1m * Lx * sizeof(double2);
     dim3 gz((n1m + 2 * Lz - 1) / (2 * Lz), n2m);   // 2 Lz real lines per block
     int nxl = n3mh * n2m;
@@ -241,7 +257,7 @@ extern "C" int lesgpu_poisson_ftft_noalloc(const lesgpu_grid *g, const double *d
     lg::fft_z_fwd64(gz, smz, st, p, p.f.divgsum, ccap, pz, Lz, sk, sj);
     lg::fft_x64((nxl + Lx - 1) / Lx, smx, st, ccap, nxl, px, Lx, 0);
     long long nl = (long long)n1m * n3mh;
-    lg::k_ytri_elim<<<lg::blocks_for(nl, 128), 128, 0, st>>>(p, ccap, d.ak1, d.ak3, gam);
+    lg::k_ytri_elim<<<lg::blocks_for((nl + 15) / 16 * 32, 64), 64, 0, st>>>(n1m, n2m, n3mh, ccap, d.ak1, d.ak3, d.rows, gam);
     lg::fft_x64((nxl + Lx - 1) / Lx, smx, st, ccap, nxl, px, Lx, 1);
     lg::fft_z_inv64(gz, smz, st, p, ccap, pz, Lz, sk, sj);
     // a launch that failed leaves its error pending; report it, leave it for the caller to see
