@@ -2,9 +2,9 @@
 // update: the routines of 02_solver/f90/lib/slv_auxi.f90, meanpg of
 // slv_mmtm.f90:2-177 and the checks of misc_init.f90:1047-1104.
 //
-// Every global sum is a two-stage deterministic reduction: a fixed grid of
-// kRedBlocks blocks strides over the cells in a fixed order, each block
-// writes its partials, and a one-block kernel folds them in a fixed tree and
+// Every global sum is a two-stage deterministic reduction: a grid whose size
+// depends on the box alone strides over the cells in a fixed order, each block
+// writes its partials, and the last block folds them in a fixed tree and
 // applies the scalar logic of the reference routine.  The result is the same
 // bit pattern on every run.
 #include "lesgpu_internal.cuh"
@@ -79,12 +79,12 @@ __global__ void k_zero_fcvavg(KP p) {
 
 void launch_stepinit(lesgpu_case *c) {
     if (c->kp.c.ibmon == 1) k_zero_fcvavg<<<64, kThreads, 0, c->stream>>>(c->kp);
-    reduce<1, true>(c, interior(c->kp.g), CflTerm{}, StepinitFinal{});
+    reduce<1, 1u>(c, interior(c->kp.g), CflTerm{}, StepinitFinal{});
 }
 
 // substepinit, slv_auxi.f90:105-123 (RK3 coefficients of rk3coefinit,
 // misc_init.f90:1031-1044)
-__global__ void k_substepinit(KP p, int s) {
+__global__ void k_substepinit(KP p, int s, int carry) {
     const double gam[4] = {0.0, 8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
     const double ro[4] = {0.0, 0.0, -17.0 / 60.0, -5.0 / 12.0};
     DScal *S = p.S;
@@ -96,9 +96,12 @@ __global__ void k_substepinit(KP p, int s) {
     S->acoefi = 1.0 / S->acoef;
     S->pmiavg = S->pmiavg + S->pmi[0] * 2.0 * S->alpha;
     S->subdt = S->subdt + S->dtconst;
+    if (carry) S->qvol[1] = S->qvol[0];
 }
 
-void launch_substepinit(lesgpu_case *c, int msub) { k_substepinit<<<1, 1, 0, c->stream>>>(c->kp, msub); }
+void launch_substepinit(lesgpu_case *c, int msub, bool carry) {
+    k_substepinit<<<1, 1, 0, c->stream>>>(c->kp, msub, carry ? 1 : 0);
+}
 
 // ------------------------------------------------------------ qvol / tvol
 struct QvolTerm {   // qvolcalc, slv_auxi.f90:126-149
@@ -111,7 +114,7 @@ struct QvolFinal {
     int slot;
     __device__ void operator()(const KP &p, const double *out) const { p.S->qvol[slot] = out[0]; }
 };
-void launch_qvolcalc(lesgpu_case *c, int slot) { reduce<1, false>(c, interior(c->kp.g), QvolTerm{}, QvolFinal{slot}); }
+void launch_qvolcalc(lesgpu_case *c, int slot) { reduce<1, 0u>(c, interior(c->kp.g), QvolTerm{}, QvolFinal{slot}); }
 
 struct TvolTerm {   // tvolcalc, slv_auxi.f90:152-173
     __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
@@ -123,7 +126,7 @@ struct TvolFinal {
     int slot;
     __device__ void operator()(const KP &p, const double *out) const { p.S->tvol[slot] = out[0]; }
 };
-void launch_tvolcalc(lesgpu_case *c, int slot) { reduce<1, false>(c, interior(c->kp.g), TvolTerm{}, TvolFinal{slot}); }
+void launch_tvolcalc(lesgpu_case *c, int slot) { reduce<1, 0u>(c, interior(c->kp.g), TvolTerm{}, TvolFinal{slot}); }
 
 // Weights of the volume reductions: the cell-volume products and fluid masks
 // of qvolcalc / meanpg (fb_u), the bulk velocity (fb_c) and tvolcalc (1/c*),
@@ -141,9 +144,28 @@ __global__ void k_red_weights(KP p, Box b) {
         p.f.wt[q] = g.f2fx[i] * g.f2fy[j] * g.f2fz[k] / p.f.cstar[q];
     }
 }
+// The volumes those weights sum to, which meanpg, the bulk velocity, the bulk
+// temperature and the mean eddy viscosity divide by: constant, so summed here
+// and not with every reduction.
+struct VolumeTerm {
+    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+        const long long q = p.g.ix(i, j, k);
+        w[0] = p.f.wq[q];
+        w[1] = p.f.wb[q];
+        w[2] = p.f.fb_c[q] >= 1.0e-10 ? p.g.f2fx[i] * p.g.f2fy[j] * p.g.f2fz[k] : 0.0;
+    }
+};
+struct VolumeFinal {
+    __device__ void operator()(const KP &p, const double *o) const {
+        p.S->flowvol = o[0];
+        p.S->cellvol = o[1];
+        p.S->fluidvol = o[2];
+    }
+};
 void launch_red_weights(lesgpu_case *c) {
     Box b = interior(c->kp.g);
     k_red_weights<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+    reduce<3, 0u>(c, b, VolumeTerm{}, VolumeFinal{});
 }
 
 // tvolcorr, slv_auxi.f90:206-230.  The volume integral of 1/c* does not
@@ -169,10 +191,27 @@ struct TvolCorrFinal {
         if (slot0) p.S->tvol[0] = out[0];
     }
 };
-void launch_tvolcalc_corr(lesgpu_case *c, bool slot0) {
-    reduce<1, false>(c, interior(c->kp.g), TvolTerm{}, TvolCorrFinal{slot0 ? 1 : 0});
+// the same with the fluid cells' temperature sum of writehistory
+struct TvolBulkTerm {
+    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+        const long long q = p.g.ix(i, j, k);
+        const double t = p.f.t[q];
+        w[0] = t * p.f.wt[q];
+        w[1] = t * p.f.wb[q];
+    }
+};
+struct TvolBulkFinal {
+    int slot0;
+    __device__ void operator()(const KP &p, const double *out) const {
+        TvolCorrFinal{slot0}(p, out);
+        p.S->tbulk_sum = out[1];
+    }
+};
+void launch_tvolcalc_corr(lesgpu_case *c, bool slot0, bool bulk) {
+    if (bulk) reduce<2, 0u>(c, interior(c->kp.g), TvolBulkTerm{}, TvolBulkFinal{slot0 ? 1 : 0});
+    else reduce<1, 0u>(c, interior(c->kp.g), TvolTerm{}, TvolCorrFinal{slot0 ? 1 : 0});
 }
-void launch_cvol(lesgpu_case *c) { reduce<1, false>(c, interior(c->kp.g), CvolTerm{}, CvolFinal{}); }
+void launch_cvol(lesgpu_case *c) { reduce<1, 0u>(c, interior(c->kp.g), CvolTerm{}, CvolFinal{}); }
 
 // tcalc, slv_auxi.f90:496-516
 __global__ void k_tcalc(KP p, Box b) {
@@ -191,18 +230,10 @@ void launch_tcalc(lesgpu_case *c) {
 }
 
 // ------------------------------------------------------------------ meanpg
-// Two passes: flow volume and flow rate over every cell, and the four
-// wall-shear sums over the planes next to no-slip walls only (the terms are
-// zero elsewhere; carrying them through the volume pass cost it two thirds
-// of its time).  The wall pass runs first and leaves its sums in pmiw.
-struct MeanpgTerm {
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
-        const long long q = p.g.ix(i, j, k);
-        const double vol = p.f.wq[q];    // c2cx f2fy f2fz over the fluid u points, else 0
-        w[0] = vol;
-        w[1] = p.f.u[q] * vol;
-    }
-};
+// The flow rate -- the projection's where it has just formed it with qvol(0)
+// (ICH = 1), else a pass of its own; only ICH = 1 reads it -- and the four
+// wall-shear sums over the planes next to no-slip walls only.  The wall pass
+// runs last and finishes the update.
 // Box (i, plane, c): plane 0 / 1 = the y-bottom / top wall (j = 1 / n2m,
 // k = c), 2 / 3 = the z-bottom / top wall (k = 1 / n3m, j = c); c beyond the
 // plane's extent contributes nothing.  A cell on two walls is visited once
@@ -225,28 +256,11 @@ struct MeanpgWallTerm {
         }
         const long long q = g.ix(i, j, k);
         if (p.f.fb_u[q] < 1.0e-10) return;
-        if (plane == 0) {
-            double dy1 = 1.0 / g.c2cyi[1], dy2 = dy1 + 1.0 / g.c2cyi[2];
-            double gu = (u[q] * (dy2 * dy2) - u[q + g.sx] * (dy1 * dy1)) / (dy1 * dy2 * (dy2 - dy1));
-            w[0] = gu * g.c2cx[i] * g.f2fz[k] / c.re;
-        } else if (plane == 1) {
-            double dy1 = 1.0 / g.c2cyi[g.n2], dy2 = dy1 + 1.0 / g.c2cyi[g.n2m];
-            double gu = (u[q] * (dy2 * dy2) - u[q - g.sx] * (dy1 * dy1)) / (dy1 * dy2 * (dy2 - dy1));
-            w[1] = gu * g.c2cx[i] * g.f2fz[k] / c.re;
-        } else if (plane == 2) {
-            double dz1 = 1.0 / g.c2czi[1], dz2 = dz1 + 1.0 / g.c2czi[2];
-            double gu = (u[q] * (dz2 * dz2) - u[q + g.sxy] * (dz1 * dz1)) / (dz1 * dz2 * (dz2 - dz1));
-            w[2] = gu * g.c2cx[i] * g.f2fy[j] / c.re;
-        } else {
-            double dz1 = 1.0 / g.c2czi[g.n3], dz2 = dz1 + 1.0 / g.c2czi[g.n3m];
-            double gu = (u[q] * (dz2 * dz2) - u[q - g.sxy] * (dz1 * dz1)) / (dz1 * dz2 * (dz2 - dz1));
-            w[3] = gu * g.c2cx[i] * g.f2fy[j] / c.re;
-        }
-    }
-};
-struct MeanpgWallFinal {
-    __device__ void operator()(const KP &p, const double *o) const {
-        for (int q = 0; q < 4; q++) p.S->pmiw[q] = o[q];
+        // the one-sided second-order wall gradient over re, its two weights
+        // formed once on the host (per cell they cost four divisions)
+        const long long in = plane == 0 ? g.sx : plane == 1 ? -g.sx : plane == 2 ? g.sxy : -g.sxy;
+        const double gu = c.wall_a[plane] * u[q] - c.wall_b[plane] * u[q + in];
+        w[plane] = gu * (g.c2cx[i] * (plane <= 1 ? g.f2fz[k] : g.f2fy[j]));
     }
 };
 
@@ -258,26 +272,26 @@ __global__ void k_meanpg_ibm(KP p) {
         int m = t + 1;
         v[0] += p.f.fcv[0][m] * p.g.c2cx[p.f.ifc[0][m]] * p.g.f2fy[p.f.jfc[0][m]] * p.g.f2fz[p.f.kfc[0][m]];
     }
-    block_reduce<1, false>(v);
+    block_totals<1, 0u>(v);
     if (threadIdx.x == 0) p.f.part[(size_t)kRedBlocks * kMaxRed] = v[0];
 }
 
+struct FlowFinal {
+    __device__ void operator()(const KP &p, const double *o) const { p.S->qcur = o[0]; }
+};
 struct MeanpgFinal {
     __device__ void operator()(const KP &p, const double *o) const {
         DScal *S = p.S;
         const DCfg &c = p.c;
-        double flowvol = o[0], qcur = o[1];
-        double ubulk = flowvol > 0.0 ? qcur / flowvol : 0.0;
-        for (int q = 0; q < 5; q++) S->pmi[q] = 0.0;
-        if (c.bc_ybtm == 0) S->pmi[1] += S->pmiw[0];
-        if (c.bc_ytop == 0) S->pmi[2] += S->pmiw[1];
-        if (c.bc_zbtm == 0) S->pmi[3] += S->pmiw[2];
-        if (c.bc_ztop == 0) S->pmi[4] += S->pmiw[3];
-        S->pmi[0] = S->pmi[1] + S->pmi[2] + S->pmi[3] + S->pmi[4];
+        for (int q = 0; q < 4; q++) S->pmiw[q] = o[q];
+        const double qcur = S->qcur;
+        double ubulk = S->flowvol > 0.0 ? qcur / S->flowvol : 0.0;
+        double pm[5] = {0.0, c.bc_ybtm == 0 ? o[0] : 0.0, c.bc_ytop == 0 ? o[1] : 0.0, c.bc_zbtm == 0 ? o[2] : 0.0,
+                        c.bc_ztop == 0 ? o[3] : 0.0};
+        pm[0] = pm[1] + pm[2] + pm[3] + pm[4];
         double ibm = (c.nbody[0] > 0) ? p.f.part[(size_t)kRedBlocks * kMaxRed] : 0.0;
-        S->pmi[0] = S->pmi[0] + ibm;
-        double volume = p.g.xl * p.g.yl * p.g.zl;
-        for (int q = 0; q < 5; q++) S->pmi[q] = S->pmi[q] / volume;
+        pm[0] = pm[0] + ibm;
+        for (int q = 0; q < 5; q++) S->pmi[q] = pm[q] * c.ivol;
         if (c.ich == 0) {
             S->pmi[0] = 0.0;
         } else if (c.ich == 1) {
@@ -292,11 +306,11 @@ struct MeanpgFinal {
     }
 };
 
-void launch_meanpg(lesgpu_case *c) {
+void launch_meanpg(lesgpu_case *c, bool have_q) {
     const DGrid &g = c->kp.g;
     if (c->kp.c.nbody[0] > 0) k_meanpg_ibm<<<1, kThreads, 0, c->stream>>>(c->kp);
-    reduce<4, false>(c, Box{1, 0, 1, g.n1m, 4, g.n2m > g.n3m ? g.n2m : g.n3m}, MeanpgWallTerm{}, MeanpgWallFinal{});
-    reduce<2, false>(c, interior(g), MeanpgTerm{}, MeanpgFinal{});
+    if (!have_q && c->kp.c.ich == 1) reduce<1, 0u>(c, interior(g), QvolTerm{}, FlowFinal{});
+    reduce<4, 0u>(c, Box{1, 0, 1, g.n1m, 4, g.n2m > g.n3m ? g.n2m : g.n3m}, MeanpgWallTerm{}, MeanpgFinal{});
 }
 
 // ------------------------------------------------------------------- ucalc
@@ -382,12 +396,15 @@ struct UcalcQvolTerm {
     }
 };
 struct UcalcQvolFinal {
-    __device__ void operator()(const KP &p, const double *o) const { p.S->qvol[2] = o[0]; p.S->qvol[0] = o[1]; }
+    __device__ void operator()(const KP &p, const double *o) const {
+        p.S->qvol[2] = o[0];
+        p.S->qvol[0] = p.S->qcur = o[1];
+    }
 };
 
 static void ucalc_interior(lesgpu_case *c, bool with_qvol) {
     Box b = interior(c->kp.g);
-    if (with_qvol) reduce<2, false>(c, b, UcalcQvolTerm{}, UcalcQvolFinal{});
+    if (with_qvol) reduce<2, 0u>(c, b, UcalcQvolTerm{}, UcalcQvolFinal{});
     else k_ucalc<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
 }
 
@@ -442,7 +459,7 @@ __global__ void __launch_bounds__(kThreads) k_pcalc(KP p, Box b) {
 void launch_ucalc_pcalc(lesgpu_case *c, bool with_qvol) {
     const DGrid &g = c->kp.g;
     ucalc_interior(c, with_qvol);
-    reduce<1, false>(c, Box{1, 1, 1, 1, g.n2m, g.n3m}, PhirefTerm{}, PhirefFinal{});
+    reduce<1, 0u>(c, Box{1, 1, 1, 1, g.n2m, g.n3m}, PhirefTerm{}, PhirefFinal{});
     Box b = interior(g);
     k_pcalc<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
     DFields &f = c->kp.f;
@@ -481,25 +498,33 @@ struct DivFinal {
         if (o[2] > 0.0 || !isfinite(o[0])) p.S->err |= 2;
     }
 };
-void launch_advance_and_convergence(lesgpu_case *c) { reduce<3, true>(c, interior(c->kp.g), DivTerm{}, DivFinal{}); }
+void launch_advance_and_convergence(lesgpu_case *c) { reduce<3, 7u>(c, interior(c->kp.g), DivTerm{}, DivFinal{}); }
 
-// writehistory's bulk quantities, misc_hist.f90:73-181: the flow rate and
-// the fluid cells' temperature sums in one pass; the solid cells' sums
-// (temperature inside bodies) in a second pass only when some cell centre
-// lies inside a body -- carried through one pass they cost it half its time
-// on bodiless cases, where they are zero.
+// writehistory's bulk quantities, misc_hist.f90:73-181: the flow rate and the
+// fluid cells' temperature sum where the step has not formed them already (the
+// volumes are constants), then the scalars; the solid cells' sums
+// (temperature inside bodies) in a pass of their own only when some cell
+// centre lies inside a body.
 struct BulkTerm {
     __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
-        const DGrid &g = p.g;
-        long long q = g.ix(i, j, k);
-        double cv = g.c2cx[i] * g.f2fy[j] * g.f2fz[k];
-        bool flu = p.f.fb_u[q] >= 1.0e-10;
-        w[0] = flu ? p.f.u[q] * cv : 0.0;
-        w[1] = flu ? cv : 0.0;
-        w[2] = w[3] = 0.0;
-        if (p.c.ihtrans == 1 && p.f.fb_c[q] >= 1.0e-10) { w[2] = cv; w[3] = p.f.t[q] * cv; }
+        const long long q = p.g.ix(i, j, k);
+        w[0] = p.f.u[q] * p.f.wq[q];
+        w[1] = p.c.ihtrans == 1 ? p.f.t[q] * p.f.wb[q] : 0.0;
     }
 };
+struct BulkTTerm {
+    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+        const long long q = p.g.ix(i, j, k);
+        w[0] = p.f.t[q] * p.f.wb[q];
+    }
+};
+__device__ __forceinline__ void bulk_scalars(const KP &p, double q, double t, int solid) {
+    DScal *S = p.S;
+    S->ubulk = S->flowvol > 0.0 ? q / S->flowvol : 0.0;
+    S->qflux = q / p.g.xl;
+    S->tbulk_fluid = p.c.ihtrans == 1 && S->cellvol > 0.0 ? t / S->cellvol : 0.0;
+    if (!solid) S->tbulk_solid = 0.0;
+}
 struct BulkSolidTerm {
     __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
         const DGrid &g = p.g;
@@ -514,23 +539,25 @@ struct BulkSolidTerm {
 };
 struct BulkFinal {
     int solid;      // the solid pass follows (else the solid bulk temperature is 0)
-    __device__ void operator()(const KP &p, const double *o) const {
-        DScal *S = p.S;
-        S->ubulk = o[1] > 0.0 ? o[0] / o[1] : 0.0;
-        S->qflux = o[0] / p.g.xl;
-        S->tbulk_fluid = o[2] > 0.0 ? o[3] / o[2] : 0.0;
-        if (!solid) S->tbulk_solid = 0.0;
-    }
+    __device__ void operator()(const KP &p, const double *o) const { bulk_scalars(p, o[0], o[1], solid); }
 };
+struct BulkTFinal {
+    int solid;
+    __device__ void operator()(const KP &p, const double *o) const { bulk_scalars(p, p.S->qcur, o[0], solid); }
+};
+__global__ void k_bulk_scalars(KP p, int solid) { bulk_scalars(p, p.S->qcur, p.S->tbulk_sum, solid); }
 struct BulkSolidFinal {
     __device__ void operator()(const KP &p, const double *o) const {
         p.S->tbulk_solid = o[0] > 0.0 ? o[1] / o[0] : 0.0;
     }
 };
-void launch_bulk_diag(lesgpu_case *c) {
+void launch_bulk_diag(lesgpu_case *c, bool have_q, bool have_t) {
     const bool solid = c->kp.c.ihtrans == 1 && c->bulk_solid;
-    reduce<4, false>(c, interior(c->kp.g), BulkTerm{}, BulkFinal{solid ? 1 : 0});
-    if (solid) reduce<2, false>(c, interior(c->kp.g), BulkSolidTerm{}, BulkSolidFinal{});
+    const int sl = solid ? 1 : 0;
+    if (have_q && (have_t || c->kp.c.ihtrans != 1)) k_bulk_scalars<<<1, 1, 0, c->stream>>>(c->kp, sl);
+    else if (have_q) reduce<1, 0u>(c, interior(c->kp.g), BulkTTerm{}, BulkTFinal{sl});
+    else reduce<2, 0u>(c, interior(c->kp.g), BulkTerm{}, BulkFinal{sl});
+    if (solid) reduce<2, 0u>(c, interior(c->kp.g), BulkSolidTerm{}, BulkSolidFinal{});
 }
 
 

@@ -9,21 +9,24 @@ namespace lg {
 struct UbulkTerm {
     __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
         const long long q = p.g.ix(i, j, k);
-        const double cv = p.f.wb[q];     // c2cx f2fy f2fz over the fluid cells, else 0
-        w[0] = cv;
-        w[1] = 0.5 * (p.f.u[q] + p.f.u[q + 1]) * cv;
+        w[0] = 0.5 * (p.f.u[q] + p.f.u[q + 1]) * p.f.wb[q];     // c2cx f2fy f2fz over the fluid cells, else 0
     }
 };
 struct UbulkFinal {
+    int carry;      // tvol(1) is tvol(0) of the substep before
     __device__ void operator()(const KP &p, const double *o) const {
         double ub;
-        if (o[0] > 1.0e-12) ub = o[1] / o[0];
+        if (p.S->cellvol > 1.0e-12) ub = o[0] / p.S->cellvol;
         else if (fabs(p.c.udrv_i) > 1.0e-12) ub = p.c.udrv_i;
         else ub = 1.0;
         p.S->u_bulk_t = ub;
+        if (carry) p.S->tvol[1] = p.S->tvol[0];
     }
 };
-__global__ void k_set_ubulk_one(KP p) { p.S->u_bulk_t = 1.0; }
+__global__ void k_set_ubulk_one(KP p, int carry) {
+    p.S->u_bulk_t = 1.0;
+    if (carry) p.S->tvol[1] = p.S->tvol[0];
+}
 
 // tvolcalc(tvol(1)) and the bulk velocity in one reduction (both read every
 // interior cell; each sum keeps the order of its own launch, bitwise)
@@ -37,19 +40,19 @@ struct TvolUbulkTerm {
 struct TvolUbulkFinal {
     __device__ void operator()(const KP &p, const double *o) const {
         p.S->tvol[1] = o[0];
-        UbulkFinal{}(p, o + 1);
+        UbulkFinal{0}(p, o + 1);
     }
 };
 
-void launch_rhs_t(lesgpu_case *c, int msub, bool with_tvol) {
+void launch_rhs_t(lesgpu_case *c, int msub, int tvol) {
     const DGrid &g = c->kp.g;
     const Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     if (c->kp.c.idecomp == 1) {
-        if (with_tvol) reduce<3, false>(c, b, TvolUbulkTerm{}, TvolUbulkFinal{});
-        else reduce<2, false>(c, b, UbulkTerm{}, UbulkFinal{});
+        if (tvol == 1) reduce<2, 0u>(c, b, TvolUbulkTerm{}, TvolUbulkFinal{});
+        else reduce<1, 0u>(c, b, UbulkTerm{}, UbulkFinal{tvol == 2 ? 1 : 0});
     } else {
-        if (with_tvol) launch_tvolcalc(c, 1);
-        k_set_ubulk_one<<<1, 1, 0, c->stream>>>(c->kp);
+        if (tvol == 1) launch_tvolcalc(c, 1);
+        k_set_ubulk_one<<<1, 1, 0, c->stream>>>(c->kp, tvol == 2 ? 1 : 0);
     }
     launch_rhs_t_kernel(c, msub);
 }
@@ -144,7 +147,7 @@ void launch_energy_bc(lesgpu_case *c) {
             GhostSpec s[1] = {{t, 0, g.n2, 0, g.n3}};
             ghost(c, 0, s, 1);
         } else {
-            reduce<2, false>(c, Box{1, 1, 1, 1, g.n2m, g.n3m}, RecycTerm{}, RecycFinal{});
+            reduce<2, 0u>(c, Box{1, 1, 1, 1, g.n2m, g.n3m}, RecycTerm{}, RecycFinal{});
             k_recyc_apply<<<blocks_for((long long)(g.n2 + 1) * (g.n3 + 1)), kThreads, 0, c->stream>>>(c->kp);
         }
     }

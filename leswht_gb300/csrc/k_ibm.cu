@@ -173,7 +173,7 @@ static Box ibm_box(const lesgpu_case *c) {
 void launch_lagforce(lesgpu_case *c, int msub) {
     const double gam[4] = {0.0, 8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
     const double ro[4] = {0.0, 0.0, -17.0 / 60.0, -5.0 / 12.0};
-    reduce<3, false>(c, ibm_box(c), LagTerm{gam[msub], ro[msub]}, LagFinal{msub});
+    reduce<3, 0u>(c, ibm_box(c), LagTerm{gam[msub], ro[msub]}, LagFinal{msub});
 }
 
 // draglift, slv_auxi.f90:666-840: IB forcing integral + inertia, then the
@@ -261,11 +261,11 @@ struct HeatIbFinal {
 
 void launch_draglift(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
-    reduce<3, false>(c, ibm_box(c), DragIbTerm{}, DragIbFinal{});
+    reduce<3, 0u>(c, ibm_box(c), DragIbTerm{}, DragIbFinal{});
     if (c->kp.c.ihtrans == 1 && c->kp.c.nbody[3] > 0)
-        reduce<1, false>(c, Box{0, 0, 0, c->kp.c.nbody[3], 1, 1}, HeatIbTerm{}, HeatIbFinal{});
+        reduce<1, 0u>(c, Box{0, 0, 0, c->kp.c.nbody[3], 1, 1}, HeatIbTerm{}, HeatIbFinal{});
     Box faces{0, 0, 0, 2 * g.n1m * g.n3m + 2 * g.n1m * g.n2m, 1, 1};
-    reduce<3, false>(c, faces, WallShearTerm{}, DragFinal{});
+    reduce<3, 0u>(c, faces, WallShearTerm{}, DragFinal{});
 }
 
 // heatflux, slv_auxi.f90:573-663: convective heat flux through the six
@@ -325,7 +325,7 @@ struct HeatFluxFinal {
 void launch_heatflux(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     Box faces{0, 0, 0, 2 * (g.n2m * g.n3m + g.n1m * g.n3m + g.n1m * g.n2m), 1, 1};
-    reduce<6, false>(c, faces, HeatFluxTerm{}, HeatFluxFinal{});
+    reduce<6, 0u>(c, faces, HeatFluxTerm{}, HeatFluxFinal{});
 }
 
 }  // namespace lg

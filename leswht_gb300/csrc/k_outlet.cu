@@ -168,9 +168,9 @@ static void outlet(lesgpu_case *c, int thermal) {
     // create on and nothing else writes them
     if (cf.ich == 1) return;
     const long long nplane = (long long)g.n2m * g.n3m;
-    reduce<2, false>(c, Box{0, 0, 0, (int)(nplane + (long long)g.n1m * g.n3m + (long long)g.n1m * g.n2m), 1, 1},
+    reduce<2, 0u>(c, Box{0, 0, 0, (int)(nplane + (long long)g.n1m * g.n3m + (long long)g.n1m * g.n2m), 1, 1},
                      OutletQTerm{}, OutletQFinal{});
-    reduce<1, false>(c, Box{0, 0, 0, (int)nplane, 1, 1}, OutletOutTerm{thermal}, OutletOutFinal{thermal});
+    reduce<1, 0u>(c, Box{0, 0, 0, (int)nplane, 1, 1}, OutletOutTerm{thermal}, OutletOutFinal{thermal});
     k_outlet_scale<<<blocks_for(nplane), kThreads, 0, c->stream>>>(c->kp, thermal);
     if (cf.yprdic == 1) k_outlet_ghost<<<blocks_for(g.n3 + 1), kThreads, 0, c->stream>>>(c->kp, thermal, 1);
     if (cf.zprdic == 1) k_outlet_ghost<<<blocks_for(g.n2 + 1), kThreads, 0, c->stream>>>(c->kp, thermal, 2);

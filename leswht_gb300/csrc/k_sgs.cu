@@ -304,41 +304,26 @@ __global__ void k_zero_list(KP p, double *f) {
 }
 
 // nutzero / alpzero statistics with the in-body zeroing (sgs.f90:898-925)
-struct ZeroSumTerm {
+struct ZeroTerm {
     double *f;
     __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
         long long q = p.g.ix(i, j, k);
+        w[0] = w[1] = 0.0;
         if (p.f.fb_c[q] >= 1.0e-10) {
-            double vol = p.g.f2fx[i] * p.g.f2fy[j] * p.g.f2fz[k];
-            w[0] = f[q] * vol;
-            w[1] = vol;
+            const double x = f[q];
+            w[0] = x * (p.g.f2fx[i] * p.g.f2fy[j] * p.g.f2fz[k]);
+            w[1] = max_bits(x, 0.0);
         } else {
             f[q] = 0.0;
-            w[0] = 0.0;
-            w[1] = 0.0;
         }
     }
 };
-struct ZeroMaxTerm {
-    const double *f;
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
-        long long q = p.g.ix(i, j, k);
-        w[0] = (p.f.fb_c[q] >= 1.0e-10) ? fmax(f[q], 0.0) : 0.0;
-    }
-};
-struct ZeroSumFinal {
+struct ZeroFinal {
     int thermal;
     __device__ void operator()(const KP &p, const double *o) const {
-        double avg = o[0] / o[1];
-        if (thermal) p.S->alpavg = avg * p.c.re * p.c.pr;
-        else p.S->nutavg = avg * p.c.re;
-    }
-};
-struct ZeroMaxFinal {
-    int thermal;
-    __device__ void operator()(const KP &p, const double *o) const {
-        if (thermal) p.S->alpmax = o[0] * p.c.re * p.c.pr;
-        else p.S->nutmax = o[0] * p.c.re;
+        const double avg = o[0] / p.S->fluidvol;
+        if (thermal) { p.S->alpavg = avg * p.c.re * p.c.pr; p.S->alpmax = o[1] * p.c.re * p.c.pr; }
+        else { p.S->nutavg = avg * p.c.re; p.S->nutmax = o[1] * p.c.re; }
     }
 };
 
@@ -459,8 +444,7 @@ static void zero_in_body(lesgpu_case *c, double *f, int thermal) {
     const DGrid &g = c->kp.g;
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     if (c->kp.c.nzero > 0) k_zero_list<<<blocks_for(c->kp.c.nzero), kThreads, 0, c->stream>>>(c->kp, f);
-    reduce<2, false>(c, b, ZeroSumTerm{f}, ZeroSumFinal{thermal});
-    reduce<1, true>(c, b, ZeroMaxTerm{f}, ZeroMaxFinal{thermal});
+    reduce<2, 2u>(c, b, ZeroTerm{f}, ZeroFinal{thermal});
 }
 
 void launch_sgs_zero_first(lesgpu_case *c, int thermal) {
@@ -487,8 +471,8 @@ void launch_sgs(lesgpu_case *c) {
         G.na = 9;
         for (int m = 0; m < 9; m++) { G.src[m] = f.scr[3 + m]; G.dst[m] = f.scr[24 + m]; }
         filter_batch(c, G);
-        if (mixed(c)) reduce<2, false>(c, b, LmMmTerm<float>{}, CsgstsFinal{});
-        else reduce<2, false>(c, b, LmMmTerm<double>{}, CsgstsFinal{});
+        if (mixed(c)) reduce<2, 0u>(c, b, LmMmTerm<float>{}, CsgstsFinal{});
+        else reduce<2, 0u>(c, b, LmMmTerm<double>{}, CsgstsFinal{});
         k_scale<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, f.nusgs, 0);
     } else {
         if (mixed(c)) k_vreman1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
@@ -607,8 +591,8 @@ void launch_sgs_t(lesgpu_case *c) {
         G.na = 7;
         for (int m = 0; m < 7; m++) { G.src[m] = f.scr[3 + m]; G.dst[m] = f.scr[24 + m]; }
         filter_batch(c, G);
-        if (mixed(c)) reduce<2, false>(c, b, LmMmTTerm<float>{}, CsgshfFinal{});
-        else reduce<2, false>(c, b, LmMmTTerm<double>{}, CsgshfFinal{});
+        if (mixed(c)) reduce<2, 0u>(c, b, LmMmTTerm<float>{}, CsgshfFinal{});
+        else reduce<2, 0u>(c, b, LmMmTTerm<double>{}, CsgshfFinal{});
         k_scale<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, f.alsgs, 1);
     } else {
         if (mixed(c)) k_edm1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);

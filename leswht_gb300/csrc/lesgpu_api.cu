@@ -269,6 +269,17 @@ extern "C" int lesgpu_create(const lesgpu_config *cfg, const lesgpu_grid *g, les
         k.rei_d = 1.0 / re; k.rei_f = (float)(1.0 / re);
         k.inv_repr_d = 1.0 / (re * pr); k.inv_repr_f = (float)(1.0 / (re * pr));
         k.gterm = cfg->gr / (re * re);
+        k.ivol = 1.0 / (g->xl * g->yl * g->zl);
+        // the gradient at a wall from the first two points, d1 and d2 away
+        auto wall = [&](int q, double ci1, double ci2) {
+            const double d1 = 1.0 / ci1, d2 = d1 + 1.0 / ci2, den = d1 * d2 * (d2 - d1) * re;
+            k.wall_a[q] = d2 * d2 / den;
+            k.wall_b[q] = d1 * d1 / den;
+        };
+        wall(0, g->c2cyi[1], g->c2cyi[2]);
+        wall(1, g->c2cyi[g->n2], g->c2cyi[g->n2m]);
+        wall(2, g->c2czi[1], g->c2czi[g->n3m > 1 ? 2 : 1]);
+        wall(3, g->c2czi[g->n3], g->c2czi[g->n3m]);
         k.adi_cd[0] = iles * re; k.adi_cd[1] = 2.0 * iles * re; k.adi_cd[2] = iles * re * pr;
         k.adi_cf[0] = (float)(iles * re_f); k.adi_cf[1] = (float)(2.0 * iles * re_f); k.adi_cf[2] = (float)(iles * re_f * pr);
     }
@@ -736,10 +747,13 @@ static void enqueue_rhsnlhs(lesgpu_case *c, int msub) {
     mark_mirror(c, kMirVel);
 }
 
-static void enqueue_energy(lesgpu_case *c, int msub) {
+// in_step: the phases before it are this step's, so sums that cannot have
+// changed since are taken over instead of formed again (substeps 2 and 3 start
+// from the t and u the one before them left)
+static void enqueue_energy(lesgpu_case *c, int msub, bool in_step) {
     const lesgpu_config &g = c->cfg;
     launch_mirror(c, kMirVel | kMirT);     // the projected velocity
-    launch_rhs_t(c, msub, g.ich == 1);              // with tvolcalc(tvol(1)) when ICH = 1
+    launch_rhs_t(c, msub, g.ich != 1 ? 0 : in_step && msub > 1 ? 2 : 1);     // with tvolcalc(tvol(1)) when ICH = 1
     if (g.ibmon != 0 && g.iconjg == 0) launch_rhs_ibm_t(c);
     launch_convbc_t(c);
     launch_adi_t(c);
@@ -747,7 +761,7 @@ static void enqueue_energy(lesgpu_case *c, int msub) {
     // tvolcalc(tvol(2)) + tvolcorr; tcalc changes t only when x is not
     // periodic, otherwise tvolcalc(tvol(0)) is the same sum
     const bool tcalc_runs = g.ich == 1 && g.xprdic == 0;
-    if (g.ich == 1) launch_tvolcalc_corr(c, !tcalc_runs);
+    if (g.ich == 1) launch_tvolcalc_corr(c, !tcalc_runs, in_step && msub == 3 && !tcalc_runs);
     launch_tcalc(c);
     if (tcalc_runs) launch_tvolcalc(c, 0);
     mark_mirror(c, kMirT);
@@ -759,8 +773,8 @@ static void enqueue_energy(lesgpu_case *c, int msub) {
 static void enqueue_substep_pre(lesgpu_case *c, int msub, bool first) {
     const lesgpu_config &g = c->cfg;
     if (msub == 1) launch_stepinit(c);
-    launch_substepinit(c, msub);
-    if (g.ich == 1) launch_qvolcalc(c, 1);
+    launch_substepinit(c, msub, g.ich == 1 && msub > 1);
+    if (g.ich == 1 && msub == 1) launch_qvolcalc(c, 1);
     if (g.iles == 1 && msub == 1) enqueue_sgs(c, first);
     enqueue_rhsnlhs(c, msub);
     launch_divgs(c);
@@ -770,12 +784,12 @@ static void enqueue_substep_post(lesgpu_case *c, int msub) {
     const lesgpu_config &g = c->cfg;
     launch_ucalc_pcalc(c, g.ich == 1);        // qvolcalc(qvol(2)), ucalc, qvolcalc(qvol(0)), pcalc
     mark_mirror(c, kMirVel | kMirP);
-    if (g.ich != 0) launch_meanpg(c);
+    if (g.ich != 0) launch_meanpg(c, g.ich == 1);
     if (g.ibmon == 1) launch_lagforce(c, msub);
-    if (g.ihtrans == 1) enqueue_energy(c, msub);
+    if (g.ihtrans == 1) enqueue_energy(c, msub, true);
     if (msub == 3) {
         launch_advance_and_convergence(c);          // time += dt, convergence_check
-        launch_bulk_diag(c);
+        launch_bulk_diag(c, g.ich == 1, g.ich == 1 && g.xprdic == 1);
         if (g.ibmon == 1) launch_draglift(c);
         if (g.ihtrans == 1) launch_heatflux(c);
         if (g.iavg == 1) launch_field_avg(c);
@@ -1193,7 +1207,7 @@ extern "C" int lesgpu_run_phase(lesgpu_case *c, int64_t phase, int64_t msub) {
         launch_ucalc_pcalc(c, g.ich == 1);        // qvolcalc(qvol(2)), ucalc, qvolcalc(qvol(0)), pcalc
         break;
     case LESGPU_PH_MEANPG: if (g.ich != 0) launch_meanpg(c); break;
-    case LESGPU_PH_ENERGY: if (g.ihtrans == 1) enqueue_energy(c, (int)msub); break;
+    case LESGPU_PH_ENERGY: if (g.ihtrans == 1) enqueue_energy(c, (int)msub, false); break;
     default: return LESGPU_ERR_ARG;
     }
     return cuda_rc(cudaStreamSynchronize(c->stream));

@@ -52,6 +52,8 @@ struct DCfg {
     // value (FP64 arithmetic on the FP32-rounded re, then rounded)
     double rei_d, inv_repr_d, gterm;   // 1/re, 1/(re pr), gr/re^2
     float rei_f, inv_repr_f;
+    double ivol;                        // 1 / (xl yl zl)
+    double wall_a[4], wall_b[4];        // meanpg's one-sided wall gradients / re: a u(wall) - b u(next), y bottom, y top, z bottom, z top
     double adi_cd[3];                   // ADI: iles re, 2 iles re, iles re pr
     float adi_cf[3];
 };
@@ -65,6 +67,11 @@ struct DScal {
     double alpha, dtconst, dtconsti, test1, acoef, acoefi;
     double pmi[5], pmiavg, qvol[3], tvol[3], thcap;
     double pmiw[4];           // meanpg's wall-shear sums (y bottom, y top, z bottom, z top)
+    // volumes of the fluid, summed once (launch_red_weights): u points and cells
+    // with the flow-rate weights, cells with f2fx f2fy f2fz
+    double flowvol, cellvol, fluidvol;
+    double qcur;              // flow rate of the projected u (qvol(0) under ICH = 1)
+    double tbulk_sum;         // sum of t over the fluid cells (writehistory)
     double csgsts, csgshf, nutavg, nutmax, alpavg, alpmax;
     double err_integral;
     double dudta, dvdta, dwdta;
@@ -271,33 +278,47 @@ inline int blocks_for(long long n, int threads = kThreads) {
     return (int)b;
 }
 
-// Deterministic block reduction of NV doubles (sum or max); result valid in thread 0.
-template <int NV, bool MAX>
-__device__ __forceinline__ void block_reduce(double (&v)[NV]) {
-    __shared__ double sh[NV][kThreads / 32];
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// The larger of two doubles on their bit patterns, a NaN passed over as fmax
+// does: a comparison on the FP64 pipe takes a warp 64 clocks on GB300.
+__device__ __forceinline__ double max_bits(double a, double b) {
+    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
+    constexpr long long kAbs = 0x7fffffffffffffffLL, kInf = 0x7ff0000000000000LL;
+    const long long ka = ia ^ ((ia >> 63) & kAbs), kb = ib ^ ((ib >> 63) & kAbs);
+    const bool na = (ia & kAbs) > kInf, nb = (ib & kAbs) > kInf;
+    return (nb || (!na && ka >= kb)) ? a : b;
+}
+
+// Deterministic block totals of NV doubles (the sum, or the maximum for the
+// values in MAXM); every thread gets them.  Warp q totals value q: eight
+// partials a lane, then a shuffle tree -- twelve dependent FP64 operations
+// whatever NV, where a tree of every value in every warp took fifteen NV.
+template <int NV, unsigned MAXM>
+__device__ __forceinline__ void block_totals(double (&v)[NV]) {
+    __shared__ double sh[NV][kThreads];
+    __shared__ double tot[NV];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int q = 0; q < NV; q++) {
-        double x = v[q];
+    for (int q = 0; q < NV; q++) sh[q][threadIdx.x] = v[q];
+    __syncthreads();
+    if (wid < NV) {
+        const bool mx = (MAXM >> wid) & 1u;
+        double x = sh[wid][lane];
+#pragma unroll
+        for (int w = 1; w < kThreads / 32; w++) {
+            const double y = sh[wid][lane + 32 * w];
+            if (mx) x = max_bits(x, y);
+            else x = x + y;
+        }
         for (int o = 16; o > 0; o >>= 1) {
-            double y = __shfl_down_sync(0xffffffffu, x, o);
-            x = MAX ? fmax(x, y) : x + y;
+            const double y = __shfl_down_sync(0xffffffffu, x, o);
+            if (mx) x = max_bits(x, y);
+            else x = x + y;
         }
-        if (lane == 0) sh[q][wid] = x;
+        if (lane == 0) tot[wid] = x;
     }
     __syncthreads();
-    if (wid == 0) {
 #pragma unroll
-        for (int q = 0; q < NV; q++) {
-            double x = (lane < (int)(blockDim.x >> 5)) ? sh[q][lane] : (MAX ? -1.0e308 : 0.0);
-            for (int o = 16; o > 0; o >>= 1) {
-                double y = __shfl_down_sync(0xffffffffu, x, o);
-                x = MAX ? fmax(x, y) : x + y;
-            }
-            v[q] = x;
-        }
-    }
-    __syncthreads();
+    for (int q = 0; q < NV; q++) v[q] = tot[q];
 }
 
 }  // namespace lg
@@ -357,22 +378,27 @@ inline void inst_end(lesgpu_case *c, int cls) {
 namespace lg {
 // launch wrappers implemented in the k_*.cu files
 void launch_stepinit(lesgpu_case *c);
-void launch_substepinit(lesgpu_case *c, int msub);
+// carry: qvol(1) of the substep is qvol(0) of the one before it
+void launch_substepinit(lesgpu_case *c, int msub, bool carry = false);
 void launch_qvolcalc(lesgpu_case *c, int slot);
 void launch_tvolcalc(lesgpu_case *c, int slot);
-// tvolcalc(tvol(2)) + tvolcorr; slot0: also tvol(0) (tcalc will not change t)
-void launch_tvolcalc_corr(lesgpu_case *c, bool slot0);
-void launch_meanpg(lesgpu_case *c);
+// tvolcalc(tvol(2)) + tvolcorr; slot0: also tvol(0) (tcalc will not change t);
+// bulk: also the fluid cells' temperature sum
+void launch_tvolcalc_corr(lesgpu_case *c, bool slot0, bool bulk = false);
+// have_q: S->qcur is the flow rate of u as it stands
+void launch_meanpg(lesgpu_case *c, bool have_q = false);
 // ucalc; with_qvol: fused with the qvolcalc before (qvol(2)) and after (qvol(0))
 void launch_ucalc_pcalc(lesgpu_case *c, bool with_qvol);
 void launch_tcalc(lesgpu_case *c);
 void launch_advance_and_convergence(lesgpu_case *c);
-void launch_bulk_diag(lesgpu_case *c);
+// have_q: S->qcur is u's flow rate; have_t: tbulk_sum the temperature sum
+void launch_bulk_diag(lesgpu_case *c, bool have_q = false, bool have_t = false);
 void launch_rhs(lesgpu_case *c, int msub);
 void launch_divgs(lesgpu_case *c);
 void launch_ghost_uvw(lesgpu_case *c);
-// rhs_t with its bulk velocity; with_tvol: tvolcalc(tvol(1)) in the same reduction
-void launch_rhs_t(lesgpu_case *c, int msub, bool with_tvol);
+// rhs_t with its bulk velocity; tvol 1: tvolcalc(tvol(1)) in the same
+// reduction, 2: tvol(1) is tvol(0) of the substep before, 0: not wanted
+void launch_rhs_t(lesgpu_case *c, int msub, int tvol);
 void launch_energy_bc(lesgpu_case *c);
 void launch_adi_uvw(lesgpu_case *c);
 void launch_adi_t(lesgpu_case *c);
@@ -399,12 +425,13 @@ namespace lg {
 // finish (counted with an atomic ticket after a release fence) sums all the
 // partials in block order -- the same fixed order as a separate finalize
 // kernel, so results are deterministic -- applies g and resets the ticket.
-template <int NV, bool MAX, class F, class G>
+template <int NV, unsigned MAXM, class F, class G>
 __global__ void __launch_bounds__(kThreads, 4) k_reduce_fin(KP p, Box b, F f, G g) {
+    static_assert(NV <= kThreads / 32 && NV <= kMaxRed, "one warp per value");
     __shared__ int last;
     double v[NV];
 #pragma unroll
-    for (int q = 0; q < NV; q++) v[q] = MAX ? -1.0e308 : 0.0;
+    for (int q = 0; q < NV; q++) v[q] = (MAXM >> q) & 1u ? -1.0e308 : 0.0;
     const long long n = b.count();
     const long long S = (long long)gridDim.x * blockDim.x;
     // a sum skips exact +0 terms (integer test): FP64 adds issue on the
@@ -413,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_reduce_fin(KP p, Box b, F f, G 
     auto add_terms = [&](const double (&w)[NV]) {
 #pragma unroll
         for (int q = 0; q < NV; q++) {
-            if (MAX) v[q] = fmax(v[q], w[q]);
+            if ((MAXM >> q) & 1u) v[q] = max_bits(v[q], w[q]);
             else if (__double_as_longlong(w[q]) != 0LL) v[q] = v[q] + w[q];
         }
     };
@@ -441,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_reduce_fin(KP p, Box b, F f, G 
         f(p, i, j, k, w);
         add_terms(w);
     }
-    block_reduce<NV, MAX>(v);
+    block_totals<NV, MAXM>(v);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < NV; q++) p.f.part[(size_t)blockIdx.x * kMaxRed + q] = v[q];
@@ -453,25 +480,28 @@ __global__ void __launch_bounds__(kThreads, 4) k_reduce_fin(KP p, Box b, F f, G 
     __threadfence();
     double acc[NV];
 #pragma unroll
-    for (int q = 0; q < NV; q++) acc[q] = MAX ? -1.0e308 : 0.0;
+    for (int q = 0; q < NV; q++) acc[q] = (MAXM >> q) & 1u ? -1.0e308 : 0.0;
     for (int bk = threadIdx.x; bk < (int)gridDim.x; bk += blockDim.x)
 #pragma unroll
         for (int q = 0; q < NV; q++) {
             const double x = __ldcg(p.f.part + (size_t)bk * kMaxRed + q);
-            acc[q] = MAX ? fmax(acc[q], x) : acc[q] + x;
+            acc[q] = (MAXM >> q) & 1u ? max_bits(acc[q], x) : acc[q] + x;
         }
-    block_reduce<NV, MAX>(acc);
+    block_totals<NV, MAXM>(acc);
     if (threadIdx.x == 0) {
         g(p, acc);
         *p.f.red_count = 0u;
     }
 }
 
-template <int NV, bool MAX, class F, class G>
+// Four blocks an SM at any size: one or two blocks an SM below 3e5 or 6e5
+// elements, whose SMs would total fewer blocks, are slower (64^3: 17.8 us
+// against 14.3 for the projection with its two flow rates, 9.7 against 8.4 for
+// the bulk velocity) -- loads in flight count for more than totals.
+template <int NV, unsigned MAXM, class F, class G>
 inline void reduce(lesgpu_case *c, Box b, F f, G g) {
-    int nb = blocks_for(b.count());
-    if (nb > kRedBlocks) nb = kRedBlocks;
-    k_reduce_fin<NV, MAX><<<nb, kThreads, 0, c->stream>>>(c->kp, b, f, g);
+    const int nb = blocks_for(b.count());
+    k_reduce_fin<NV, MAXM><<<nb < kRedBlocks ? nb : kRedBlocks, kThreads, 0, c->stream>>>(c->kp, b, f, g);
 }
 
 
