@@ -1138,6 +1138,306 @@ static bool adit_launch(lesgpu_case *c, const AdiBatch &B, int ncomp, int nmax) 
     return per ? adit_launch2<0, true>(grid, ts, c->stream, c->kp, B) : adit_launch2<0, false>(grid, ts, c->stream, c->kp, B);
 }
 
+// ------------------------------------------------------------------------
+// FP64 sweeps from both ends of a line.  A warp holds 16 lines: lane s
+// eliminates line s from its first row up, lane s + 16 from its last row
+// down, until they meet in the middle, where a 2x2 system joins them; the
+// substitution runs back out.  The rows' arithmetic is that of the one-sided
+// sweep (nothing is added for the split, where the warp-scan form computes 2x2
+// products), over half the serial steps and twice the warps.  On GB300 an FP64
+// instruction holds its sub-partition's pipe for 64 clocks whatever the lanes,
+// so a row's FP64 instructions are the time: 13, and 17 on a periodic line
+// (k_adi: 15 and 22), the system being divided by its diagonal through tables
+// of a line's metric factors formed once per warp.
+//
+// Shared memory holds a warp's rows: the right-hand sides and the viscosities
+// arrive by cp.async, all in flight at once, and are replaced by the
+// provisional solution and the factors as the elimination passes.  x lines
+// are contiguous, so they are fetched and written with the lanes along the
+// line (pitch 33 keeps both views free of bank conflicts).
+//
+// A periodic line is cut at its last unknown X: the rows before it carry the
+// coefficient s of X beside the solution, x = y + s X, and the last row then
+// gives X from its two neighbours.
+//
+// us a sweep, three components, against the better of one thread a line and
+// the warp-scan form: 64^3 z 38 (91), y 30 (62), x 42 (95); 90x81x96 92 (179),
+// 69 (91), 97 (179); 128^3 339 (375), 200 (220), 369 (453).  One component:
+// 64^3 31 (34), 23 (29), 34 (38).  A few hundred lines leave most pipes
+// without a warp and the scan form's shorter chain wins (64x48x8 x: 28 (17)).
+constexpr int kEnds = 256 | 16;      // the tuned table's code: 16 lines a warp
+constexpr int kEndsCh = 4;           // rows whose loads are issued together
+
+__host__ __device__ inline int ends_rows(int nline, bool per) { return ((per ? nline - 1 : nline) + 1) / 2; }
+static size_t ends_smem(int nline, int dir, bool per) {
+    return sizeof(double) * ((size_t)4 * nline + (size_t)(per ? 3 : 2) * ends_rows(nline, per) * (dir == 0 ? 33 : 32));
+}
+
+__device__ __forceinline__ void cp_async8(double *s, const double *g) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(s);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory"); }
+
+template <int DIR, bool PER>
+__global__ void __launch_bounds__(32) k_adie(KP p, AdiBatch B) {
+    extern __shared__ double4 ends_sm[];
+    const AdiArgs &A = B.a[blockIdx.y];
+    const DGrid &g = p.g;
+    const int na = A.a1 - A.a0 + 1, nb = A.b1 - A.b0 + 1;
+    const long long nl = (long long)na * nb, t0 = (long long)blockIdx.x * 16;
+    const int nline = A.l2 - A.l1 + 1;
+    if (nline <= 0 || t0 >= nl) return;
+    const long long stride = DIR == 2 ? g.sxy : DIR == 1 ? g.sx : 1;
+    constexpr int P = DIR == 0 ? 33 : 32;
+    const int nr = PER ? nline - 1 : nline;          // rows of the tridiagonal part
+    const int H = (nr + 1) / 2;                      // rows 0 .. H-1 from the front, the rest from the back
+    const int lane = threadIdx.x, back = lane >> 4, ln = lane & 15;
+    const bool mine = t0 + ln < nl;
+    const long long t = mine ? t0 + ln : nl - 1;
+    int i0, j0, k0;
+    line_coords(DIR, A.l1, A.a0 + (int)(t % na), A.b0 + (int)(t / na), i0, j0, k0);
+    const long long q0 = g.ix(i0, j0, k0);
+    const AdiFacs<double> F = adi_facs<double>(p, A.comp, DIR);
+    const double sc = A.comp == CT ? p.S->acoef * p.c.ipr : p.S->acoef;       // 1 / diagonal
+    double4 *tab = ends_sm;                          // (ma, ma cre, mc, mc cre) sc of each row
+    double *sx = reinterpret_cast<double *>(ends_sm + nline);       // right-hand side, then solution
+    double *sg = sx + H * P;                                        // outer face's viscosity, then factor
+    double *ss = sg + H * P;                                        // periodic: coefficient of X
+
+    // ---- rows to shared memory; row l sits in slot l of lane s (front) or
+    // slot nr - 1 - l of lane s + 16 (back), its viscosity the one of the face
+    // towards the middle
+    if (DIR == 0) {
+        for (int s = 0; s < 16; s++) {
+            const long long qs = __shfl_sync(0xffffffffu, q0, s);
+            for (int l = lane; l < nr; l += 32) {
+                const bool bk = l >= H;
+                const int o = (bk ? nr - 1 - l : l) * P + s + (bk ? 16 : 0);
+                cp_async8(sx + o, A.src + qs + l);
+                cp_async8(sg + o, F.nv + qs + F.oa + (bk ? l : l + 1));
+            }
+        }
+    } else {
+        const int mr = back ? nr - H : H;
+        for (int r = 0; r < mr; r++) {
+            const long long q = q0 + (long long)(back ? nr - 1 - r : r) * stride;
+            cp_async8(sx + r * P + lane, A.src + q);
+            cp_async8(sg + r * P + lane, F.nv + q + F.oa + (back ? 0 : stride));
+        }
+    }
+    double fin = F.nv[q0 + F.oa + (back ? (long long)nr * stride : 0)];       // the face the sweep starts at
+    double flast = 0.0, rlast = 0.0;
+    if (PER) {
+        flast = F.nv[q0 + F.oa + (long long)nline * stride];
+        rlast = A.src[q0 + (long long)nr * stride];
+    }
+    for (int l = lane; l < nline; l += 32) {
+        const double a = F.ma[A.l1 + l] * sc, c = F.mc[A.l1 + l] * sc;
+        tab[l] = make_double4(a, a * F.cre, c, c * F.cre);
+    }
+    cp_async_wait();
+    __syncwarp();
+
+    // ---- elimination towards the middle: x_r = y_r - g_r x_(r+1) + s_r X.
+    // Whole chunks run as one straight line: a chunk's coefficients, which
+    // nothing waits for, are formed while the pivots of the one before it pass
+    // (a lone warp issues in order, so a branch per row would leave the pipe
+    // idle for each reciprocal's latency).
+    const int mr = back ? nr - H : H;
+    double y = 0.0, gm = 0.0, sv = 1.0;              // the first row's inner neighbour: the wall (0) or X
+    const double fend = fin;
+    const double *tb = reinterpret_cast<const double *>(tab);
+    auto coefs = [&](int r, double &f, double &in, double &out, double &d) {
+        const double *m = tb + 4 * (back ? nr - 1 - r : r) + (back ? 2 : 0);       // towards the end, then the middle
+        const double *n = tb + 4 * (back ? nr - 1 - r : r) + (back ? 0 : 2);
+        in = fma(f, m[1], m[0]);
+        f = sg[r * P + lane];
+        out = fma(f, n[1], n[0]);
+        d = (1.0 - in) - out;
+    };
+    auto row = [&](int r, double rv, double in, double bet, double g) {
+        y = fma(-in, y, rv) * bet;
+        if (PER) {
+            sv = -(in * sv) * bet;
+            ss[r * P + lane] = sv;
+        }
+        gm = g;
+        sx[r * P + lane] = y;
+        sg[r * P + lane] = g;
+    };
+    int r = 0;
+    const int nfull = (nr - H) / kEndsCh;            // whole chunks of both sides
+    if (nfull > 0) {
+        double rv[kEndsCh], in[kEndsCh], out[kEndsCh], d[kEndsCh];
+#pragma unroll
+        for (int u = 0; u < kEndsCh; u++) {
+            rv[u] = sx[u * P + lane];
+            coefs(u, fin, in[u], out[u], d[u]);
+        }
+        for (int q = 0; q < nfull; q++, r += kEndsCh) {
+            double rn[kEndsCh], inn[kEndsCh], on[kEndsCh], dn[kEndsCh], bet[kEndsCh], gv[kEndsCh];
+            const int nx = q + 1 < nfull ? r + kEndsCh : 0;          // the last pass forms a chunk nobody reads
+            double ff = fin;
+            bool ok = true;
+#pragma unroll
+            for (int u = 0; u < kEndsCh; u++) {
+                rn[u] = sx[(nx + u) * P + lane];
+                coefs(nx + u, ff, inn[u], on[u], dn[u]);
+                bet[u] = rcp_fp64_fast(fma(-in[u], u == 0 ? gm : gv[u > 0 ? u - 1 : 0], d[u]), ok);
+                gv[u] = out[u] * bet[u];
+            }
+            if (!ok) {                                // zero, NaN or out of range: divisions, as rcp_fp64 takes
+#pragma unroll
+                for (int u = 0; u < kEndsCh; u++) {
+                    bet[u] = rcp_fp64(fma(-in[u], u == 0 ? gm : gv[u > 0 ? u - 1 : 0], d[u]));
+                    gv[u] = out[u] * bet[u];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kEndsCh; u++) row(r + u, rv[u], in[u], bet[u], gv[u]);
+            if (q + 1 < nfull) fin = ff;
+#pragma unroll
+            for (int u = 0; u < kEndsCh; u++) {
+                rv[u] = rn[u];
+                in[u] = inn[u];
+                out[u] = on[u];
+                d[u] = dn[u];
+            }
+        }
+    }
+    for (; r < H; r++)
+        if (r < mr) {
+            const double rv = sx[r * P + lane];
+            double in, out, d;
+            coefs(r, fin, in, out, d);
+            const double bet = rcp_fp64(fma(-in, gm, d));
+            row(r, rv, in, bet, out * bet);
+        }
+    // ---- the two middle rows
+    double go = __shfl_xor_sync(0xffffffffu, gm, 16), yo = __shfl_xor_sync(0xffffffffu, y, 16);
+    double so = PER ? __shfl_xor_sync(0xffffffffu, sv, 16) : 0.0;
+    if (nr == 1) go = yo = so = 0.0;                 // nothing from the back
+    const double w = rcp_fp64(fma(-gm, go, 1.0));
+    double x = fma(-gm, yo, y) * w, s1 = PER ? fma(-gm, so, sv) * w : 0.0;
+
+    // ---- substitution outwards
+    auto put = [&](int r, double v) {
+        const long long q = q0 + (long long)(back ? nr - 1 - r : r) * stride;
+        if (mine) {
+            if (A.add) A.dst[q] += v;
+            else A.dst[q] = v;
+        }
+    };
+    if (mr > 0) {
+        if (PER || DIR == 0) {
+            sx[(mr - 1) * P + lane] = x;
+            if (PER) ss[(mr - 1) * P + lane] = s1;
+        } else {
+            put(mr - 1, x);
+        }
+    }
+    for (int r1 = mr - 2; r1 >= 0; r1 -= kEndsCh) {
+        double yv[kEndsCh], gv[kEndsCh], zv[kEndsCh];
+#pragma unroll
+        for (int u = 0; u < kEndsCh; u++) {
+            const int r = r1 - u;
+            if (r >= 0) {
+                yv[u] = sx[r * P + lane];
+                gv[u] = sg[r * P + lane];
+                if (PER) zv[u] = ss[r * P + lane];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kEndsCh; u++) {
+            const int r = r1 - u;
+            if (r >= 0) {
+                x = fma(-gv[u], x, yv[u]);
+                if (PER) {
+                    s1 = fma(-gv[u], s1, zv[u]);
+                    ss[r * P + lane] = s1;
+                }
+                if (PER || DIR == 0) sx[r * P + lane] = x;
+                else put(r, x);
+            }
+        }
+    }
+    double X = 0.0;
+    if (PER) {
+        // last row: a x_(nr-1) + c x_0 + (1 - a - c) X = its right-hand side;
+        // x and s1 are those of row 0 (front) and row nr - 1 (back)
+        const double4 m = tab[nr];
+        const double a = fma(__shfl_sync(0xffffffffu, fend, ln + 16), m.y, m.x), c = fma(flast, m.w, m.z);
+        const double k = back ? a : c;
+        double kx = k * x, ks = k * s1;
+        kx += __shfl_xor_sync(0xffffffffu, kx, 16);
+        ks += __shfl_xor_sync(0xffffffffu, ks, 16);
+        X = (rlast - kx) * rcp_fp64(((1.0 - a) - c) + ks);
+        if (DIR != 0) {
+            for (int r = 0; r < mr; r++) put(r, fma(ss[r * P + lane], X, sx[r * P + lane]));
+            if (back == 0) put(nr, X);
+        }
+    }
+    // ---- x lines out, lanes along the line
+    if (DIR == 0) {
+        __syncwarp();
+        for (int s0 = 0; s0 < 16; s0 += 8) {
+            long long qs[8];
+            double Xs[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                qs[u] = __shfl_sync(0xffffffffu, q0, s0 + u);
+                Xs[u] = PER ? __shfl_sync(0xffffffffu, X, s0 + u) : 0.0;
+            }
+            for (int l = lane; l < nline; l += 32) {
+                const bool bk = l >= H;
+                double v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = A.add && t0 + s0 + u < nl ? A.dst[qs[u] + l] : 0.0;
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    if (t0 + s0 + u >= nl) continue;
+                    double x1 = Xs[u];
+                    if (!PER || l < nr) {
+                        const int o = (bk ? nr - 1 - l : l) * P + s0 + u + (bk ? 16 : 0);
+                        x1 = PER ? fma(ss[o], Xs[u], sx[o]) : sx[o];
+                    }
+                    A.dst[qs[u] + l] = A.add ? v[u] + x1 : x1;
+                }
+            }
+        }
+    }
+}
+
+// dynamic shared memory a warp of the two-ended form may take: three on an SM
+// at the least (lines of up to ~280 rows, 190 periodic ones)
+constexpr size_t kEndsSmemMax = 72 * 1024;
+
+template <int DIR, bool PER>
+static void ends_launch2(dim3 grid, size_t smem, cudaStream_t st, const KP &kp, const AdiBatch &B) {
+    static const bool ok = cudaFuncSetAttribute(k_adie<DIR, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)kEndsSmemMax) == cudaSuccess;
+    (void)ok;
+    k_adie<DIR, PER><<<grid, 32, smem, st>>>(kp, B);
+}
+
+// The two-ended FP64 sweep of a batch (factored coefficients); false when it
+// does not apply: a line too long for shared memory, or a periodic line whose
+// last row's neighbours are not two different rows.
+static bool ends_launch(lesgpu_case *c, const AdiBatch &B, int ncomp, long long mx, int nmax) {
+    const int dir = B.a[0].dir;
+    const bool per = B.a[0].periodic != 0;
+    const size_t smem = ends_smem(nmax, dir, per);
+    if (smem > kEndsSmemMax) return false;
+    for (int q = 0; q < ncomp; q++)
+        if (per && B.a[q].l2 - B.a[q].l1 + 1 < 3) return false;
+    const dim3 grid((unsigned)((mx + 15) / 16), (unsigned)ncomp);
+    if (dir == 0) { if (per) ends_launch2<0, true>(grid, smem, c->stream, c->kp, B); else ends_launch2<0, false>(grid, smem, c->stream, c->kp, B); }
+    else if (dir == 1) { if (per) ends_launch2<1, true>(grid, smem, c->stream, c->kp, B); else ends_launch2<1, false>(grid, smem, c->stream, c->kp, B); }
+    else { if (per) ends_launch2<2, true>(grid, smem, c->stream, c->kp, B); else ends_launch2<2, false>(grid, smem, c->stream, c->kp, B); }
+    return true;
+}
+
 template <class R, int W>
 static bool adis_launch(lesgpu_case *c, const AdiBatch &B, int ncomp, long long mx, int nmax, bool capped) {
     const int m = (nmax + W - 1) / W;
@@ -1163,11 +1463,12 @@ static bool adis_launch(lesgpu_case *c, const AdiBatch &B, int ncomp, long long 
 // independent of each other, and three times the lines keep three times as
 // many FP64 pipes busy on small grids.
 //
-// Lanes per line (W) of each sweep class -- 1 = one thread per line
-// (k_adi), else the warp-scan form k_adis -- are picked by an autotuner: at
-// the first start of a case of a given shape every feasible W is timed on the
-// case's own sweeps (results redirected to scratch) and the fastest kept in a
-// process-wide table, so later cases of the shape (the serving loop) reuse it.
+// The form of each sweep class -- one thread per line (k_adi), W lanes per
+// line (the warp-scan form k_adis), tiled FP32 or two-ended FP64 -- is picked
+// by an autotuner: at the first start of a case of a given shape every
+// feasible form is timed on the case's own sweeps (results redirected to
+// scratch) and the fastest kept in a process-wide table, so later cases of the
+// shape (the serving loop) reuse it.
 // Mixed form: FP32 arithmetic for the x and z sweeps, the wall-normal
 // (stretched) y sweep stays FP64.
 struct AdiShape {
@@ -1186,19 +1487,27 @@ static AdiShape adi_shape(const lesgpu_case *c, const AdiBatch &B, int ncomp) {
     return h;
 }
 
+// factored coefficients unless a temperature sweep reads conjugate tables
+// that are not all 1
+static bool adi_factored(const lesgpu_case *c, const AdiBatch &B) {
+    return !(B.a[0].comp == CT && c->kp.c.iconjg == 1 && c->conj_general);
+}
+
 // launch with W = w & 63 lanes per line (w & 64: the register-capped warp-scan
 // kernel; w == kTiled: the tiled FP32 sweep); false if that form cannot take
 // the batch (W cannot hold the line, MC <= 12; the tiled form needs FP32
-// and factored coefficients)
+// and factored coefficients; kEnds: the two-ended FP64 sweep, likewise)
 constexpr int kTiled = 128;
 static bool adi_run(lesgpu_case *c, const AdiBatch &B, const AdiShape &h, int wcode) {
     if (h.mx <= 0) return true;
-    // factored coefficients unless a temperature sweep reads conjugate
-    // tables that are not all 1
-    const bool fac = !(B.a[0].comp == CT && c->kp.c.iconjg == 1 && c->conj_general);
+    const bool fac = adi_factored(c, B);
     if (wcode == kTiled) {
         if (!h.f32 || !fac) return false;
         return adit_launch(c, B, h.ncomp, h.nmax);
+    }
+    if (wcode == kEnds) {
+        if (h.f32 || !fac) return false;
+        return ends_launch(c, B, h.ncomp, h.mx, h.nmax);
     }
     const int w = wcode & 63;
     const bool capped = (wcode & 64) != 0;
@@ -1245,10 +1554,14 @@ static AdiTuneKey adi_key(const lesgpu_case *c, const AdiBatch &B, const AdiShap
     return AdiTuneKey{g.n1m, g.n2m, g.n3m, B.a[0].dir, h.ncomp, h.f32 ? 1 : 0, B.a[0].periodic, h.nmax};
 }
 
-// W used until a shape is tuned: the FP32 form 32 lanes; FP64 about 64k threads
-static int adi_default_w(const AdiShape &h) {
+// W used until a shape is tuned: the FP32 form 32 lanes; FP64 the two-ended
+// form from 3000 lines (48x48x32 with 1536: 19 us against 20, 32x32x16 with
+// 512: 15 against 13) of up to 128 rows (128^3: 200 against 220, 160x192x160
+// y: 510 against 449), else about 64k threads
+static int adi_default_w(const lesgpu_case *c, const AdiBatch &B, const AdiShape &h) {
     if (h.f32) return 32;
     const long long lines = h.mx * h.ncomp;
+    if (lines >= 3000 && h.nmax <= 128 && adi_factored(c, B) && (!B.a[0].periodic || h.nmax >= 4)) return kEnds;
     int w = 1;
     while (w < 32 && lines * w < 65536) w <<= 1;
     return w < 8 ? 1 : w;
@@ -1257,7 +1570,7 @@ static int adi_default_w(const AdiShape &h) {
 static void adi_launch(lesgpu_case *c, const AdiBatch &B, int ncomp) {
     const AdiShape h = adi_shape(c, B, ncomp);
     if (h.mx <= 0) return;
-    int w = adi_default_w(h);
+    int w = adi_default_w(c, B, h);
     if (c->autotune) {
         std::lock_guard<std::mutex> lk(g_adi_mu);
         auto it = g_adi_w.find(adi_key(c, B, h));
@@ -1291,12 +1604,12 @@ static void adi_tune_batch(lesgpu_case *c, AdiBatch B, int ncomp) {
     cudaEventCreate(&e1);
     // the register-capped warp-scan variant only differs where a lane holds
     // more than 4 rows
-    const int cand[8] = {1, 8, 16, 32, 8 | 64, 16 | 64, 32 | 64, kTiled};
-    int best = adi_default_w(h);
+    const int cand[9] = {1, 8, 16, 32, 8 | 64, 16 | 64, 32 | 64, kTiled, kEnds};
+    int best = adi_default_w(c, B, h);
     float best_ms = 3.0e38f;
-    for (int q = 0; q < 8; q++) {
+    for (int q = 0; q < 9; q++) {
         if (cand[q] == kTiled && (!h.f32 || B.a[0].dir == 1)) continue;
-        if (cand[q] != kTiled && (cand[q] & 64) && (h.nmax + (cand[q] & 63) - 1) / (cand[q] & 63) <= 4) continue;
+        if (cand[q] != kTiled && cand[q] != kEnds && (cand[q] & 64) && (h.nmax + (cand[q] & 63) - 1) / (cand[q] & 63) <= 4) continue;
         if (!adi_run(c, B, h, cand[q])) continue;          // warm-up launch (also the feasibility check)
         cudaEventRecord(e0, c->stream);
         for (int r = 0; r < 3; r++) adi_run(c, B, h, cand[q]);
@@ -1386,9 +1699,9 @@ static void adi_table_load(const char *path) {
     while (fscanf(f, "%15s %d %d %d %d %d %d %d %d %d", tag, &k.n1m, &k.n2m, &k.n3m, &k.dir, &k.ncomp, &k.f32,
                   &k.periodic, &k.nmax, &w) == 10)
         if (!strcmp(tag, "adi") && !g_adi_w.count(k)) {
-            const int wl = w & 63;    // lanes; + 64: the register-capped warp-scan kernel; 128: tiled
+            const int wl = w & 63;    // lanes; + 64: the register-capped warp-scan kernel; 128: tiled; 272: two-ended
             if ((wl == 1 && w == 1) || ((wl == 8 || wl == 16 || wl == 32) && (w == wl || w == (wl | 64))) ||
-                w == kTiled)
+                w == kTiled || w == kEnds)
                 g_adi_w[k] = w;
         }
     fclose(f);

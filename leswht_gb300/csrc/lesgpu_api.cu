@@ -270,6 +270,7 @@ extern "C" int lesgpu_create(const lesgpu_config *cfg, const lesgpu_grid *g, les
         k.inv_repr_d = 1.0 / (re * pr); k.inv_repr_f = (float)(1.0 / (re * pr));
         k.gterm = cfg->gr / (re * re);
         k.ivol = 1.0 / (g->xl * g->yl * g->zl);
+        k.ipr = 1.0 / pr;
         // the gradient at a wall from the first two points, d1 and d2 away
         auto wall = [&](int q, double ci1, double ci2) {
             const double d1 = 1.0 / ci1, d2 = d1 + 1.0 / ci2, den = d1 * d2 * (d2 - d1) * re;

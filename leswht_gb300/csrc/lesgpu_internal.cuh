@@ -52,7 +52,7 @@ struct DCfg {
     // value (FP64 arithmetic on the FP32-rounded re, then rounded)
     double rei_d, inv_repr_d, gterm;   // 1/re, 1/(re pr), gr/re^2
     float rei_f, inv_repr_f;
-    double ivol;                        // 1 / (xl yl zl)
+    double ivol, ipr;                   // 1 / (xl yl zl), 1 / pr
     double wall_a[4], wall_b[4];        // meanpg's one-sided wall gradients / re: a u(wall) - b u(next), y bottom, y top, z bottom, z top
     double adi_cd[3];                   // ADI: iles re, 2 iles re, iles re pr
     float adi_cf[3];
@@ -227,6 +227,24 @@ __device__ __forceinline__ double rcp_fp64(double d) {
                                 | ((unsigned long long)(((rs >> 23) & 0xffu) - 127u + 1023u) << 52)
                                 | ((unsigned long long)(rs & 0x7fffffu) << 29);
     const double r = __longlong_as_double((long long)rb);
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+// The same without its branch, for straight-line code: from the approximate
+// FP32 reciprocal of the significand (error below 2^-22, its cube below
+// 2^-66) and the exponent negated.  ok is cleared where the operand or result
+// would leave the normal range; the caller then takes rcp_fp64.
+__device__ __forceinline__ double rcp_fp64_fast(double d, bool &ok) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(d);
+    const unsigned hi = (unsigned)(bits >> 32);
+    const unsigned ed = hi & 0x7ff00000u;
+    ok = ok && ed - 0x06400000u < 0x73700000u;                // biased exponents 100 .. 1946
+    float rs;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(__uint_as_float(0x3f800000u | ((unsigned)(bits >> 29) & 0x7fffffu))));
+    const unsigned rf = __float_as_uint(rs);                  // in (1/2, 1]
+    const unsigned rh = ((rf >> 3) + ((1023u - 127u) << 20) - (ed - (1023u << 20))) | (hi & 0x80000000u);
+    const double r = __longlong_as_double((long long)(((unsigned long long)rh << 32) | (unsigned long long)(rf << 29)));
     const double e = fma(-d, r, 1.0);
     return fma(r, fma(e, e, e), r);
 }
