@@ -20,11 +20,13 @@ struct UbulkFinal {
         else if (fabs(p.c.udrv_i) > 1.0e-12) ub = p.c.udrv_i;
         else ub = 1.0;
         p.S->u_bulk_t = ub;
+        p.S->hub = 0.5 / ub;
         if (carry) p.S->tvol[1] = p.S->tvol[0];
     }
 };
 __global__ void k_set_ubulk_one(KP p, int carry) {
     p.S->u_bulk_t = 1.0;
+    p.S->hub = 0.5;
     if (carry) p.S->tvol[1] = p.S->tvol[0];
 }
 

@@ -5,16 +5,15 @@
 // One thread per cell computes all three momentum components, so u, v, w, p
 // and the eddy viscosities around a cell are read once per cell from L1/L2
 // instead of once per component; the SGS cross term never goes to memory.
-// Each expression keeps the reference's operation order.
+// The FP32 expressions keep the reference's operation order.
 #include "lesgpu_internal.cuh"
 
 namespace lg {
 
-// R: arithmetic type (double; float in the mixed-precision form).  Every
-// load is converted to R, so the whole stencil runs in R; the reference's
-// operation order is kept either way.
+// R: arithmetic type.  Instantiated for float, the mixed-precision form; the
+// FP64 form is k_rhs64 (and k_rhs_t64).
 template <class R>
-__global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 3 : 1) k_rhs(KP p, Box b, R gam, R ro) {
+__global__ void __launch_bounds__(kThreads, 3) k_rhs(KP p, Box b, R gam, R ro) {
     const Mir<R> &M = mir<R>(p);
     const DGrid &g = p.g;
     const DCfg &c = p.c;
@@ -161,6 +160,110 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 3 : 1) k_rhs(KP p, 
     }
 }
 
+// The FP64 form.  One thread a cell, the metric products from the 1-D weights
+// of Stn, the viscous and eddy-viscous gradients of a face under one
+// coefficient and the cell's lower edges shared by the equations that use
+// them: 195 FP64 operations a cell where the written-out form of k_rhs took
+// 405, each 64 clocks a warp (k_grad64.cuh).  64^3: 175 us -> 100; 90x81x96:
+// 451 us -> 254.
+__global__ void __launch_bounds__(kThreads, 2) k_rhs64(KP p, Box b, double gam, double ro) {
+    const DGrid &g = p.g;
+    const DCfg &c = p.c;
+    const Stn &T = p.st;
+    const DFields &f = p.f;
+    const double *u = f.u, *v = f.v, *w = f.w, *pp = f.p;
+    const double *nu = f.nusgs, *nu1 = f.nusgs1[0], *nu2 = f.nusgs1[1], *nu3 = f.nusgs1[2];
+    const double dt = p.S->dt;
+    const double cg = dt * gam, cr = dt * ro, ca = dt * (2.0 * p.S->alpha);
+    const double pmi = c.ich != 0 ? p.S->pmi[0] : 0.0;
+    const double rei = c.rei_d;
+    const long long sx = g.sx, sxy = g.sxy;
+    const bool les = c.iles == 1, grav = c.ihtrans == 1 && c.gterm != 0.0;
+    const long long n = b.count();
+    for (long long tt = (long long)blockIdx.x * blockDim.x + threadIdx.x; tt < n; tt += (long long)gridDim.x * blockDim.x) {
+        int i, j, k;
+        b.at(tt, i, j, k);
+        const long long q = g.ix(i, j, k);
+        const double2 X0 = T.gx[i], X1 = T.gx[i + 1], Y0 = T.gy[j], Y1 = T.gy[j + 1], Z0 = T.gz[k], Z1 = T.gz[k + 1];
+        const double fx = g.f2fxi[i], fy = g.f2fyi[j], fz = g.f2fzi[k];
+        const double cx = g.c2cxi[i], cy = g.c2cyi[j], cz = g.c2czi[k];
+        const double uq = u[q], vq = v[q], wq = w[q];
+        const double nq = les ? fma(2.0, nu[q], rei) : rei;
+        // the cell's lower edges: 3 = (x, y) between u and v, 2 = (x, z)
+        // between u and w, 1 = (y, z) between v and w
+        const double us = u[q - sx], ub = u[q - sxy], vw = v[q - 1], vb = v[q - sxy], ww = w[q - 1], ws = w[q - sx];
+        const double e3 = les ? nu3[q] : 0.0, e2 = les ? nu2[q] : 0.0, e1 = les ? nu1[q] : 0.0;
+        const double uy = Y0.x * us + Y0.y * uq, vx = X0.x * vw + X0.y * vq;
+        const double uz = Z0.x * ub + Z0.y * uq, wx = X0.x * ww + X0.y * wq;
+        const double vz = Z0.x * vb + Z0.y * vq, wy = Y0.x * ws + Y0.y * wq;
+        const double du3 = uq - us, dv3 = vq - vw, du2 = uq - ub, dw2 = wq - ww, dv1 = vq - vb, dw1 = wq - ws;
+        const double n3 = rei + e3, n2 = rei + e2, n1 = rei + e1;
+        const double pq = pp[q], bq = grav ? c.gterm * f.t[q] : 0.0;
+        const double ue = u[q + 1], vn = v[q + sx], wt = w[q + sxy];
+
+        if (i >= g.i_bgpx) {
+            const double un = u[q + sx], ut = u[q + sxy], uw = u[q - 1], vnw = v[q + sx - 1], wtw = w[q + sxy - 1];
+            const double en = les ? nu3[q + sx] : 0.0, et = les ? nu2[q + sxy] : 0.0;
+            const double nw = les ? fma(2.0, nu[q - 1], rei) : rei;
+            const double y = (en * (vn - vnw) - e3 * dv3) * cx
+                           - ((Y1.x * uq + Y1.y * un) * (X0.x * vnw + X0.y * vn) - uy * vx);
+            const double z = (et * (wt - wtw) - e2 * dw2) * cx
+                           - ((Z1.x * uq + Z1.y * ut) * (X0.x * wtw + X0.y * wt) - uz * wx);
+            const double s = ue + uq, r = uq + uw;
+            double rk = fy * y + fz * z - T.qx[i] * (s * s - r * r);
+            if (grav && c.grdir == 1) rk = rk + bq;
+            const double ax = nq * ((ue - uq) * fx) - nw * ((uq - uw) * g.f2fxi[i - 1]) - (pq - pp[q - 1]);
+            const double ay = (rei + en) * ((un - uq) * g.c2cyi[j + 1]) - n3 * (du3 * cy);
+            const double az = (rei + et) * ((ut - uq) * g.c2czi[k + 1]) - n2 * (du2 * cz);
+            const double al = (ax * cx + ay * fy + az * fz) - pmi;
+            const double h = f.rk3o[0][q];
+            f.rhs1[0][q] = cg * rk + cr * h + ca * al;
+            f.rk3oo[0][q] = h;
+            f.rk3o[0][q] = rk;
+        }
+        if (j >= g.j_bgpy) {
+            const double ve = v[q + 1], vt = v[q + sxy], vs = v[q - sx], use = u[q + 1 - sx], wts = w[q + sxy - sx];
+            const double ee = les ? nu3[q + 1] : 0.0, et = les ? nu1[q + sxy] : 0.0;
+            const double ns = les ? fma(2.0, nu[q - sx], rei) : rei;
+            const double x = (ee * (ue - use) - e3 * du3) * cy
+                           - ((Y0.x * use + Y0.y * ue) * (X1.x * vq + X1.y * ve) - uy * vx);
+            const double z = (et * (wt - wts) - e1 * dw1) * cy
+                           - ((Z1.x * vq + Z1.y * vt) * (Y0.x * wts + Y0.y * wt) - vz * wy);
+            const double s = vn + vq, r = vq + vs;
+            double rk = fx * x + fz * z - T.qy[j] * (s * s - r * r);
+            if (grav && c.grdir == 2) rk = rk + bq;
+            const double ax = (rei + ee) * ((ve - vq) * g.c2cxi[i + 1]) - n3 * (dv3 * cx);
+            const double ay = nq * ((vn - vq) * fy) - ns * ((vq - vs) * g.f2fyi[j - 1]) - (pq - pp[q - sx]);
+            const double az = (rei + et) * ((vt - vq) * g.c2czi[k + 1]) - n1 * (dv1 * cz);
+            const double al = ax * fx + ay * cy + az * fz;
+            const double h = f.rk3o[1][q];
+            f.rhs1[1][q] = cg * rk + cr * h + ca * al;
+            f.rk3oo[1][q] = h;
+            f.rk3o[1][q] = rk;
+        }
+        if (k >= g.k_bgpz && g.n3m != 1) {
+            const double we = w[q + 1], wn = w[q + sx], wb = w[q - sxy], ube = u[q + 1 - sxy], vnb = v[q + sx - sxy];
+            const double ee = les ? nu2[q + 1] : 0.0, en = les ? nu1[q + sx] : 0.0;
+            const double nb = les ? fma(2.0, nu[q - sxy], rei) : rei;
+            const double x = (ee * (ue - ube) - e2 * du2) * cz
+                           - ((Z0.x * ube + Z0.y * ue) * (X1.x * wq + X1.y * we) - uz * wx);
+            const double y = (en * (vn - vnb) - e1 * dv1) * cz
+                           - ((Z0.x * vnb + Z0.y * vn) * (Y1.x * wq + Y1.y * wn) - vz * wy);
+            const double s = wt + wq, r = wq + wb;
+            double rk = fx * x + fy * y - T.qz[k] * (s * s - r * r);
+            if (grav && c.grdir == 3) rk = rk + bq;
+            const double ax = (rei + ee) * ((we - wq) * g.c2cxi[i + 1]) - n2 * (dw2 * cx);
+            const double ay = (rei + en) * ((wn - wq) * g.c2cyi[j + 1]) - n1 * (dw1 * cy);
+            const double az = nq * ((wt - wq) * fz) - nb * ((wq - wb) * g.f2fzi[k - 1]) - (pq - pp[q - sxy]);
+            const double al = ax * fx + ay * fy + az * cz;
+            const double h = f.rk3o[2][q];
+            f.rhs1[2][q] = cg * rk + cr * h + ca * al;
+            f.rk3oo[2][q] = h;
+            f.rk3o[2][q] = rk;
+        }
+    }
+}
+
 void launch_rhs(lesgpu_case *c, int msub) {
     const double gam[4] = {0.0, 8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
     const double ro[4] = {0.0, 0.0, -17.0 / 60.0, -5.0 / 12.0};
@@ -170,7 +273,7 @@ void launch_rhs(lesgpu_case *c, int msub) {
     if (c->cfg.precision == LESGPU_PREC_MIXED)
         k_rhs<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, (float)gam[msub], (float)ro[msub]);
     else
-        k_rhs<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, gam[msub], ro[msub]);
+        k_rhs64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, gam[msub], ro[msub]);
     inst_end(c, LESGPU_K_RHS);
 }
 
@@ -291,6 +394,71 @@ __global__ void __launch_bounds__(kThreads) k_rhs_t(KP p, Box b, R gam, R ro, in
     }
 }
 
+// The FP64 form: 1-D weights, one coefficient per face for the molecular and
+// the eddy diffusivity, the bulk velocity's reciprocal formed once: 55 FP64
+// operations a cell for 127.  64^3: 57 us -> 31.
+__global__ void __launch_bounds__(kThreads) k_rhs_t64(KP p, Box b, double gam, double ro, int conj) {
+    const DGrid &g = p.g;
+    const DCfg &c = p.c;
+    const Stn &T = p.st;
+    const DFields &f = p.f;
+    const double *t = f.t, *u = f.u, *v = f.v, *w = f.w;
+    const double *al1 = f.alsgs1[0], *al2 = f.alsgs1[1], *al3 = f.alsgs1[2];
+    const double dt = p.S->dt;
+    const double cg = dt * gam, cr = dt * ro, ca = dt * (2.0 * p.S->alpha), hub = p.S->hub;
+    const double ir = c.inv_repr_d;
+    const bool les = c.iles == 1;
+    const bool ghost_x = c.xprdic == 1 && c.idecomp == 0;       // x neighbours by the ghost layers
+    const long long n = b.count();
+    for (long long tt = (long long)blockIdx.x * blockDim.x + threadIdx.x; tt < n; tt += (long long)gridDim.x * blockDim.x) {
+        int i, j, k;
+        b.at(tt, i, j, k);
+        const long long q = g.ix(i, j, k);
+        const int kp = g.kpv[k], km = g.kmv[k], jp = g.jpv[j], jm = g.jmv[j];
+        int ip = g.ipv[i], im = g.imv[i];
+        if (ghost_x) {
+            if (i == g.n1m) ip = g.n1;
+            if (i == 1) im = 0;
+        }
+        const double2 *fx = ghost_x ? T.gx : T.wx;
+        const double2 X0 = fx[i], X1 = fx[ip], Y0 = T.wy[j], Y1 = T.wy[jp], Z0 = T.wz[k], Z1 = T.wz[kp];
+        const long long qip = g.ix(ip, j, k), qim = g.ix(im, j, k), qjp = g.ix(i, jp, k), qjm = g.ix(i, jm, k);
+        const long long qkp = g.ix(i, j, kp), qkm = g.ix(i, j, km);
+        const double tq = t[q], te = t[qip], tw = t[qim], tn = t[qjp], ts = t[qjm], tc = t[qkp], tf = t[qkm];
+        const double ant = ((X1.x * tq + X1.y * te) * u[qip] - (X0.x * tw + X0.y * tq) * u[q]) * g.f2fxi[i]
+                         + ((Y1.x * tq + Y1.y * tn) * v[qjp] - (Y0.x * ts + Y0.y * tq) * v[q]) * g.f2fyi[j]
+                         + ((Z1.x * tq + Z1.y * tc) * w[qkp] - (Z0.x * tf + Z0.y * tq) * w[q]) * g.f2fzi[k];
+        double rk = c.idecomp == 1 ? hub * (u[q] + u[q + 1]) - ant : -ant;
+        double ke = ir, kw = ir, kn = ir, ks = ir, kc = ir, kf = ir, om = 1.0;
+        if (conj) {
+            om = c.imovingon == 0 ? (double)f.omega[q] : 1.0;
+            rk = om * rk;
+            const double cs = ir * f.cstar[q];
+            ke = cs * f.kstar[0][q]; kw = cs * f.kstar[1][q];
+            kn = cs * f.kstar[2][q]; ks = cs * f.kstar[3][q];
+            kc = cs * f.kstar[4][q]; kf = cs * f.kstar[5][q];
+        }
+        if (les) {
+            if (conj) {
+                ke = ke + om * al1[qip]; kw = kw + om * al1[q];
+                kn = kn + om * al2[qjp]; ks = ks + om * al2[q];
+                kc = kc + om * al3[qkp]; kf = kf + om * al3[q];
+            } else {
+                ke = ke + al1[qip]; kw = kw + al1[q];
+                kn = kn + al2[qjp]; ks = ks + al2[q];
+                kc = kc + al3[qkp]; kf = kf + al3[q];
+            }
+        }
+        const double alt = (ke * ((te - tq) * g.c2cxi[ip]) - kw * ((tq - tw) * g.c2cxi[i])) * g.f2fxi[i]
+                         + (kn * ((tn - tq) * g.c2cyi[jp]) - ks * ((tq - ts) * g.c2cyi[j])) * g.f2fyi[j]
+                         + (kc * ((tc - tq) * g.c2czi[kp]) - kf * ((tq - tf) * g.c2czi[k])) * g.f2fzi[k];
+        const double h = f.rk3o[3][q];
+        f.rhs1[3][q] = cg * rk + cr * h + ca * alt;
+        f.rk3oo[3][q] = h;
+        f.rk3o[3][q] = rk;
+    }
+}
+
 void launch_rhs_t_kernel(lesgpu_case *c, int msub) {
     const double gam[4] = {0.0, 8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
     const double ro[4] = {0.0, 0.0, -17.0 / 60.0, -5.0 / 12.0};
@@ -301,7 +469,7 @@ void launch_rhs_t_kernel(lesgpu_case *c, int msub) {
     if (c->cfg.precision == LESGPU_PREC_MIXED)
         k_rhs_t<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, (float)gam[msub], (float)ro[msub], conj);
     else
-        k_rhs_t<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, gam[msub], ro[msub], conj);
+        k_rhs_t64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, gam[msub], ro[msub], conj);
     inst_end(c, LESGPU_K_RHS_T);
 }
 

@@ -10,11 +10,11 @@
 // x-filtered values at k-1, k, k+1 in registers and applies the z weights to
 // them, which is the reference's arithmetic with its rounding order and a
 // third of its memory traffic.
-#include "lesgpu_internal.cuh"
+#include "k_grad64.cuh"
 
 namespace lg {
 
-// velgrad, sgs.f90:772-875.  R: arithmetic type (float in the mixed form).
+// velgrad, sgs.f90:772-875, of the mixed form (R = float; FP64: k_grad64.cuh).
 template <class R>
 __device__ void velgrad(const KP &p, int i, int j, int k, R a[9], R sr[6]) {
     const Mir<R> &M = mir<R>(p);
@@ -112,6 +112,22 @@ __device__ __forceinline__ void vreman(const R alp[9], R sdx2, R sdy2, R sdz2, R
     bbb = b;
 }
 
+// Vreman's invariants in FP64 with the widths multiplied into the gradients:
+// 43 operations
+__device__ __forceinline__ void vreman64(const double a[9], double dx, double dy, double dz, double &aaa, double &bbb) {
+    const double x0 = dx * a[0], x1 = dx * a[1], x2 = dx * a[2];
+    const double y0 = dy * a[3], y1 = dy * a[4], y2 = dy * a[5];
+    const double z0 = dz * a[6], z1 = dz * a[7], z2 = dz * a[8];
+    const double b1 = x0 * x0 + y0 * y0 + z0 * z0, b2 = x0 * x1 + y0 * y1 + z0 * z1, b3 = x0 * x2 + y0 * y2 + z0 * z2;
+    const double b4 = x1 * x1 + y1 * y1 + z1 * z1, b5 = x1 * x2 + y1 * y2 + z1 * z2, b6 = x2 * x2 + y2 * y2 + z2 * z2;
+    double s = a[0] * a[0];
+#pragma unroll
+    for (int q = 1; q < 9; q++) s = s + a[q] * a[q];
+    const double b = b1 * b4 + b4 * b6 + b6 * b1 - b2 * b2 - b3 * b3 - b5 * b5;
+    aaa = s;
+    bbb = b < 1.0e-16 ? 1.0e-16 : b;
+}
+
 // Test-filter width at a cell: the sum of the three test-filter cell widths
 // used in the second Vreman / eddy-diffusivity evaluation (sgs.f90:528-533).
 template <class R, class T>
@@ -151,6 +167,31 @@ __global__ void __launch_bounds__(kThreads) k_vreman1(KP p, Box b, int dynamic) 
         for (int m = 0; m < 6; m++) scr<R>(p, 3 + m)[q] = nu * str[m];
 #pragma unroll
         for (int m = 0; m < 9; m++) scr<R>(p, 9 + m)[q] = alp[m];
+    }
+}
+
+// The FP64 form (k_grad64.cuh): 64^3 104 us -> 55.
+__global__ void __launch_bounds__(kThreads) k_vreman1_64(KP p, Box b, int dynamic) {
+    const Stn &T = p.st;
+    GRID_LOOP(b) {
+        int i, j, k;
+        b.at(tt, i, j, k);
+        double a[9], aaa, bbb;
+        velgrad64<true>(p, i, j, k, p.f.u, p.f.v, p.f.w, a);
+        vreman64(a, T.lx[i].x, T.ly[j].x, T.lz[k].x, aaa, bbb);
+        const long long q = p.g.ix(i, j, k);
+        const double nu = aaa == 0.0 ? 0.0 : sqrt(bbb / aaa);
+        if (!dynamic) {
+            p.f.nusgs[q] = p.c.csgsts * nu;
+            continue;
+        }
+        p.f.nusgs[q] = nu;
+        const double nh = 0.5 * nu;
+        double *const *m = p.f.scr + 3;
+        m[0][q] = nu * a[0]; m[1][q] = nh * (a[3] + a[1]); m[2][q] = nh * (a[6] + a[2]);
+        m[3][q] = nu * a[4]; m[4][q] = nh * (a[7] + a[5]); m[5][q] = nu * a[8];
+#pragma unroll
+        for (int l = 0; l < 9; l++) p.f.scr[9 + l][q] = a[l];
     }
 }
 
@@ -259,6 +300,30 @@ __global__ void __launch_bounds__(kThreads) k_vreman2(KP p, Box b) {
         scr<R>(p, 3)[q] = u1; scr<R>(p, 4)[q] = u2; scr<R>(p, 5)[q] = u3;
         scr<R>(p, 6)[q] = u1 * u1; scr<R>(p, 7)[q] = u1 * u2; scr<R>(p, 8)[q] = u1 * u3;
         scr<R>(p, 9)[q] = u2 * u2; scr<R>(p, 10)[q] = u2 * u3; scr<R>(p, 11)[q] = u3 * u3;
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_vreman2_64(KP p, Box b) {
+    const Stn &T = p.st;
+    GRID_LOOP(b) {
+        int i, j, k;
+        b.at(tt, i, j, k);
+        const long long q = p.g.ix(i, j, k);
+        double a[9], aaa, bbb;
+#pragma unroll
+        for (int l = 0; l < 9; l++) a[l] = p.f.scr[24 + l][q];
+        vreman64(a, T.lx[i].y, T.ly[j].y, T.lz[k].y, aaa, bbb);
+        const double nu = aaa == 0.0 ? 0.0 : sqrt(bbb / aaa), nh = 0.5 * nu;
+        double *const *m = p.f.scr + 18;
+        m[0][q] = nu * a[0] - m[0][q]; m[1][q] = nh * (a[3] + a[1]) - m[1][q]; m[2][q] = nh * (a[6] + a[2]) - m[2][q];
+        m[3][q] = nu * a[4] - m[3][q]; m[4][q] = nh * (a[7] + a[5]) - m[4][q]; m[5][q] = nu * a[8] - m[5][q];
+        const double u1 = 0.5 * (p.f.u[q] + p.f.u[q + 1]);
+        const double u2 = 0.5 * (p.f.v[q] + p.f.v[q + p.g.sx]);
+        const double u3 = 0.5 * (p.f.w[q] + p.f.w[q + p.g.sxy]);
+        double *const *o = p.f.scr + 3;
+        o[0][q] = u1; o[1][q] = u2; o[2][q] = u3;
+        o[3][q] = u1 * u1; o[4][q] = u1 * u2; o[5][q] = u1 * u3;
+        o[6][q] = u2 * u2; o[7][q] = u2 * u3; o[8][q] = u3 * u3;
     }
 }
 
@@ -459,14 +524,14 @@ void launch_sgs(lesgpu_case *c) {
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     if (c->kp.c.idvmon == 1) {
         if (mixed(c)) k_vreman1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
-        else k_vreman1<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
+        else k_vreman1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
         FiltBatch F{};
         F.na = 15;
         for (int m = 0; m < 6; m++) { F.src[m] = f.scr[3 + m]; F.dst[m] = f.scr[18 + m]; }
         for (int m = 0; m < 9; m++) { F.src[6 + m] = f.scr[9 + m]; F.dst[6 + m] = f.scr[24 + m]; }
         filter_batch(c, F);
         if (mixed(c)) k_vreman2<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
-        else k_vreman2<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+        else k_vreman2_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
         FiltBatch G{};
         G.na = 9;
         for (int m = 0; m < 9; m++) { G.src[m] = f.scr[3 + m]; G.dst[m] = f.scr[24 + m]; }
@@ -476,7 +541,7 @@ void launch_sgs(lesgpu_case *c) {
         k_scale<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, f.nusgs, 0);
     } else {
         if (mixed(c)) k_vreman1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
-        else k_vreman1<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
+        else k_vreman1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
     }
 }
 
@@ -496,16 +561,18 @@ __global__ void __launch_bounds__(kThreads) k_edm1(KP p, Box b, int dynamic) {
         b.at(tt, i, j, k);
         R d[9], s[6], alp[3];
         velgrad<R>(p, i, j, k, d, s);
-        R del = pow(R(M.f2fx[i]) * R(M.f2fy[j]) * R(M.f2fz[k]), R(1.0) / R(3.0));
+        // squared filter width, (f2fx f2fy f2fz)^(2/3), as the product of
+        // tabulated cube roots: a pow per cell was most of the FP64 kernel
+        const R del2 = M.dx[i] * M.dy[j] * M.dz[k];
         R sss = s[0] * s[0] + R(2.0) * s[1] * s[1] + R(2.0) * s[2] * s[2] + s[3] * s[3] + R(2.0) * s[4] * s[4] + s[5] * s[5];
         if (sss < R(1.0e-16)) sss = R(1.0e-16);
         long long q = g.ix(i, j, k);
         if (!dynamic) {
-            p.f.alsgs[q] = R(p.c.csgshf) * (del * del) * sqrt(R(2.0) * sss);
+            p.f.alsgs[q] = R(p.c.csgshf) * del2 * sqrt(R(2.0) * sss);
             continue;
         }
         temgrad<R>(p, i, j, k, alp);
-        R al = (del * del) * sqrt(R(2.0) * sss);
+        R al = del2 * sqrt(R(2.0) * sss);
         p.f.alsgs[q] = al;
 #pragma unroll
         for (int m = 0; m < 3; m++) scr<R>(p, 3 + m)[q] = al * alp[m];
@@ -513,6 +580,45 @@ __global__ void __launch_bounds__(kThreads) k_edm1(KP p, Box b, int dynamic) {
         for (int m = 0; m < 6; m++) scr<R>(p, 6 + m)[q] = s[m];
 #pragma unroll
         for (int m = 0; m < 3; m++) scr<R>(p, 12 + m)[q] = alp[m];
+    }
+}
+
+// The FP64 form (k_grad64.cuh): 64^3 150 us -> 43 (the pow of the filter width
+// alone was some 150 operations).
+__global__ void __launch_bounds__(kThreads) k_edm1_64(KP p, Box b, int dynamic) {
+    const DGrid &g = p.g;
+    const Stn &T = p.st;
+    GRID_LOOP(b) {
+        int i, j, k;
+        b.at(tt, i, j, k);
+        const long long q = g.ix(i, j, k);
+        double a[9];
+        velgrad64<true>(p, i, j, k, p.f.u, p.f.v, p.f.w, a);
+        const double s1 = 0.5 * (a[3] + a[1]), s2 = 0.5 * (a[6] + a[2]), s4 = 0.5 * (a[7] + a[5]);
+        const double dg = a[0] * a[0] + a[4] * a[4] + a[8] * a[8], od = s1 * s1 + s2 * s2 + s4 * s4;
+        double sss = fma(2.0, od, dg);
+        if (sss < 1.0e-16) sss = 1.0e-16;
+        const double al = (T.lx[i].z * T.ly[j].z) * T.lz[k].z * sqrt(2.0 * sss);
+        if (!dynamic) {
+            p.f.alsgs[q] = p.c.csgshf * al;
+            continue;
+        }
+        p.f.alsgs[q] = al;
+        const double4 X = T.dwx[i], Y = T.dwy[j], Z = T.dwz[k];
+        const double *t = p.f.t;
+        const double tq = t[q];
+        const double tg[3] = {
+            2.0 * (X.x * t[g.ix(g.imv[i], j, k)] + X.y * tq + X.z * t[g.ix(g.ipv[i], j, k)]),
+            2.0 * (Y.x * t[g.ix(i, g.jmv[j], k)] + Y.y * tq + Y.z * t[g.ix(i, g.jpv[j], k)]),
+            2.0 * (Z.x * t[g.ix(i, j, g.kmv[k])] + Z.y * tq + Z.z * t[g.ix(i, j, g.kpv[k])])};
+        double *const *m = p.f.scr + 3;
+#pragma unroll
+        for (int l = 0; l < 3; l++) {
+            m[l][q] = al * tg[l];
+            m[9 + l][q] = tg[l];
+        }
+        m[3][q] = a[0]; m[4][q] = s1; m[5][q] = s2;
+        m[6][q] = a[4]; m[7][q] = s4; m[8][q] = a[8];
     }
 }
 
@@ -527,15 +633,12 @@ __global__ void __launch_bounds__(kThreads) k_edm2(KP p, Box b) {
         int i, j, k;
         b.at(tt, i, j, k);
         long long q = g.ix(i, j, k);
-        R d1 = tf_width<R>(M.f2fx, g.fixil, g.fixiu, i);
-        R d2 = tf_width<R>(M.f2fy, g.fixjl, g.fixju, j);
-        R d3 = tf_width<R>(M.f2fz, g.fixkl, g.fixku, k);
-        R del = pow(d1 * d2 * d3, R(1.0) / R(3.0));
+        const R del2 = M.ex[i] * M.ey[j] * M.ez[k];
         R s0 = scr<R>(p, 21)[q], s1 = scr<R>(p, 22)[q], s2 = scr<R>(p, 23)[q];
         R s3 = scr<R>(p, 24)[q], s4 = scr<R>(p, 25)[q], s5 = scr<R>(p, 26)[q];
         R sss = s0 * s0 + R(2.0) * s1 * s1 + R(2.0) * s2 * s2 + s3 * s3 + R(2.0) * s4 * s4 + s5 * s5;
         if (sss < R(1.0e-16)) sss = R(1.0e-16);
-        R ami = (del * del) * sqrt(R(2.0) * sss);
+        R ami = del2 * sqrt(R(2.0) * sss);
 #pragma unroll
         for (int m = 0; m < 3; m++) scr<R>(p, 18 + m)[q] = ami * scr<R>(p, 27 + m)[q] - scr<R>(p, 18 + m)[q];
         R u1 = R(0.5) * (R(M.u[q]) + R(M.u[q + 1]));
@@ -545,6 +648,29 @@ __global__ void __launch_bounds__(kThreads) k_edm2(KP p, Box b) {
         scr<R>(p, 3)[q] = u1; scr<R>(p, 4)[q] = u2; scr<R>(p, 5)[q] = u3;
         scr<R>(p, 6)[q] = tq;
         scr<R>(p, 7)[q] = u1 * tq; scr<R>(p, 8)[q] = u2 * tq; scr<R>(p, 9)[q] = u3 * tq;
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_edm2_64(KP p, Box b) {
+    const Stn &T = p.st;
+    GRID_LOOP(b) {
+        int i, j, k;
+        b.at(tt, i, j, k);
+        const long long q = p.g.ix(i, j, k);
+        const double s0 = p.f.scr[21][q], s1 = p.f.scr[22][q], s2 = p.f.scr[23][q];
+        const double s3 = p.f.scr[24][q], s4 = p.f.scr[25][q], s5 = p.f.scr[26][q];
+        double sss = fma(2.0, s1 * s1 + s2 * s2 + s4 * s4, s0 * s0 + s3 * s3 + s5 * s5);
+        if (sss < 1.0e-16) sss = 1.0e-16;
+        const double al = (T.lx[i].w * T.ly[j].w) * T.lz[k].w * sqrt(2.0 * sss);
+#pragma unroll
+        for (int m = 0; m < 3; m++) p.f.scr[18 + m][q] = al * p.f.scr[27 + m][q] - p.f.scr[18 + m][q];
+        const double u1 = 0.5 * (p.f.u[q] + p.f.u[q + 1]);
+        const double u2 = 0.5 * (p.f.v[q] + p.f.v[q + p.g.sx]);
+        const double u3 = 0.5 * (p.f.w[q] + p.f.w[q + p.g.sxy]);
+        const double tq = p.f.t[q];
+        double *const *o = p.f.scr + 3;
+        o[0][q] = u1; o[1][q] = u2; o[2][q] = u3; o[3][q] = tq;
+        o[4][q] = u1 * tq; o[5][q] = u2 * tq; o[6][q] = u3 * tq;
     }
 }
 
@@ -579,14 +705,14 @@ void launch_sgs_t(lesgpu_case *c) {
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     if (c->kp.c.idvmon == 1) {
         if (mixed(c)) k_edm1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
-        else k_edm1<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
+        else k_edm1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
         FiltBatch F{};
         F.na = 12;
         for (int m = 0; m < 3; m++) { F.src[m] = f.scr[3 + m]; F.dst[m] = f.scr[18 + m]; }
         for (int m = 0; m < 9; m++) { F.src[3 + m] = f.scr[6 + m]; F.dst[3 + m] = f.scr[21 + m]; }
         filter_batch(c, F);
         if (mixed(c)) k_edm2<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
-        else k_edm2<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+        else k_edm2_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
         FiltBatch G{};
         G.na = 7;
         for (int m = 0; m < 7; m++) { G.src[m] = f.scr[3 + m]; G.dst[m] = f.scr[24 + m]; }
@@ -596,7 +722,7 @@ void launch_sgs_t(lesgpu_case *c) {
         k_scale<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, f.alsgs, 1);
     } else {
         if (mixed(c)) k_edm1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
-        else k_edm1<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
+        else k_edm1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
     }
 }
 

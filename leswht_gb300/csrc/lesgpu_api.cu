@@ -466,6 +466,52 @@ extern "C" int lesgpu_create(const lesgpu_config *cfg, const lesgpu_grid *g, les
         m.aiu = f.aiu; m.ciu = f.ciu; m.aivw = f.aivw; m.civw = f.civw; m.ajv = f.ajv; m.cjv = f.cjv;
         m.ajuw = f.ajuw; m.cjuw = f.cjuw; m.akw = f.akw; m.ckw = f.ckw; m.akuv = f.akuv; m.ckuv = f.ckuv;
         m.cfx1 = f.cfx1; m.cfy1 = f.cfy1; m.cfz1 = f.cfz1;
+        struct Axis {
+            const double *f, *fi, *ci;                       // f2f, f2fi, c2ci (0:n)
+            const int64_t *pv, *mv, *fl, *fu;                // (1:n-1)
+            long long n;
+            const double2 **face[2];                         // ghost, wrapped
+            const double4 **der[2], **width;
+            const double **quarter, **d, **e;
+        };
+        Stn &st = c->kp.st;
+        const Axis axes[3] = {
+            {g->f2fx, g->f2fxi, g->c2cxi, g->ipv, g->imv, g->fixil, g->fixiu, d.n1, {&st.gx, &st.wx}, {&st.dgx, &st.dwx}, &st.lx, &st.qx, &m.dx, &m.ex},
+            {g->f2fy, g->f2fyi, g->c2cyi, g->jpv, g->jmv, g->fixjl, g->fixju, d.n2, {&st.gy, &st.wy}, {&st.dgy, &st.dwy}, &st.ly, &st.qy, &m.dy, &m.ey},
+            {g->f2fz, g->f2fzi, g->c2czi, g->kpv, g->kmv, g->fixkl, g->fixku, d.n3, {&st.gz, &st.wz}, {&st.dgz, &st.dwz}, &st.lz, &st.qz, &m.dz, &m.ez}};
+        for (const Axis &x : axes) {
+            const long long n = x.n, nm = n - 1;
+            std::vector<double> quarter(n + 1), dv(n + 1, 0.0), ev(n + 1, 0.0);
+            std::vector<double4> width(n + 1, make_double4(0, 0, 0, 0));
+            for (long long i = 0; i <= n; i++) quarter[i] = 0.25 * x.ci[i];
+            for (long long i = 1; i <= nm; i++) {
+                const double t = 0.5 * x.f[i - 1] * (1.0 - (double)x.fu[i - 1]) + x.f[i] + 0.5 * x.f[i + 1] * (1.0 - (double)x.fl[i - 1]);
+                dv[i] = cbrt(x.f[i] * x.f[i]);
+                ev[i] = cbrt(t * t);
+                width[i] = make_double4(x.f[i], t, dv[i], ev[i]);
+            }
+            *x.quarter = upload(A, quarter.data(), quarter.size());
+            *x.width = upload(A, width.data(), width.size());
+            *x.d = upload(A, dv.data(), dv.size());
+            *x.e = upload(A, ev.data(), ev.size());
+            for (int wrap = 0; wrap < 2; wrap++) {
+                std::vector<double2> face(n + 1, make_double2(0, 0));
+                std::vector<double4> der(n + 1, make_double4(0, 0, 0, 0));
+                for (long long q = 1; q <= n; q++) {
+                    const double wall = q < n ? (double)x.fl[q - 1] : (double)x.fu[nm - 1];
+                    const long long lo = wrap && q < n ? (long long)x.mv[q - 1] : q - 1;
+                    const double k = 0.5 * x.ci[q] * (1.0 - wall);
+                    face[q] = make_double2(k * x.f[q] + (q < n ? wall : 0.0), k * x.f[lo] + (q < n ? 0.0 : wall));
+                }
+                for (long long i = 1; i <= nm; i++) {
+                    const double2 a = face[i], b = face[wrap ? (long long)x.pv[i - 1] : i + 1];
+                    const double h = 0.5 * x.fi[i];
+                    der[i] = make_double4(-h * a.x, h * (b.x - a.y), h * b.y, 0.0);
+                }
+                *x.face[wrap] = upload(A, face.data(), face.size());
+                *x.der[wrap] = upload(A, der.data(), der.size());
+            }
+        }
         auto flags = [&](const int64_t *src, long long n) {     // (1:n) int64 -> (0:n+1) double
             std::vector<double> h(n + 2, 0.0);
             for (long long q = 1; q <= n; q++) h[q] = (double)src[q - 1];
@@ -503,6 +549,8 @@ extern "C" int lesgpu_create(const lesgpu_config *cfg, const lesgpu_grid *g, les
             r.aiu = v32(f.aiu, nx); r.ciu = v32(f.ciu, nx); r.aivw = v32(f.aivw, nx); r.civw = v32(f.civw, nx);
             r.ajv = v32(f.ajv, ny); r.cjv = v32(f.cjv, ny); r.ajuw = v32(f.ajuw, ny); r.cjuw = v32(f.cjuw, ny);
             r.akw = v32(f.akw, nz); r.ckw = v32(f.ckw, nz); r.akuv = v32(f.akuv, nz); r.ckuv = v32(f.ckuv, nz);
+            r.dx = v32(m.dx, d.n1 + 1); r.dy = v32(m.dy, d.n2 + 1); r.dz = v32(m.dz, d.n3 + 1);
+            r.ex = v32(m.ex, d.n1 + 1); r.ey = v32(m.ey, d.n2 + 1); r.ez = v32(m.ez, d.n3 + 1);
             r.cfx1 = v32(f.cfx1, 3 * (d.n1m + 2)); r.cfy1 = v32(f.cfy1, 3 * (d.n2m + 2)); r.cfz1 = v32(f.cfz1, 3 * (d.n3m + 2));
             r.fixil = v32(m.fixil, d.n1m + 2); r.fixiu = v32(m.fixiu, d.n1m + 2);
             r.fixjl = v32(m.fixjl, d.n2m + 2); r.fixju = v32(m.fixju, d.n2m + 2);

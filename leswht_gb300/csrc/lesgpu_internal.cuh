@@ -70,6 +70,7 @@ struct DScal {
     // volumes of the fluid, summed once (launch_red_weights): u points and cells
     // with the flow-rate weights, cells with f2fx f2fy f2fz
     double flowvol, cellvol, fluidvol;
+    double hub;               // 0.5 / u_bulk_t
     double qcur;              // flow rate of the projected u (qvol(0) under ICH = 1)
     double tbulk_sum;         // sum of t over the fluid cells (writehistory)
     double csgsts, csgshf, nutavg, nutmax, alpavg, alpmax;
@@ -170,9 +171,23 @@ struct Mir {
     const T *f2fx, *f2fy, *f2fz, *f2fxi, *f2fyi, *f2fzi, *c2cxi, *c2cyi, *c2czi;
     const T *aiu, *ciu, *aivw, *civw, *ajv, *cjv, *ajuw, *cjuw, *akw, *ckw, *akuv, *ckuv;
     const T *cfx1, *cfy1, *cfz1;     // test-filter weights
+    // cube roots of the squared cell widths (d) and test-filter widths (e)
+    const T *dx, *dy, *dz, *ex, *ey, *ez;
     // the wall flags fix?? (1-based) as T: a stencil loads them instead of
     // converting an int per cell (conversions issue on GB300's FP64 pipe)
     const T *fixil, *fixiu, *fixjl, *fixju, *fixkl, *fixku;
+};
+
+// 1-D weights of the FP64 stencils (k_grad64.cuh), indices 0 .. n:
+//  g? / w?  value at face f (between cells f - 1 and f) = x lower + y upper,
+//           the wall flags folded in; neighbours by ghost layer / wrapped
+//  dg? dw?  half the derivative over cell i of that value: x lower + y own + z upper
+//  l?       cell width, test-filter width, and the cube roots of their squares
+//  q?       c2ci / 4
+struct Stn {
+    const double2 *gx, *gy, *gz, *wx, *wy, *wz;
+    const double4 *dgx, *dgy, *dgz, *dwx, *dwy, *dwz, *lx, *ly, *lz;
+    const double *qx, *qy, *qz;
 };
 
 struct KP {                   // everything a kernel may read, passed by value
@@ -182,6 +197,7 @@ struct KP {                   // everything a kernel may read, passed by value
     DScal *S;
     Mir<double> md;
     Mir<float> mf;            // mixed form only (null otherwise)
+    Stn st;
 };
 
 template <class R> __device__ __forceinline__ R pickr(double d, float f);
