@@ -6,10 +6,9 @@
 //
 // The reference filters each of its 24 temporaries with two full-array
 // passes (x, then z) through stack copies.  Here one kernel filters a whole
-// batch of arrays in a single pass: for output (i,k) it rebuilds the three
-// x-filtered values at k-1, k, k+1 in registers and applies the z weights to
-// them, which is the reference's arithmetic with its rounding order and a
-// third of its memory traffic.
+// batch of arrays in a single pass: it keeps the x-filtered values at k-1, k,
+// k+1 in registers and applies the z weights to them, with a third of the
+// reference's memory traffic.
 #include "k_grad64.cuh"
 
 namespace lg {
@@ -203,58 +202,74 @@ struct FiltBatch {
     int na;
 };
 
-// One cell's x filter (sgs.f90:650-733) of the rows qm, q0, qp of every array
-// of the batch is formed from the same offsets and weights: the cell's index
-// decoding, periodic wrap and weights are computed once for all arrays.
-struct FiltX {
-    int im, ip;              // x neighbours (wrapped); == i when x is not filtered here
-    bool filt;
-};
+// One thread filters `run` consecutive planes of one (i, j) of kFiltA arrays
+// (the blockIdx.y-th group): the x-filtered values of planes k - 1, k, k + 1
+// roll through registers, so a plane's x filter (sgs.f90:650-733) is formed
+// once and its three values loaded once, where a thread per cell forms and
+// loads them three times over (12 FP64 operations and 9 loads a value against
+// 6 and 4).  The arrays share the addresses and weights, which in FP32 are
+// most of the instructions.  The mean of a step's four
+// launches, us: 64^3 FP64 63 -> 43, FP32 12.9 -> 9.5; 384x256x384 FP32
+// 1479 -> 860.
+constexpr int kFiltA = 3;
 
 template <class R>
-__global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F) {
+__global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F, int run) {
     const DGrid &g = p.g;
-    const int xf = (p.c.filter == 1 || p.c.filter == 3) ? 1 : 0;
-    const int zf = (p.c.filter == 2 || p.c.filter == 3) ? 1 : 0;
+    const bool xf = p.c.filter == 1 || p.c.filter == 3, zf = p.c.filter == 2 || p.c.filter == 3;
+    const int a0 = blockIdx.y * kFiltA, na = F.na - a0 < kFiltA ? F.na - a0 : kFiltA;
+    const R *__restrict__ s[kFiltA];
+    R *__restrict__ d[kFiltA];
+#pragma unroll
+    for (int a = 0; a < kFiltA; a++) {               // a short group repeats its last array
+        s[a] = static_cast<const R *>(F.src[a0 + (a < na ? a : na - 1)]);
+        d[a] = static_cast<R *>(F.dst[a0 + (a < na ? a : na - 1)]);
+    }
     const long long n = b.count();
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        b.at(t, i, j, k);
+        int i, j, kc;
+        b.at(t, i, j, kc);
+        const int ka = (kc - 1) * run + 1, kb = ka + run - 1 < g.n3m ? ka + run - 1 : g.n3m;
         // x: interior points use i-1, i, i+1; x-periodic ends wrap (with n1m = 1
         // the value is unfiltered); other ends are unfiltered
-        FiltX X{i, i, false};
+        int om = 0, op = 0;
         if (xf) {
-            if (i >= 2 && i <= g.n1m - 1) X = FiltX{i - 1, i + 1, true};
-            else if (p.c.xprdic == 1 && g.n1m > 1) X = FiltX{i == 1 ? g.n1m : g.n1m - 1, i == 1 ? 2 : 1, true};
+            if (i >= 2 && i <= g.n1m - 1) { om = -1; op = 1; }
+            else if (p.c.xprdic == 1 && g.n1m > 1) { om = i == 1 ? g.n1m - 1 : -1; op = i == 1 ? 1 : 1 - i; }
         }
+        const bool filt = op != 0;
         const R *cfx = mir<R>(p).cfx1 + 3 * i;
-        const R c0 = X.filt ? R(cfx[0]) : R(0.0), c1 = X.filt ? R(cfx[1]) : R(0.0), c2 = X.filt ? R(cfx[2]) : R(0.0);
-        // z-periodic ends use the wrapped neighbours; with n3m = 1 the weights
-        // are zero (sgsfilterinit skips them), so the filtered value is 0 as
-        // in test_filter (sgs.f90:735-764)
-        const bool zin = zf && ((k >= 2 && k <= g.n3m - 1) || p.c.zprdic == 1);
-        const int km = k == 1 ? g.n3m : k - 1, kp = k == g.n3m ? 1 : k + 1;
-        const R *cfz = mir<R>(p).cfz1 + 3 * k;
-        const R z0 = zin ? R(cfz[0]) : R(0.0), z1 = zin ? R(cfz[1]) : R(0.0), z2 = zin ? R(cfz[2]) : R(0.0);
-        const long long r0 = g.ix(0, j, k), rm = g.ix(0, j, km), rp = g.ix(0, j, kp);
-        // sources and destinations are distinct arrays: two arrays' loads
-        // can be in flight at once
-#pragma unroll 2
-        for (int a = 0; a < F.na; a++) {
-            const R *__restrict__ s = static_cast<const R *>(F.src[a]);
-            R *__restrict__ d = static_cast<R *>(F.dst[a]);
-            R out;
-            if (!zin) {
-                out = X.filt ? c0 * s[r0 + X.im] + c1 * s[r0 + i] + c2 * s[r0 + X.ip] : s[r0 + i];
-            } else if (X.filt) {
-                const R xm = c0 * s[rm + X.im] + c1 * s[rm + i] + c2 * s[rm + X.ip];
-                const R x0 = c0 * s[r0 + X.im] + c1 * s[r0 + i] + c2 * s[r0 + X.ip];
-                const R xp = c0 * s[rp + X.im] + c1 * s[rp + i] + c2 * s[rp + X.ip];
-                out = z0 * xm + z1 * x0 + z2 * xp;
-            } else {
-                out = z0 * s[rm + i] + z1 * s[r0 + i] + z2 * s[rp + i];
+        const R c0 = cfx[0], c1 = cfx[1], c2 = cfx[2];
+        auto xval = [&](const R *__restrict__ r) {
+            const R x = r[0], y = fma(c2, r[op], fma(c0, r[om], c1 * x));
+            return filt ? y : x;
+        };
+        R xm[kFiltA], x0[kFiltA];
+        const long long qa = g.ix(i, j, ka), qm = g.ix(i, j, ka == 1 ? g.n3m : ka - 1);
+#pragma unroll
+        for (int a = 0; a < kFiltA; a++) {
+            x0[a] = xval(s[a] + qa);
+            xm[a] = xval(s[a] + qm);
+        }
+        const R *cfz = mir<R>(p).cfz1 + 3 * ka;
+        long long q = qa;
+        for (int k = ka; k <= kb; k++, q += g.sxy, cfz += 3) {
+            // z-periodic ends use the wrapped neighbours; with n3m = 1 the weights
+            // are zero (sgsfilterinit skips them), so the filtered value is 0 as
+            // in test_filter (sgs.f90:735-764)
+            const long long qp = k == g.n3m ? g.ix(i, j, 1) : q + g.sxy;
+            const bool zin = zf && ((k >= 2 && k <= g.n3m - 1) || p.c.zprdic == 1);
+            const R z0 = cfz[0], z1 = cfz[1], z2 = cfz[2];
+            R xp[kFiltA];
+#pragma unroll
+            for (int a = 0; a < kFiltA; a++) xp[a] = xval(s[a] + qp);
+#pragma unroll
+            for (int a = 0; a < kFiltA; a++) {
+                const R y = fma(z2, xp[a], fma(z0, xm[a], z1 * x0[a]));
+                if (a < na) d[a][q] = zin ? y : x0[a];
+                xm[a] = x0[a];
+                x0[a] = xp[a];
             }
-            d[r0 + i] = out;
         }
     }
 }
@@ -263,10 +278,16 @@ static bool mixed(const lesgpu_case *c) { return c->cfg.precision == LESGPU_PREC
 
 static void filter_batch(lesgpu_case *c, FiltBatch &F) {
     const DGrid &g = c->kp.g;
-    Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
+    // planes a thread: eight while that still fills the GPU's thread slots, in
+    // FP64 a quarter of them (its pipe is busy with that), fewer on small boxes
+    const int groups = (F.na + kFiltA - 1) / kFiltA;
+    int run = 8;
+    while (run > 1 && (long long)g.n1m * g.n2m * ((g.n3m + run - 1) / run) * groups < 152LL * (mixed(c) ? 2048 : 512)) run >>= 1;
+    Box b{1, 1, 1, g.n1m, g.n2m, (g.n3m + run - 1) / run};
+    const dim3 grid((unsigned)blocks_for(b.count()), (unsigned)groups);
     inst_begin(c, LESGPU_K_SGS);
-    if (mixed(c)) k_filter<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, F);
-    else k_filter<double><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, F);
+    if (mixed(c)) k_filter<float><<<grid, kThreads, 0, c->stream>>>(c->kp, b, F, run);
+    else k_filter<double><<<grid, kThreads, 0, c->stream>>>(c->kp, b, F, run);
     inst_end(c, LESGPU_K_SGS);
 }
 
