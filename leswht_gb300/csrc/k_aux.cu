@@ -18,13 +18,16 @@ static Box interior(const DGrid &g) { return Box{1, 1, 1, g.n1m, g.n2m, g.n3m}; 
 // The reference multiplies each cell's sum by dt before the max; dt > 0 so
 // max(s)*dt is the same rounded value.
 struct CflTerm {
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+    static constexpr int kLoads = 1;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
         const DGrid &g = p.g;
-        long long q = g.ix(i, j, k);
-        double c1 = fabs(p.f.u[q] + p.f.u[q + 1]) * 0.5 * g.f2fxi[i];
-        double c2 = fabs(p.f.v[q] + p.f.v[q + g.sx]) * 0.5 * g.f2fyi[j];
-        double c3 = fabs(p.f.w[q] + p.f.w[q + g.sxy]) * 0.5 * g.f2fzi[k];
-        w[0] = c1 + c2 + c3;
+        const long long q = g.ix(i, j, k);
+        const double c1 = abs_bits(p.f.u[q] + p.f.u[q + 1]), c2 = abs_bits(p.f.v[q] + p.f.v[q + g.sx]);
+        const double c3 = abs_bits(p.f.w[q] + p.f.w[q + g.sxy]);
+        x[0] = fma(c3, p.st.hz[k], fma(c2, p.st.hy[j], c1 * p.st.hx[i]));
+    }
+    __device__ void add(const KP &, int, int, int, const double *x, double *v) const {
+        take_max(v[0], x[0]);
     }
 };
 
@@ -88,8 +91,16 @@ __global__ void k_substepinit(KP p, int s, int carry) {
     const double gam[4] = {0.0, 8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
     const double ro[4] = {0.0, 0.0, -17.0 / 60.0, -5.0 / 12.0};
     DScal *S = p.S;
+    // the projection's metric factors (k_ucalc), a multiplication per line
+    // and not one per cell
+    const double dtc = S->dt * (gam[s] + ro[s]);
+    const DGrid &g = p.g;
+    for (int i = threadIdx.x; i <= g.n1; i += blockDim.x) p.st.px[i] = dtc * g.c2cxi[i];
+    for (int j = threadIdx.x; j <= g.n2; j += blockDim.x) p.st.py[j] = dtc * g.c2cyi[j];
+    for (int k = threadIdx.x; k <= g.n3; k += blockDim.x) p.st.pz[k] = dtc * g.c2czi[k];
+    if (threadIdx.x != 0) return;
     S->alpha = 0.5 * (gam[s] + ro[s]);
-    S->dtconst = S->dt * (gam[s] + ro[s]);
+    S->dtconst = dtc;
     S->dtconsti = 1.0 / S->dtconst;
     S->test1 = p.c.resid1 * S->dtconsti;
     S->acoef = S->alpha * S->dt / p.c.re;
@@ -100,15 +111,18 @@ __global__ void k_substepinit(KP p, int s, int carry) {
 }
 
 void launch_substepinit(lesgpu_case *c, int msub, bool carry) {
-    k_substepinit<<<1, 1, 0, c->stream>>>(c->kp, msub, carry ? 1 : 0);
+    k_substepinit<<<1, kThreads, 0, c->stream>>>(c->kp, msub, carry ? 1 : 0);
 }
 
 // ------------------------------------------------------------ qvol / tvol
 struct QvolTerm {   // qvolcalc, slv_auxi.f90:126-149
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
-        long long q = p.g.ix(i, j, k);
-        w[0] = p.f.u[q] * p.f.wq[q];     // u c2cx f2fy f2fz over the fluid u points
+    static constexpr int kLoads = 2;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
+        const long long q = p.g.ix(i, j, k);
+        x[0] = p.f.u[q];
+        x[1] = p.f.wq[q];                // c2cx f2fy f2fz over the fluid u points
     }
+    __device__ void add(const KP &p, int i, int j, int k, const double *x, double *v) const { v[0] = fma(x[0], x[1], v[0]); }
 };
 struct QvolFinal {
     int slot;
@@ -117,10 +131,13 @@ struct QvolFinal {
 void launch_qvolcalc(lesgpu_case *c, int slot) { reduce<1, 0u>(c, interior(c->kp.g), QvolTerm{}, QvolFinal{slot}); }
 
 struct TvolTerm {   // tvolcalc, slv_auxi.f90:152-173
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
-        long long q = p.g.ix(i, j, k);
-        w[0] = p.f.t[q] * p.f.wt[q];     // t / c* f2fx f2fy f2fz
+    static constexpr int kLoads = 2;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
+        const long long q = p.g.ix(i, j, k);
+        x[0] = p.f.t[q];
+        x[1] = p.f.wt[q];                // f2fx f2fy f2fz / c*
     }
+    __device__ void add(const KP &p, int i, int j, int k, const double *x, double *v) const { v[0] = fma(x[0], x[1], v[0]); }
 };
 struct TvolFinal {
     int slot;
@@ -193,11 +210,16 @@ struct TvolCorrFinal {
 };
 // the same with the fluid cells' temperature sum of writehistory
 struct TvolBulkTerm {
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+    static constexpr int kLoads = 3;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
         const long long q = p.g.ix(i, j, k);
-        const double t = p.f.t[q];
-        w[0] = t * p.f.wt[q];
-        w[1] = t * p.f.wb[q];
+        x[0] = p.f.t[q];
+        x[1] = p.f.wt[q];
+        x[2] = p.f.wb[q];
+    }
+    __device__ void add(const KP &p, int i, int j, int k, const double *x, double *v) const {
+        v[0] = fma(x[0], x[1], v[0]);
+        v[1] = fma(x[0], x[2], v[1]);
     }
 };
 struct TvolBulkFinal {
@@ -255,7 +277,7 @@ struct MeanpgWallTerm {
             if (j > g.n2m || (plane == 2 && c.bc_zbtm != 0) || (plane == 3 && c.bc_ztop != 0)) return;
         }
         const long long q = g.ix(i, j, k);
-        if (p.f.fb_u[q] < 1.0e-10) return;
+        if (!fluid(p.f.fb_u[q])) return;
         // the one-sided second-order wall gradient over re, its two weights
         // formed once on the host (per cell they cost four divisions)
         const long long in = plane == 0 ? g.sx : plane == 1 ? -g.sx : plane == 2 ? g.sxy : -g.sxy;
@@ -318,22 +340,15 @@ void launch_meanpg(lesgpu_case *c, bool have_q) {
 __global__ void __launch_bounds__(kThreads) k_ucalc(KP p, Box b) {
     long long n = b.count();
     const DGrid &g = p.g;
-    double dtc = p.S->dtconst;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         b.at(t, i, j, k);
         long long q = g.ix(i, j, k);
         const double *phi = p.f.phi;
         double ph = phi[q];
-        if (i >= g.i_bgpx) {
-            int im = g.imv[i];
-            p.f.u[q] = p.f.u[q] - dtc * (ph - phi[g.ix(im, j, k)]) * g.c2cxi[i];
-        }
-        if (j >= 2) p.f.v[q] = p.f.v[q] - dtc * (ph - phi[q - g.sx]) * g.c2cyi[j];
-        if (k >= g.k_bgpz) {
-            int km = g.kmv[k];
-            p.f.w[q] = p.f.w[q] - dtc * (ph - phi[g.ix(i, j, km)]) * g.c2czi[k];
-        }
+        if (i >= g.i_bgpx) p.f.u[q] = fma(phi[g.ix(g.imv[i], j, k)] - ph, p.st.px[i], p.f.u[q]);
+        if (j >= 2) p.f.v[q] = fma(phi[q - g.sx] - ph, p.st.py[j], p.f.v[q]);
+        if (k >= g.k_bgpz) p.f.w[q] = fma(phi[g.ix(i, j, g.kmv[k])] - ph, p.st.pz[k], p.f.w[q]);
     }
 }
 
@@ -380,19 +395,33 @@ void ghost(lesgpu_case *c, int dir, GhostSpec *s, int na) {
 // flow-rate term of the predicted u, the projection of u, v, w (which reads
 // only phi's neighbours), then the flow-rate term of the projected u.  The
 // sums run in the reduction kernel's own order, so qvol(2) and qvol(0) are
-// bitwise those of two separate qvolcalc launches.
+// bitwise those of two separate qvolcalc launches.  Eight FP64 operations a
+// cell (16 with dtconst multiplied in per cell and the sums unfused):
+// 384x256x384 922 us -> 559.
 struct UcalcQvolTerm {
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+    static constexpr int kLoads = 8;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
         const DGrid &g = p.g;
         const long long q = g.ix(i, j, k);
-        const double dtc = p.S->dtconst;
         const double *phi = p.f.phi;
-        w[0] = p.f.u[q] * p.f.wq[q];
-        const double ph = phi[q];
-        if (i >= g.i_bgpx) p.f.u[q] = p.f.u[q] - dtc * (ph - phi[g.ix(g.imv[i], j, k)]) * g.c2cxi[i];
-        if (j >= 2) p.f.v[q] = p.f.v[q] - dtc * (ph - phi[q - g.sx]) * g.c2cyi[j];
-        if (k >= g.k_bgpz) p.f.w[q] = p.f.w[q] - dtc * (ph - phi[g.ix(i, j, g.kmv[k])]) * g.c2czi[k];
-        w[1] = p.f.u[q] * p.f.wq[q];
+        x[0] = p.f.u[q];
+        x[1] = p.f.v[q];
+        x[2] = p.f.w[q];
+        x[3] = phi[q];
+        x[4] = phi[g.ix(g.imv[i], j, k)];
+        x[5] = phi[q - g.sx];
+        x[6] = phi[g.ix(i, j, g.kmv[k])];
+        x[7] = p.f.wq[q];
+    }
+    __device__ void add(const KP &p, int i, int j, int k, const double *x, double *v) const {
+        const DGrid &g = p.g;
+        const long long q = g.ix(i, j, k);
+        double u = x[0];
+        if (i >= g.i_bgpx) p.f.u[q] = u = fma(x[4] - x[3], p.st.px[i], u);
+        if (j >= 2) p.f.v[q] = fma(x[5] - x[3], p.st.py[j], x[1]);
+        if (k >= g.k_bgpz) p.f.w[q] = fma(x[6] - x[3], p.st.pz[k], x[2]);
+        v[0] = fma(x[0], x[7], v[0]);
+        v[1] = fma(u, x[7], v[1]);
     }
 };
 struct UcalcQvolFinal {
@@ -440,15 +469,14 @@ struct PhirefFinal {
 __global__ void __launch_bounds__(kThreads) k_pcalc(KP p, Box b) {
     long long n = b.count();
     const DGrid &g = p.g;
-    // 1/re (formed once) in place of a per-cell division: an FP64 division
-    // is some ten operations on the narrow FP64 pipe
-    double dtc = p.S->dtconst, phiref = p.S->phiref, rei = p.c.rei_d;
+    // three FP64 operations a cell, the factor formed once for a thread's cells
+    // (384x256x384 368 us with one cell a thread -> 240)
+    const double phiref = p.S->phiref, h = 0.5 * p.S->dtconst * p.c.rei_d;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         b.at(t, i, j, k);
         long long q = g.ix(i, j, k);
-        double pn = p.f.p[q] + p.f.phi[q] - 0.5 * dtc * p.f.divgsum[q] * rei;
-        p.f.p[q] = pn - phiref;
+        p.f.p[q] = fma(-h, p.f.divgsum[q], p.f.p[q] + (p.f.phi[q] - phiref));
     }
 }
 
@@ -461,7 +489,8 @@ void launch_ucalc_pcalc(lesgpu_case *c, bool with_qvol) {
     ucalc_interior(c, with_qvol);
     reduce<1, 0u>(c, Box{1, 1, 1, 1, g.n2m, g.n3m}, PhirefTerm{}, PhirefFinal{});
     Box b = interior(g);
-    k_pcalc<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+    const int nb = blocks_for(b.count());
+    k_pcalc<<<nb < 2 * kRedBlocks ? nb : 2 * kRedBlocks, kThreads, 0, c->stream>>>(c->kp, b);
     DFields &f = c->kp.f;
     if (c->kp.c.zprdic == 1) {
         GhostSpec s[4] = {{f.u, 1, g.n1, 0, g.n2}, {f.v, 0, g.n1, 1, g.n2}, {f.w, 0, g.n1, 0, g.n2}, {f.p, 1, g.n1m, 1, g.n2m}};
@@ -475,17 +504,26 @@ void launch_ucalc_pcalc(lesgpu_case *c, bool with_qvol) {
 
 // ------------------------------------------------------- end-of-step checks
 struct DivTerm {   // convergence_check, misc_init.f90:1047-1077
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+    static constexpr int kLoads = 3;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
         const DGrid &g = p.g;
-        long long q = g.ix(i, j, k);
-        double d1 = (p.f.u[q + 1] - p.f.u[q]) * g.f2fxi[i];
-        double d2 = (p.f.v[q + g.sx] - p.f.v[q]) * g.f2fyi[j];
-        double d3 = (p.f.w[q + g.sxy] - p.f.w[q]) * g.f2fzi[k];
-        double dv = (p.c.masson == 1) ? d1 + d2 + d3 - p.f.qmass[q] : d1 + d2 + d3;
-        w[0] = fabs(dv);
-        w[1] = fabs(p.f.qmass[q]);
-        double fin = p.f.u[q] + p.f.v[q] + p.f.w[q] + p.f.p[q];
-        w[2] = isfinite(fin) ? 0.0 : 1.0;
+        const long long q = g.ix(i, j, k);
+        const double u = p.f.u[q], v = p.f.v[q], z = p.f.w[q], r = p.f.p[q];
+        const double d1 = (p.f.u[q + 1] - u) * g.f2fxi[i];
+        const double d2 = (p.f.v[q + g.sx] - v) * g.f2fyi[j];
+        const double d3 = (p.f.w[q + g.sxy] - z) * g.f2fzi[k];
+        x[0] = d1 + d2 + d3;
+        x[1] = p.f.qmass[q];
+        // u + v + w + p finite, on the exponents: FP64 operations are this
+        // pass's time and a compiled fabs or maximum is some
+        // (384x256x384 1429 us so, 434 on the bits)
+        auto inf = [](double a) { return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000; };
+        x[2] = inf(u) | inf(v) | inf(z) | inf(r) ? 1.0 : 0.0;
+    }
+    __device__ void add(const KP &p, int, int, int, const double *x, double *v) const {
+        take_max(v[0], abs_bits(p.c.masson == 1 ? x[0] - x[1] : x[0]));
+        take_max(v[1], abs_bits(x[1]));
+        take_max(v[2], x[2]);
     }
 };
 // the last block also advances time (k_time_advance's work; the divergence

@@ -7,16 +7,21 @@
 namespace lg {
 
 struct UbulkTerm {
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+    static constexpr int kLoads = 3;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
         const long long q = p.g.ix(i, j, k);
-        w[0] = 0.5 * (p.f.u[q] + p.f.u[q + 1]) * p.f.wb[q];     // c2cx f2fy f2fz over the fluid cells, else 0
+        x[0] = p.f.u[q];
+        x[1] = p.f.u[q + 1];
+        x[2] = p.f.wb[q];                // c2cx f2fy f2fz over the fluid cells, else 0
     }
+    // twice the sum
+    __device__ void add(const KP &p, int i, int j, int k, const double *x, double *v) const { v[0] = fma(x[0] + x[1], x[2], v[0]); }
 };
 struct UbulkFinal {
     int carry;      // tvol(1) is tvol(0) of the substep before
     __device__ void operator()(const KP &p, const double *o) const {
         double ub;
-        if (p.S->cellvol > 1.0e-12) ub = o[0] / p.S->cellvol;
+        if (p.S->cellvol > 1.0e-12) ub = 0.5 * o[0] / p.S->cellvol;
         else if (fabs(p.c.udrv_i) > 1.0e-12) ub = p.c.udrv_i;
         else ub = 1.0;
         p.S->u_bulk_t = ub;
@@ -33,10 +38,16 @@ __global__ void k_set_ubulk_one(KP p, int carry) {
 // tvolcalc(tvol(1)) and the bulk velocity in one reduction (both read every
 // interior cell; each sum keeps the order of its own launch, bitwise)
 struct TvolUbulkTerm {
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
+    static constexpr int kLoads = 5;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
         const long long q = p.g.ix(i, j, k);
-        w[0] = p.f.t[q] * p.f.wt[q];
-        UbulkTerm{}(p, i, j, k, w + 1);
+        x[0] = p.f.t[q];
+        x[1] = p.f.wt[q];
+        UbulkTerm{}.load(p, i, j, k, x + 2);
+    }
+    __device__ void add(const KP &p, int i, int j, int k, const double *x, double *v) const {
+        v[0] = fma(x[0], x[1], v[0]);
+        UbulkTerm{}.add(p, i, j, k, x + 2, v + 1);
     }
 };
 struct TvolUbulkFinal {

@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F, i
         const R *cfx = mir<R>(p).cfx1 + 3 * i;
         const R c0 = cfx[0], c1 = cfx[1], c2 = cfx[2];
         auto xval = [&](const R *__restrict__ r) {
-            const R x = r[0], y = fma(c2, r[op], fma(c0, r[om], c1 * x));
+            const R x = r[0], y = fma(c2, r[op], fma(c1, x, c0 * r[om]));
             return filt ? y : x;
         };
         R xm[kFiltA], x0[kFiltA];
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F, i
             for (int a = 0; a < kFiltA; a++) xp[a] = xval(s[a] + qp);
 #pragma unroll
             for (int a = 0; a < kFiltA; a++) {
-                const R y = fma(z2, xp[a], fma(z0, xm[a], z1 * x0[a]));
+                const R y = fma(z2, xp[a], fma(z1, x0[a], z0 * xm[a]));
                 if (a < na) d[a][q] = zin ? y : x0[a];
                 xm[a] = x0[a];
                 x0[a] = xp[a];
@@ -374,42 +374,39 @@ struct CsgstsFinal {
     }
 };
 
-__global__ void k_scale(KP p, Box b, double *f, int which) {
-    double cs = which == 0 ? p.S->csgsts : p.S->csgshf;
-    GRID_LOOP(b) {
-        int i, j, k;
-        b.at(tt, i, j, k);
-        long long q = p.g.ix(i, j, k);
-        f[q] = cs * f[q];
-    }
-}
-
 __global__ void k_zero_list(KP p, double *f) {
     for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < p.c.nzero; l += gridDim.x * blockDim.x)
         f[p.g.ix(p.f.inz[l + 1], p.f.jnz[l + 1], p.f.knz[l + 1])] = 0.0;
 }
 
 // nutzero / alpzero statistics with the in-body zeroing (sgs.f90:898-925)
+// and, where the dynamic model has just formed its coefficient, the
+// multiplication with it (SCALE): 384x256x384 596 us and a pass of 178 us
+// -> 304.
+template <bool SCALE>
 struct ZeroTerm {
     double *f;
-    __device__ void operator()(const KP &p, int i, int j, int k, double *w) const {
-        long long q = p.g.ix(i, j, k);
-        w[0] = w[1] = 0.0;
-        if (p.f.fb_c[q] >= 1.0e-10) {
-            const double x = f[q];
-            w[0] = x * (p.g.f2fx[i] * p.g.f2fy[j] * p.g.f2fz[k]);
-            w[1] = max_bits(x, 0.0);
-        } else {
-            f[q] = 0.0;
-        }
+    int thermal;
+    static constexpr int kLoads = 2;
+    __device__ void load(const KP &p, int i, int j, int k, double *x) const {
+        const long long q = p.g.ix(i, j, k);
+        x[0] = f[q];
+        x[1] = p.f.fb_c[q];
+    }
+    __device__ void add(const KP &p, int i, int j, int k, const double *x, double *v) const {
+        const bool in = fluid(x[1]);
+        const double y = !in ? 0.0 : SCALE ? (thermal ? p.S->csgshf : p.S->csgsts) * x[0] : x[0];
+        if (SCALE || !in) f[p.g.ix(i, j, k)] = y;
+        v[0] = fma(y, p.g.f2fx[i] * p.g.f2fy[j] * p.g.f2fz[k], v[0]);
+        take_max(v[1], y);
     }
 };
 struct ZeroFinal {
     int thermal;
     __device__ void operator()(const KP &p, const double *o) const {
-        const double avg = o[0] / p.S->fluidvol;
-        if (thermal) { p.S->alpavg = avg * p.c.re * p.c.pr; p.S->alpmax = o[1] * p.c.re * p.c.pr; }
-        else { p.S->nutavg = avg * p.c.re; p.S->nutmax = o[1] * p.c.re; }
+        const double avg = o[0] / p.S->fluidvol, mx = o[1] > 0.0 ? o[1] : 0.0;
+        if (thermal) { p.S->alpavg = avg * p.c.re * p.c.pr; p.S->alpmax = mx * p.c.re * p.c.pr; }
+        else { p.S->nutavg = avg * p.c.re; p.S->nutmax = mx * p.c.re; }
     }
 };
 
@@ -526,11 +523,12 @@ static void edge_interpol(lesgpu_case *c, double *f, double **f1, int full) {
     k_edge_bc<<<blocks_for(nz), kThreads, 0, c->stream>>>(c->kp, 2, f, f1[0], f1[1], f1[2], ib, g.n1m, jb, g.n2m, full);
 }
 
-static void zero_in_body(lesgpu_case *c, double *f, int thermal) {
+static void zero_in_body(lesgpu_case *c, double *f, int thermal, bool scale) {
     const DGrid &g = c->kp.g;
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     if (c->kp.c.nzero > 0) k_zero_list<<<blocks_for(c->kp.c.nzero), kThreads, 0, c->stream>>>(c->kp, f);
-    reduce<2, 2u>(c, b, ZeroTerm{f}, ZeroFinal{thermal});
+    if (scale) reduce<2, 2u>(c, b, ZeroTerm<true>{f, thermal}, ZeroFinal{thermal});
+    else reduce<2, 2u>(c, b, ZeroTerm<false>{f, thermal}, ZeroFinal{thermal});
 }
 
 void launch_sgs_zero_first(lesgpu_case *c, int thermal) {
@@ -559,15 +557,14 @@ void launch_sgs(lesgpu_case *c) {
         filter_batch(c, G);
         if (mixed(c)) reduce<2, 0u>(c, b, LmMmTerm<float>{}, CsgstsFinal{});
         else reduce<2, 0u>(c, b, LmMmTerm<double>{}, CsgstsFinal{});
-        k_scale<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, f.nusgs, 0);
     } else {
         if (mixed(c)) k_vreman1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
         else k_vreman1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
     }
 }
 
-void launch_sgs_post(lesgpu_case *c) {
-    zero_in_body(c, c->kp.f.nusgs, 0);
+void launch_sgs_post(lesgpu_case *c, bool scale) {
+    zero_in_body(c, c->kp.f.nusgs, 0, scale);
     edge_interpol(c, c->kp.f.nusgs, c->kp.f.nusgs1, 0);
 }
 
@@ -740,15 +737,14 @@ void launch_sgs_t(lesgpu_case *c) {
         filter_batch(c, G);
         if (mixed(c)) reduce<2, 0u>(c, b, LmMmTTerm<float>{}, CsgshfFinal{});
         else reduce<2, 0u>(c, b, LmMmTTerm<double>{}, CsgshfFinal{});
-        k_scale<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, f.alsgs, 1);
     } else {
         if (mixed(c)) k_edm1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
         else k_edm1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
     }
 }
 
-void launch_sgs_t_post(lesgpu_case *c) {
-    zero_in_body(c, c->kp.f.alsgs, 1);
+void launch_sgs_t_post(lesgpu_case *c, bool scale) {
+    zero_in_body(c, c->kp.f.alsgs, 1, scale);
     edge_interpol(c, c->kp.f.alsgs, c->kp.f.alsgs1, 1);
 }
 

@@ -19,8 +19,9 @@
 using namespace lg;
 
 namespace lg {
-void launch_sgs_post(lesgpu_case *c);
-void launch_sgs_t_post(lesgpu_case *c);
+// scale: first multiply by the dynamic coefficient launch_sgs(_t) has formed
+void launch_sgs_post(lesgpu_case *c, bool scale);
+void launch_sgs_t_post(lesgpu_case *c, bool scale);
 }
 
 // ------------------------------------------------------------------ helpers
@@ -472,18 +473,21 @@ extern "C" int lesgpu_create(const lesgpu_config *cfg, const lesgpu_grid *g, les
             long long n;
             const double2 **face[2];                         // ghost, wrapped
             const double4 **der[2], **width;
-            const double **quarter, **d, **e;
+            const double **quarter, **half, **d, **e;
+            double **proj;
         };
         Stn &st = c->kp.st;
         const Axis axes[3] = {
-            {g->f2fx, g->f2fxi, g->c2cxi, g->ipv, g->imv, g->fixil, g->fixiu, d.n1, {&st.gx, &st.wx}, {&st.dgx, &st.dwx}, &st.lx, &st.qx, &m.dx, &m.ex},
-            {g->f2fy, g->f2fyi, g->c2cyi, g->jpv, g->jmv, g->fixjl, g->fixju, d.n2, {&st.gy, &st.wy}, {&st.dgy, &st.dwy}, &st.ly, &st.qy, &m.dy, &m.ey},
-            {g->f2fz, g->f2fzi, g->c2czi, g->kpv, g->kmv, g->fixkl, g->fixku, d.n3, {&st.gz, &st.wz}, {&st.dgz, &st.dwz}, &st.lz, &st.qz, &m.dz, &m.ez}};
+            {g->f2fx, g->f2fxi, g->c2cxi, g->ipv, g->imv, g->fixil, g->fixiu, d.n1, {&st.gx, &st.wx}, {&st.dgx, &st.dwx}, &st.lx, &st.qx, &st.hx, &m.dx, &m.ex, &st.px},
+            {g->f2fy, g->f2fyi, g->c2cyi, g->jpv, g->jmv, g->fixjl, g->fixju, d.n2, {&st.gy, &st.wy}, {&st.dgy, &st.dwy}, &st.ly, &st.qy, &st.hy, &m.dy, &m.ey, &st.py},
+            {g->f2fz, g->f2fzi, g->c2czi, g->kpv, g->kmv, g->fixkl, g->fixku, d.n3, {&st.gz, &st.wz}, {&st.dgz, &st.dwz}, &st.lz, &st.qz, &st.hz, &m.dz, &m.ez, &st.pz}};
         for (const Axis &x : axes) {
             const long long n = x.n, nm = n - 1;
-            std::vector<double> quarter(n + 1), dv(n + 1, 0.0), ev(n + 1, 0.0);
+            std::vector<double> quarter(n + 1), half(n + 1), dv(n + 1, 0.0), ev(n + 1, 0.0);
             std::vector<double4> width(n + 1, make_double4(0, 0, 0, 0));
-            for (long long i = 0; i <= n; i++) quarter[i] = 0.25 * x.ci[i];
+            for (long long i = 0; i <= n; i++) { quarter[i] = 0.25 * x.ci[i]; half[i] = 0.5 * x.fi[i]; }
+            *x.half = upload(A, half.data(), half.size());
+            *x.proj = A.get<double>(n + 1);
             for (long long i = 1; i <= nm; i++) {
                 const double t = 0.5 * x.f[i - 1] * (1.0 - (double)x.fu[i - 1]) + x.f[i] + 0.5 * x.f[i + 1] * (1.0 - (double)x.fl[i - 1]);
                 dv[i] = cbrt(x.f[i] * x.f[i]);
@@ -773,13 +777,14 @@ static void enqueue_sgs(lesgpu_case *c, bool first) {
     launch_mirror(c, kMirVel | kMirT);
     if (first) launch_sgs_zero_first(c, 0);
     else launch_sgs(c);
-    launch_sgs_post(c);
+    const bool scale = !first && g.idvmon == 1;
+    launch_sgs_post(c, scale);
     mark_mirror(c, kMirNu);
     launch_mirror(c, kMirNu);
     if (g.ihtrans == 1) {
         if (first) launch_sgs_zero_first(c, 1);
         else launch_sgs_t(c);
-        launch_sgs_t_post(c);
+        launch_sgs_t_post(c, scale);
         mark_mirror(c, kMirAl);
         launch_mirror(c, kMirAl);
     }

@@ -10,6 +10,7 @@
 // c2cx[0..n1]); index vectors are int32 on the device.
 #pragma once
 
+#include <type_traits>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stddef.h>
@@ -155,6 +156,7 @@ struct DPois {
     int Lz, Lx;               // FFT lines per block (0 = the shared-memory rule; set by the autotuner)
     int mixed_fft;            // poiss_ftft in the mixed form: FP32 transforms, FP64 defect correction
     double *yres;             // its FP64 residual's y rows and diagonal, 3 per j
+    double sx2, sz2;          // and its x and z coefficients
 };
 
 // The arrays a kernel of arithmetic type T reads in its stencils.  Mir<double>
@@ -183,11 +185,13 @@ struct Mir {
 //           the wall flags folded in; neighbours by ghost layer / wrapped
 //  dg? dw?  half the derivative over cell i of that value: x lower + y own + z upper
 //  l?       cell width, test-filter width, and the cube roots of their squares
-//  q?       c2ci / 4
+//  q? h? p? products with one factor, below
 struct Stn {
     const double2 *gx, *gy, *gz, *wx, *wy, *wz;
     const double4 *dgx, *dgy, *dgz, *dwx, *dwy, *dwz, *lx, *ly, *lz;
-    const double *qx, *qy, *qz;
+    const double *qx, *qy, *qz;       // c2ci / 4
+    const double *hx, *hy, *hz;       // f2fi / 2
+    double *px, *py, *pz;             // dtconst c2ci, written with each substep's coefficients
 };
 
 struct KP {                   // everything a kernel may read, passed by value
@@ -320,6 +324,17 @@ __device__ __forceinline__ double max_bits(double a, double b) {
     const long long ka = ia ^ ((ia >> 63) & kAbs), kb = ib ^ ((ib >> 63) & kAbs);
     const bool na = (ia & kAbs) > kInf, nb = (ib & kAbs) > kInf;
     return (nb || (!na && ka >= kb)) ? a : b;
+}
+
+// |x| by its bits (a compiled fabs may be an FP64 addition), and a running
+// maximum m of values that count when they are >= 0 and no NaN (m starts
+// below zero)
+__device__ __forceinline__ double abs_bits(double x) {
+    return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
+}
+__device__ __forceinline__ void take_max(double &m, double x) {
+    const long long b = __double_as_longlong(x);
+    if (b <= 0x7ff0000000000000LL && b > __double_as_longlong(m)) m = x;
 }
 
 // Deterministic block totals of NV doubles (the sum, or the maximum for the
@@ -459,9 +474,21 @@ namespace lg {
 // finish (counted with an atomic ticket after a release fence) sums all the
 // partials in block order -- the same fixed order as a separate finalize
 // kernel, so results are deterministic -- applies g and resets the ticket.
+// A term kernel either forms its NV terms, which are then added (operator()),
+// or has kLoads: load() fetches operands and nothing else (a store would hold back
+// the next cells' loads), add() accumulates them with fused multiply-adds --
+// one FP64 operation where a product and a sum take two -- and stores.
+template <class F, class = void> struct has_loads { static constexpr int n = 0; };
+template <class F> struct has_loads<F, std::void_t<decltype(F::kLoads)>> { static constexpr int n = F::kLoads; };
+
+// fb >= 1e-10 (the body functions' fluid test) on the bit pattern: an FP64
+// comparison issues on the FP64 pipe
+__device__ __forceinline__ bool fluid(double fb) { return __double_as_longlong(fb) >= __double_as_longlong(1.0e-10); }
+
 template <int NV, unsigned MAXM, class F, class G>
 __global__ void __launch_bounds__(kThreads, 4) k_reduce_fin(KP p, Box b, F f, G g) {
     static_assert(NV <= kThreads / 32 && NV <= kMaxRed, "one warp per value");
+    static_assert(MAXM == 0u || has_loads<F>::n > 0, "formed terms are summed");
     __shared__ int last;
     double v[NV];
 #pragma unroll
@@ -474,8 +501,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_reduce_fin(KP p, Box b, F f, G 
     auto add_terms = [&](const double (&w)[NV]) {
 #pragma unroll
         for (int q = 0; q < NV; q++) {
-            if ((MAXM >> q) & 1u) v[q] = max_bits(v[q], w[q]);
-            else if (__double_as_longlong(w[q]) != 0LL) v[q] = v[q] + w[q];
+            if (__double_as_longlong(w[q]) != 0LL) v[q] = v[q] + w[q];
         }
     };
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -483,24 +509,46 @@ __global__ void __launch_bounds__(kThreads, 4) k_reduce_fin(KP p, Box b, F f, G 
     // blocks of 256 threads an SM leave 64 registers a thread): their terms
     // are all formed (loads in flight together) before they are added, in
     // the sequence's order -- the sums of the one-at-a-time loop, bit for bit
-    constexpr int U = NV >= 6 ? 2 : 4;
-    for (; t + (U - 1) * S < n; t += U * S) {
-        double w[U][NV];
+    constexpr int U = NV >= 6 || has_loads<F>::n >= 6 ? 2 : 4;
+    if constexpr (has_loads<F>::n > 0) {
+        constexpr int NL = has_loads<F>::n;
+        for (; t + (U - 1) * S < n; t += U * S) {
+            double x[U][NL];
+            int i[U], j[U], k[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            int i, j, k;
-            b.at(t + u * S, i, j, k);
-            f(p, i, j, k, w[u]);
+            for (int u = 0; u < U; u++) {
+                b.at(t + u * S, i[u], j[u], k[u]);
+                f.load(p, i[u], j[u], k[u], x[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) f.add(p, i[u], j[u], k[u], x[u], v);
         }
+        for (; t < n; t += S) {
+            int i, j, k;
+            b.at(t, i, j, k);
+            double x[NL];
+            f.load(p, i, j, k, x);
+            f.add(p, i, j, k, x, v);
+        }
+    } else {
+        for (; t + (U - 1) * S < n; t += U * S) {
+            double w[U][NV];
 #pragma unroll
-        for (int u = 0; u < U; u++) add_terms(w[u]);
-    }
-    for (; t < n; t += S) {
-        int i, j, k;
-        b.at(t, i, j, k);
-        double w[NV];
-        f(p, i, j, k, w);
-        add_terms(w);
+            for (int u = 0; u < U; u++) {
+                int i, j, k;
+                b.at(t + u * S, i, j, k);
+                f(p, i, j, k, w[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) add_terms(w[u]);
+        }
+        for (; t < n; t += S) {
+            int i, j, k;
+            b.at(t, i, j, k);
+            double w[NV];
+            f(p, i, j, k, w);
+            add_terms(w);
+        }
     }
     block_totals<NV, MAXM>(v);
     if (threadIdx.x == 0) {
