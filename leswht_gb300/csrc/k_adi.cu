@@ -172,6 +172,7 @@ struct AdiBatch {
 
 template <class R, int DIR, bool PER, bool FAC>
 __global__ void __launch_bounds__(128, 6) k_adi(KP p, AdiBatch B) {
+    chained();
     const AdiArgs &A = B.a[blockIdx.y];
     const DGrid &g = p.g;
     const R diag = (A.comp == CT) ? p.S->acoefi * p.c.pr : p.S->acoefi;
@@ -364,8 +365,8 @@ __global__ void __launch_bounds__(128, 6) k_adi(KP p, AdiBatch B) {
 
 template <class R, int DIR>
 static void k_adi_launch_dir(bool per, bool fac, dim3 grid, int tpb, cudaStream_t st, const KP &kp, const AdiBatch &B) {
-    if (per) { if (fac) k_adi<R, DIR, true, true><<<grid, tpb, 0, st>>>(kp, B); else k_adi<R, DIR, true, false><<<grid, tpb, 0, st>>>(kp, B); }
-    else { if (fac) k_adi<R, DIR, false, true><<<grid, tpb, 0, st>>>(kp, B); else k_adi<R, DIR, false, false><<<grid, tpb, 0, st>>>(kp, B); }
+    if (per) { if (fac) chain(k_adi<R, DIR, true, true>, grid, tpb, 0, st)(kp, B); else chain(k_adi<R, DIR, true, false>, grid, tpb, 0, st)(kp, B); }
+    else { if (fac) chain(k_adi<R, DIR, false, true>, grid, tpb, 0, st)(kp, B); else chain(k_adi<R, DIR, false, false>, grid, tpb, 0, st)(kp, B); }
 }
 
 template <class R>
@@ -467,6 +468,7 @@ __device__ __forceinline__ R scan_affine_down(R C, R D, int lane) {
 // two is faster depends on the shape, and the autotuner times both.
 template <class R, int MC, int W, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_adis(KP p, AdiBatch B) {
+    chained();
     const AdiArgs &A = B.a[blockIdx.y];
     const DGrid &g = p.g;
     const R diag = (A.comp == CT) ? p.S->acoefi * p.c.pr : p.S->acoefi;
@@ -724,6 +726,7 @@ __device__ __forceinline__ int tpos(int r, int m, int pm) { return (r / m) * pm 
 
 template <class R, int DIR, bool PER, int MC>
 __global__ void __launch_bounds__(kTileLines * 32, 2) k_adit(KP p, AdiBatch B, int m, int pm, int lp) {
+    chained();
     extern __shared__ __align__(16) unsigned char adit_smem[];
     R *S = reinterpret_cast<R *>(adit_smem);             // lines x lp: diag*rhs -> y -> x
     R *Ca = S + kTileLines * lp;                          // lines x lp: a of rows 0..n-1
@@ -1104,7 +1107,7 @@ static void adit_launch3(dim3 grid, const TileShape &ts, cudaStream_t st, const 
         cudaFuncSetAttribute(k_adit<float, DIR, PER, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax);
         attr = true;
     }
-    k_adit<float, DIR, PER, MC><<<grid, kTileLines * 32, ts.smem, st>>>(kp, B, ts.m, ts.pm, ts.lp);
+    chain(k_adit<float, DIR, PER, MC>, grid, kTileLines * 32, ts.smem, st)(kp, B, ts.m, ts.pm, ts.lp);
 }
 
 template <int DIR, bool PER>
@@ -1181,6 +1184,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.commit_
 
 template <int DIR, bool PER>
 __global__ void __launch_bounds__(32) k_adie(KP p, AdiBatch B) {
+    chained();
     extern __shared__ double4 ends_sm[];
     const AdiArgs &A = B.a[blockIdx.y];
     const DGrid &g = p.g;
@@ -1418,7 +1422,7 @@ static void ends_launch2(dim3 grid, size_t smem, cudaStream_t st, const KP &kp, 
     static const bool ok = cudaFuncSetAttribute(k_adie<DIR, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 (int)kEndsSmemMax) == cudaSuccess;
     (void)ok;
-    k_adie<DIR, PER><<<grid, 32, smem, st>>>(kp, B);
+    chain(k_adie<DIR, PER>, grid, 32, smem, st)(kp, B);
 }
 
 // The two-ended FP64 sweep of a batch (factored coefficients); false when it
@@ -1444,14 +1448,14 @@ static bool adis_launch(lesgpu_case *c, const AdiBatch &B, int ncomp, long long 
     const long long lpb = 128 / W;
     dim3 grid((unsigned)((mx + lpb - 1) / lpb), (unsigned)ncomp);
     // up to 4 rows per lane the kernel fits the cap anyway
-    if (m <= 2) k_adis<R, 2, W, 1><<<grid, 128, 0, c->stream>>>(c->kp, B);
-    else if (m <= 4) k_adis<R, 4, W, 1><<<grid, 128, 0, c->stream>>>(c->kp, B);
+    if (m <= 2) chain(k_adis<R, 2, W, 1>, grid, 128, 0, c->stream)(c->kp, B);
+    else if (m <= 4) chain(k_adis<R, 4, W, 1>, grid, 128, 0, c->stream)(c->kp, B);
     else if (m <= 8) {
-        if (capped) k_adis<R, 8, W, 4><<<grid, 128, 0, c->stream>>>(c->kp, B);
-        else k_adis<R, 8, W, 1><<<grid, 128, 0, c->stream>>>(c->kp, B);
+        if (capped) chain(k_adis<R, 8, W, 4>, grid, 128, 0, c->stream)(c->kp, B);
+        else chain(k_adis<R, 8, W, 1>, grid, 128, 0, c->stream)(c->kp, B);
     } else if (m <= 12) {
-        if (capped) k_adis<R, 12, W, 4><<<grid, 128, 0, c->stream>>>(c->kp, B);
-        else k_adis<R, 12, W, 1><<<grid, 128, 0, c->stream>>>(c->kp, B);
+        if (capped) chain(k_adis<R, 12, W, 4>, grid, 128, 0, c->stream)(c->kp, B);
+        else chain(k_adis<R, 12, W, 1>, grid, 128, 0, c->stream)(c->kp, B);
     } else {
         return false;
     }

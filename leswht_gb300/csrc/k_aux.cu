@@ -73,6 +73,7 @@ __device__ void stepinit_pre(KP p) {
 }
 
 __global__ void k_zero_fcvavg(KP p) {
+    chained();
     for (int l = 0; l < 4; l++) {
         int n = p.c.nbody[l];
         for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
@@ -81,13 +82,14 @@ __global__ void k_zero_fcvavg(KP p) {
 }
 
 void launch_stepinit(lesgpu_case *c) {
-    if (c->kp.c.ibmon == 1) k_zero_fcvavg<<<64, kThreads, 0, c->stream>>>(c->kp);
+    if (c->kp.c.ibmon == 1) chain(k_zero_fcvavg, 64, kThreads, 0, c->stream)(c->kp);
     reduce<1, 1u>(c, interior(c->kp.g), CflTerm{}, StepinitFinal{});
 }
 
 // substepinit, slv_auxi.f90:105-123 (RK3 coefficients of rk3coefinit,
 // misc_init.f90:1031-1044)
 __global__ void k_substepinit(KP p, int s, int carry) {
+    chained();
     const double gam[4] = {0.0, 8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
     const double ro[4] = {0.0, 0.0, -17.0 / 60.0, -5.0 / 12.0};
     DScal *S = p.S;
@@ -111,7 +113,7 @@ __global__ void k_substepinit(KP p, int s, int carry) {
 }
 
 void launch_substepinit(lesgpu_case *c, int msub, bool carry) {
-    k_substepinit<<<1, kThreads, 0, c->stream>>>(c->kp, msub, carry ? 1 : 0);
+    chain(k_substepinit, 1, kThreads, 0, c->stream)(c->kp, msub, carry ? 1 : 0);
 }
 
 // ------------------------------------------------------------ qvol / tvol
@@ -149,6 +151,7 @@ void launch_tvolcalc(lesgpu_case *c, int slot) { reduce<1, 0u>(c, interior(c->kp
 // of qvolcalc / meanpg (fb_u), the bulk velocity (fb_c) and tvolcalc (1/c*),
 // formed once so each reduction does one multiply per cell.
 __global__ void k_red_weights(KP p, Box b) {
+    chained();
     const DGrid &g = p.g;
     const long long n = b.count();
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -181,7 +184,7 @@ struct VolumeFinal {
 };
 void launch_red_weights(lesgpu_case *c) {
     Box b = interior(c->kp.g);
-    k_red_weights<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+    chain(k_red_weights, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b);
     reduce<3, 0u>(c, b, VolumeTerm{}, VolumeFinal{});
 }
 
@@ -237,6 +240,7 @@ void launch_cvol(lesgpu_case *c) { reduce<1, 0u>(c, interior(c->kp.g), CvolTerm{
 
 // tcalc, slv_auxi.f90:496-516
 __global__ void k_tcalc(KP p, Box b) {
+    chained();
     long long n = b.count();
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
@@ -247,7 +251,7 @@ __global__ void k_tcalc(KP p, Box b) {
 void launch_tcalc(lesgpu_case *c) {
     if (c->kp.c.ich == 1 && c->kp.c.xprdic == 0) {
         Box b = interior(c->kp.g);
-        k_tcalc<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+        chain(k_tcalc, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b);
     }
 }
 
@@ -288,6 +292,7 @@ struct MeanpgWallTerm {
 
 // IB streamwise forcing term of meanpg (slv_mmtm.f90:141-146)
 __global__ void k_meanpg_ibm(KP p) {
+    chained();
     double v[1] = {0.0};
     int n = p.c.nbody[0];
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
@@ -330,7 +335,7 @@ struct MeanpgFinal {
 
 void launch_meanpg(lesgpu_case *c, bool have_q) {
     const DGrid &g = c->kp.g;
-    if (c->kp.c.nbody[0] > 0) k_meanpg_ibm<<<1, kThreads, 0, c->stream>>>(c->kp);
+    if (c->kp.c.nbody[0] > 0) chain(k_meanpg_ibm, 1, kThreads, 0, c->stream)(c->kp);
     if (!have_q && c->kp.c.ich == 1) reduce<1, 0u>(c, interior(g), QvolTerm{}, FlowFinal{});
     reduce<4, 0u>(c, Box{1, 0, 1, g.n1m, 4, g.n2m > g.n3m ? g.n2m : g.n3m}, MeanpgWallTerm{}, MeanpgFinal{});
 }
@@ -338,6 +343,7 @@ void launch_meanpg(lesgpu_case *c, bool have_q) {
 // ------------------------------------------------------------------- ucalc
 // ucalc, slv_auxi.f90:233-416 (interior update; ghosts by launch_ghost_*)
 __global__ void __launch_bounds__(kThreads) k_ucalc(KP p, Box b) {
+    chained();
     long long n = b.count();
     const DGrid &g = p.g;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -358,6 +364,7 @@ __global__ void __launch_bounds__(kThreads) k_ucalc(KP p, Box b) {
 //  dir 2: a(i,j,0) = a(i,j,n3m), a(i,j,n3) = a(i,j,1) over i, j
 
 __global__ void k_ghost(KP p, int dir, GhostSpec s0, GhostSpec s1, GhostSpec s2, GhostSpec s3, int na) {
+    chained();
     const DGrid &g = p.g;
     GhostSpec ss[4] = {s0, s1, s2, s3};
     for (int a = 0; a < na; a++) {
@@ -388,7 +395,7 @@ void ghost(lesgpu_case *c, int dir, GhostSpec *s, int na) {
         long long n = (long long)(s[q].hi0 - s[q].lo0 + 1) * (s[q].hi1 - s[q].lo1 + 1);
         if (n > mx) mx = n;
     }
-    k_ghost<<<blocks_for(mx), kThreads, 0, c->stream>>>(c->kp, dir, a0, a1, a2, a3, na);
+    chain(k_ghost, blocks_for(mx), kThreads, 0, c->stream)(c->kp, dir, a0, a1, a2, a3, na);
 }
 
 // qvolcalc(qvol(2)), ucalc and qvolcalc(qvol(0)) in one pass: per cell the
@@ -434,7 +441,7 @@ struct UcalcQvolFinal {
 static void ucalc_interior(lesgpu_case *c, bool with_qvol) {
     Box b = interior(c->kp.g);
     if (with_qvol) reduce<2, 0u>(c, b, UcalcQvolTerm{}, UcalcQvolFinal{});
-    else k_ucalc<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+    else chain(k_ucalc, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b);
 }
 
 // prdic_adj_uvw(0), slv_mmtm.f90:1746-1857: x, then y, then z
@@ -467,6 +474,7 @@ struct PhirefFinal {
 };
 
 __global__ void __launch_bounds__(kThreads) k_pcalc(KP p, Box b) {
+    chained();
     long long n = b.count();
     const DGrid &g = p.g;
     // three FP64 operations a cell, the factor formed once for a thread's cells
@@ -490,7 +498,7 @@ void launch_ucalc_pcalc(lesgpu_case *c, bool with_qvol) {
     reduce<1, 0u>(c, Box{1, 1, 1, 1, g.n2m, g.n3m}, PhirefTerm{}, PhirefFinal{});
     Box b = interior(g);
     const int nb = blocks_for(b.count());
-    k_pcalc<<<nb < 2 * kRedBlocks ? nb : 2 * kRedBlocks, kThreads, 0, c->stream>>>(c->kp, b);
+    chain(k_pcalc, nb < 2 * kRedBlocks ? nb : 2 * kRedBlocks, kThreads, 0, c->stream)(c->kp, b);
     DFields &f = c->kp.f;
     if (c->kp.c.zprdic == 1) {
         GhostSpec s[4] = {{f.u, 1, g.n1, 0, g.n2}, {f.v, 0, g.n1, 1, g.n2}, {f.w, 0, g.n1, 0, g.n2}, {f.p, 1, g.n1m, 1, g.n2m}};
@@ -583,7 +591,10 @@ struct BulkTFinal {
     int solid;
     __device__ void operator()(const KP &p, const double *o) const { bulk_scalars(p, p.S->qcur, o[0], solid); }
 };
-__global__ void k_bulk_scalars(KP p, int solid) { bulk_scalars(p, p.S->qcur, p.S->tbulk_sum, solid); }
+__global__ void k_bulk_scalars(KP p, int solid) {
+    chained();
+    bulk_scalars(p, p.S->qcur, p.S->tbulk_sum, solid);
+}
 struct BulkSolidFinal {
     __device__ void operator()(const KP &p, const double *o) const {
         p.S->tbulk_solid = o[0] > 0.0 ? o[1] / o[0] : 0.0;
@@ -592,7 +603,7 @@ struct BulkSolidFinal {
 void launch_bulk_diag(lesgpu_case *c, bool have_q, bool have_t) {
     const bool solid = c->kp.c.ihtrans == 1 && c->bulk_solid;
     const int sl = solid ? 1 : 0;
-    if (have_q && (have_t || c->kp.c.ihtrans != 1)) k_bulk_scalars<<<1, 1, 0, c->stream>>>(c->kp, sl);
+    if (have_q && (have_t || c->kp.c.ihtrans != 1)) chain(k_bulk_scalars, 1, 1, 0, c->stream)(c->kp, sl);
     else if (have_q) reduce<1, 0u>(c, interior(c->kp.g), BulkTTerm{}, BulkTFinal{sl});
     else reduce<2, 0u>(c, interior(c->kp.g), BulkTerm{}, BulkFinal{sl});
     if (solid) reduce<2, 0u>(c, interior(c->kp.g), BulkSolidTerm{}, BulkSolidFinal{});

@@ -30,6 +30,7 @@ struct UbulkFinal {
     }
 };
 __global__ void k_set_ubulk_one(KP p, int carry) {
+    chained();
     p.S->u_bulk_t = 1.0;
     p.S->hub = 0.5;
     if (carry) p.S->tvol[1] = p.S->tvol[0];
@@ -65,7 +66,7 @@ void launch_rhs_t(lesgpu_case *c, int msub, int tvol) {
         else reduce<1, 0u>(c, b, UbulkTerm{}, UbulkFinal{tvol == 2 ? 1 : 0});
     } else {
         if (tvol == 1) launch_tvolcalc(c, 1);
-        k_set_ubulk_one<<<1, 1, 0, c->stream>>>(c->kp, tvol == 2 ? 1 : 0);
+        chain(k_set_ubulk_one, 1, 1, 0, c->stream)(c->kp, tvol == 2 ? 1 : 0);
     }
     launch_rhs_t_kernel(c, msub);
 }
@@ -98,6 +99,7 @@ struct RecycFinal {
     }
 };
 __global__ void k_recyc_apply(KP p) {
+    chained();
     const DGrid &g = p.g;
     double tw = p.c.tsol_i, ratio = p.S->phiref;
     long long n = (long long)(g.n2 + 1) * (g.n3 + 1);
@@ -110,6 +112,7 @@ __global__ void k_recyc_apply(KP p) {
 
 // wallbc_t, one direction per launch (x, then y, then z)
 __global__ void k_wallbc_t(KP p, int dir) {
+    chained();
     const DGrid &g = p.g;
     const DCfg &c = p.c;
     double *t = p.f.t;
@@ -141,6 +144,7 @@ __global__ void k_wallbc_t(KP p, int dir) {
 }
 
 __global__ void k_retrv_t(KP p) {
+    chained();
     const DGrid &g = p.g;
     long long n = (long long)g.n2m * g.n3m;
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (long long)gridDim.x * blockDim.x) {
@@ -154,21 +158,21 @@ void launch_energy_bc(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     const DCfg &cf = c->kp.c;
     double *t = c->kp.f.t;
-    if (cf.xprdic == 0) k_retrv_t<<<blocks_for((long long)g.n2m * g.n3m), kThreads, 0, c->stream>>>(c->kp);
+    if (cf.xprdic == 0) chain(k_retrv_t, blocks_for((long long)g.n2m * g.n3m), kThreads, 0, c->stream)(c->kp);
     if (cf.xprdic == 1) {
         if (cf.idecomp == 1) {
             GhostSpec s[1] = {{t, 0, g.n2, 0, g.n3}};
             ghost(c, 0, s, 1);
         } else {
             reduce<2, 0u>(c, Box{1, 1, 1, 1, g.n2m, g.n3m}, RecycTerm{}, RecycFinal{});
-            k_recyc_apply<<<blocks_for((long long)(g.n2 + 1) * (g.n3 + 1)), kThreads, 0, c->stream>>>(c->kp);
+            chain(k_recyc_apply, blocks_for((long long)(g.n2 + 1) * (g.n3 + 1)), kThreads, 0, c->stream)(c->kp);
         }
     }
     if (cf.yprdic == 1) { GhostSpec s[1] = {{t, 0, g.n1, 0, g.n3}}; ghost(c, 1, s, 1); }
     if (cf.zprdic == 1) { GhostSpec s[1] = {{t, 0, g.n1, 0, g.n2}}; ghost(c, 2, s, 1); }
-    if (cf.xprdic == 0) k_wallbc_t<<<blocks_for((long long)(g.n2 + 1) * (g.n3 + 1)), kThreads, 0, c->stream>>>(c->kp, 0);
-    if (cf.yprdic == 0) k_wallbc_t<<<blocks_for((long long)(g.n1 + 1) * (g.n3 + 1)), kThreads, 0, c->stream>>>(c->kp, 1);
-    if (cf.zprdic == 0) k_wallbc_t<<<blocks_for((long long)(g.n1 + 1) * (g.n2 + 1)), kThreads, 0, c->stream>>>(c->kp, 2);
+    if (cf.xprdic == 0) chain(k_wallbc_t, blocks_for((long long)(g.n2 + 1) * (g.n3 + 1)), kThreads, 0, c->stream)(c->kp, 0);
+    if (cf.yprdic == 0) chain(k_wallbc_t, blocks_for((long long)(g.n1 + 1) * (g.n3 + 1)), kThreads, 0, c->stream)(c->kp, 1);
+    if (cf.zprdic == 0) chain(k_wallbc_t, blocks_for((long long)(g.n1 + 1) * (g.n2 + 1)), kThreads, 0, c->stream)(c->kp, 2);
 }
 
 }  // namespace lg

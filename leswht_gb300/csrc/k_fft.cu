@@ -170,6 +170,7 @@ DevPlan devplan(const FftPlan &p) {
 // memory, bounds these passes).  Line pair l holds i = i0 + 2l and i0 + 2l + 1.
 template <class V>
 __global__ void k_fft_z_fwd(KP p, const double *src, V *ccap, DevPlan P, int L, long long sk, long long sj) {
+    chained();
     using T = decltype(V{}.x);
     extern __shared__ __align__(16) unsigned char smraw[];
     V *sm = reinterpret_cast<V *>(smraw);
@@ -203,6 +204,7 @@ __global__ void k_fft_z_fwd(KP p, const double *src, V *ccap, DevPlan P, int L, 
 // ADD: phi += the result (the correction pass of the mixed form), else phi =
 template <class V, bool ADD>
 __global__ void k_fft_z_inv(KP p, const V *ccap, DevPlan P, int L, long long sk, long long sj) {
+    chained();
     using T = decltype(V{}.x);
     extern __shared__ __align__(16) unsigned char smraw[];
     V *sm = reinterpret_cast<V *>(smraw);
@@ -248,6 +250,7 @@ __global__ void k_fft_z_inv(KP p, const V *ccap, DevPlan P, int L, long long sk,
 // ---- x transforms of the (k,j) lines of ccap, in place -------------------
 template <class V>
 __global__ void k_fft_x(V *ccap, int nlines, DevPlan P, int L, int inv) {
+    chained();
     using T = decltype(V{}.x);
     extern __shared__ __align__(16) unsigned char smraw[];
     V *sm = reinterpret_cast<V *>(smraw);
@@ -279,6 +282,7 @@ __global__ void k_fft_x(V *ccap, int nlines, DevPlan P, int L, int inv) {
 // per mode, (k-1) + n3m*(j-1) + n3m*n2m*(iv-1).  Block = (k-tile of L lines)
 // x j: lines are read along x (contiguous) and written along k.
 __global__ void k_fft_xr_fwd(KP p, double2 *ccap, DevPlan P, int L) {
+    chained();
     extern __shared__ double2 sm[];
     const DGrid &g = p.g;
     const int N = P.n;
@@ -307,6 +311,7 @@ __global__ void k_fft_xr_fwd(KP p, double2 *ccap, DevPlan P, int L) {
 // what it stores: the sum is formed in one fixed order, so every block gets
 // the same phiref and the reference's extra pass over phi is not needed.
 __global__ void k_fft_xr_inv(KP p, const double2 *ccap, DevPlan P, int L, int pin) {
+    chained();
     extern __shared__ double2 sm[];
     __shared__ double s_ref;
     const DGrid &g = p.g;
@@ -378,6 +383,7 @@ __device__ __forceinline__ void ycoef(const DGrid &g, const double *ak1, const d
 // 128x125x120: 194 us one-ended, 55 this way.
 __global__ void __launch_bounds__(64) k_ytri_elim(int n1m, int n2m, int n3mh, double2 *ccap, const double *ak1, const double *ak3,
                                                   const double4 *rows, double *gam) {
+    chained();
     const long long nl = (long long)n1m * n3mh, sj = nl;
     const int lane = threadIdx.x & 31, up = lane >> 4;      // up: the half that comes down from row n2m
     const long long ngrp = (nl + 15) / 16;
@@ -514,6 +520,7 @@ __global__ void k_ytri_lu(KP p, const double *ak1, const double *ak3, double *yb
 template <class S>
 __global__ void __launch_bounds__(64) k_ytri(KP p, S *ccap, const S *ybet, const S *ygam,
                                              const S *yam, const S *pinref) {
+    chained();
     const DGrid &g = p.g;
     const int n1m = g.n1m, n2m = g.n2m, n3mh = g.n3mh;
     const long long nl = (long long)n1m * n3mh;
@@ -616,6 +623,7 @@ template <> YtriTabs<float> ytri_tabs<float>(const DPois &P) { return {P.ybetf, 
 // yc[3 j .. 3 j + 2] = (ajm, ajp, 2 sdx^2 + 2 sdz^2 + ajm + ajp) of row j, so a
 // cell costs a handful of FP64 operations (the FP64 pipe bounds this pass)
 __global__ void __launch_bounds__(kThreads) k_pois_resid(KP p, Box b, const double *yc, double *res, double sx2, double sz2) {
+    chained();
     const DGrid &g = p.g;
     const long long n = b.count();
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -731,8 +739,8 @@ int fft_autotune(lesgpu_case *c) {
     if (pois == LESGPU_POISSON_X_FT) {     // forward x transforms of the real lines
         const DevPlan px = devplan(P.fx);
         P.Lx = fft_time_pick(c, {2, g.n1m, g.n2m, g.n3m}, g.n1m, lines_per_block(g.n1m), [&](int L) {
-            k_fft_xr_fwd<<<dim3((g.n3m + L - 1) / L, g.n2m), kThreads, (size_t)2 * g.n1m * L * sizeof(double2),
-                           c->stream>>>(c->kp, P.ccap, px, L);
+            chain(k_fft_xr_fwd, dim3((g.n3m + L - 1) / L, g.n2m), kThreads, (size_t)2 * g.n1m * L * sizeof(double2),
+                           c->stream)(c->kp, P.ccap, px, L);
         });
         return cudaStreamSynchronize(c->stream) == cudaSuccess ? 0 : LESGPU_ERR_CUDA;
     }
@@ -743,13 +751,13 @@ int fft_autotune(lesgpu_case *c) {
     const long long sj = ftft ? (long long)g.n1m * g.n3mh : g.n1m;
     P.Lz = fft_time_pick(c, {0, g.n1m, g.n2m, g.n3m}, g.n3m, lines_per_block(g.n3m), [&](int L) {
         const dim3 gz((g.n1m + 2 * L - 1) / (2 * L), g.n2m);   // 2L real lines per block
-        k_fft_z_fwd<double2><<<gz, kThreads, (size_t)2 * g.n3m * L * sizeof(double2), c->stream>>>(c->kp, c->kp.f.divgsum, P.ccap, pz, L, sk, sj);
+        chain(k_fft_z_fwd<double2>, gz, kThreads, (size_t)2 * g.n3m * L * sizeof(double2), c->stream)(c->kp, c->kp.f.divgsum, P.ccap, pz, L, sk, sj);
     });
     if (ftft) {
         const DevPlan px = devplan(P.fx);
         const int nxl = g.n3mh * g.n2m;
         P.Lx = fft_time_pick(c, {1, g.n1m, g.n2m, g.n3m}, g.n1m, lines_per_block(g.n1m), [&](int L) {
-            k_fft_x<double2><<<(nxl + L - 1) / L, kThreads, (size_t)2 * g.n1m * L * sizeof(double2), c->stream>>>(P.ccap, nxl, px, L, 0);
+            chain(k_fft_x<double2>, (nxl + L - 1) / L, kThreads, (size_t)2 * g.n1m * L * sizeof(double2), c->stream)(P.ccap, nxl, px, L, 0);
         });
         // the mixed form: one FP64 solve, or two FP32 solves under an FP64
         // defect correction -- whichever is faster for the shape
@@ -897,13 +905,13 @@ static void ftft_solve(lesgpu_case *c, const double *src) {
     const long long sk = g.n1m, sj = (long long)g.n1m * g.n3mh;
     V *spec = reinterpret_cast<V *>(P.ccap);
     using T = decltype(V{}.x);
-    k_fft_z_fwd<V><<<gz, kThreads, smz, c->stream>>>(c->kp, src, spec, pz, Lz, sk, sj);
-    k_fft_x<V><<<(nxl + Lx - 1) / Lx, kThreads, smx, c->stream>>>(spec, nxl, px, Lx, 0);
+    chain(k_fft_z_fwd<V>, gz, kThreads, smz, c->stream)(c->kp, src, spec, pz, Lz, sk, sj);
+    chain(k_fft_x<V>, (nxl + Lx - 1) / Lx, kThreads, smx, c->stream)(spec, nxl, px, Lx, 0);
     const long long nl = (long long)g.n1m * g.n3mh;
     const YtriTabs<T> yt = ytri_tabs<T>(P);
-    k_ytri<T><<<blocks_for(2 * nl, 64), 64, 0, c->stream>>>(c->kp, reinterpret_cast<T *>(spec), yt.bet, yt.gam, yt.am, yt.pin);
-    k_fft_x<V><<<(nxl + Lx - 1) / Lx, kThreads, smx, c->stream>>>(spec, nxl, px, Lx, 1);
-    k_fft_z_inv<V, ADD><<<gz, kThreads, smz, c->stream>>>(c->kp, spec, pz, Lz, sk, sj);
+    chain(k_ytri<T>, blocks_for(2 * nl, 64), 64, 0, c->stream)(c->kp, reinterpret_cast<T *>(spec), yt.bet, yt.gam, yt.am, yt.pin);
+    chain(k_fft_x<V>, (nxl + Lx - 1) / Lx, kThreads, smx, c->stream)(spec, nxl, px, Lx, 1);
+    chain(k_fft_z_inv<V, ADD>, gz, kThreads, smz, c->stream)(c->kp, spec, pz, Lz, sk, sj);
 }
 
 void launch_poisson(lesgpu_case *c, int msub) {
@@ -921,7 +929,7 @@ void launch_poisson(lesgpu_case *c, int msub) {
         ftft_solve<float2, false>(c, c->kp.f.divgsum);
         const DGrid &g = c->kp.g;
         Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
-        k_pois_resid<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, P.yres, res, P.sx2, P.sz2);
+        chain(k_pois_resid, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, P.yres, res, P.sx2, P.sz2);
         ftft_solve<float2, true>(c, res);
     } else {
         ftft_solve<double2, false>(c, c->kp.f.divgsum);
@@ -932,14 +940,14 @@ void launch_poisson(lesgpu_case *c, int msub) {
 // FP64 launches for the other translation units
 void fft_z_fwd64(dim3 grid, size_t smem, cudaStream_t st, KP p, const double *src, double2 *ccap, DevPlan P, int L,
                  long long sk, long long sj) {
-    k_fft_z_fwd<double2><<<grid, kThreads, smem, st>>>(p, src, ccap, P, L, sk, sj);
+    chain(k_fft_z_fwd<double2>, grid, kThreads, smem, st)(p, src, ccap, P, L, sk, sj);
 }
 void fft_z_inv64(dim3 grid, size_t smem, cudaStream_t st, KP p, const double2 *ccap, DevPlan P, int L, long long sk,
                  long long sj) {
-    k_fft_z_inv<double2, false><<<grid, kThreads, smem, st>>>(p, ccap, P, L, sk, sj);
+    chain(k_fft_z_inv<double2, false>, grid, kThreads, smem, st)(p, ccap, P, L, sk, sj);
 }
 void fft_x64(int nblocks, size_t smem, cudaStream_t st, double2 *ccap, int nlines, DevPlan P, int L, int inv) {
-    k_fft_x<double2><<<nblocks, kThreads, smem, st>>>(ccap, nlines, P, L, inv);
+    chain(k_fft_x<double2>, nblocks, kThreads, smem, st)(ccap, nlines, P, L, inv);
 }
 int fft_smem64(int bytes) {
     return (cudaFuncSetAttribute(k_fft_z_fwd<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&

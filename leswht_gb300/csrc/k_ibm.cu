@@ -23,6 +23,7 @@ __device__ __forceinline__ void reindex(int n, int nm, int &ip, int &ipp) {
 
 // phase A: targets, fcv and dudtr of every forcing point of component l
 __global__ void k_ibm_target(KP p, int l, const double *fld, const double *rhs, double *targ) {
+    chained();
     const DGrid &g = p.g;
     const int nintp = p.c.nintp[l], nbody = p.c.nbody[l];
     const double dti = 1.0 / p.S->dt;
@@ -60,6 +61,7 @@ __global__ void k_ibm_target(KP p, int l, const double *fld, const double *rhs, 
 
 // phase B: rhs1 at the forcing points, running sum of the forcing
 __global__ void k_ibm_write(KP p, int l, const double *fld, double *rhs, const double *targ) {
+    chained();
     const DGrid &g = p.g;
     const int nbody = p.c.nbody[l];
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nbody; t += gridDim.x * blockDim.x) {
@@ -76,12 +78,12 @@ void launch_rhs_ibm(lesgpu_case *c) {
     for (int l = 0; l < 3; l++) {
         int nb = c->kp.c.nbody[l];
         if (nb <= 0) continue;
-        k_ibm_target<<<blocks_for(nb), kThreads, 0, c->stream>>>(c->kp, l, fld[l], f.rhs1[l], f.ibtarg[l]);
+        chain(k_ibm_target, blocks_for(nb), kThreads, 0, c->stream)(c->kp, l, fld[l], f.rhs1[l], f.ibtarg[l]);
     }
     for (int l = 0; l < 3; l++) {
         int nb = c->kp.c.nbody[l];
         if (nb <= 0) continue;
-        k_ibm_write<<<blocks_for(nb), kThreads, 0, c->stream>>>(c->kp, l, fld[l], f.rhs1[l], f.ibtarg[l]);
+        chain(k_ibm_write, blocks_for(nb), kThreads, 0, c->stream)(c->kp, l, fld[l], f.rhs1[l], f.ibtarg[l]);
     }
 }
 
@@ -89,14 +91,15 @@ void launch_rhs_ibm_t(lesgpu_case *c) {
     DFields &f = c->kp.f;
     int nb = c->kp.c.nbody[3];
     if (nb <= 0) return;
-    k_ibm_target<<<blocks_for(nb), kThreads, 0, c->stream>>>(c->kp, 3, f.t, f.rhs1[3], f.ibtarg[3]);
-    k_ibm_write<<<blocks_for(nb), kThreads, 0, c->stream>>>(c->kp, 3, f.t, f.rhs1[3], f.ibtarg[3]);
+    chain(k_ibm_target, blocks_for(nb), kThreads, 0, c->stream)(c->kp, 3, f.t, f.rhs1[3], f.ibtarg[3]);
+    chain(k_ibm_write, blocks_for(nb), kThreads, 0, c->stream)(c->kp, 3, f.t, f.rhs1[3], f.ibtarg[3]);
 }
 
 // divgs mass source/sink: one pass over one list; the six passes run in the
 // reference's order so every cell accumulates in the same sequence.  Within
 // one pass the touched cells are distinct.
 __global__ void k_divgs_ibm_pass(KP p, int l, int pass) {
+    chained();
     const DGrid &g = p.g;
     double *qm = p.f.qmass, *dv = p.f.divgsum;
     const double *vel = l == 0 ? p.f.u : l == 1 ? p.f.v : p.f.w;
@@ -125,7 +128,7 @@ void launch_divgs_ibm(lesgpu_case *c) {
         int nb = c->kp.c.nbody[l];
         if (nb <= 0) continue;
         for (int pass = 0; pass < 2; pass++)
-            k_divgs_ibm_pass<<<blocks_for(nb), kThreads, 0, c->stream>>>(c->kp, l, pass);
+            chain(k_divgs_ibm_pass, blocks_for(nb), kThreads, 0, c->stream)(c->kp, l, pass);
     }
 }
 

@@ -1175,6 +1175,7 @@ inline ZftBatchKernel zft_batch_kernel(int n2m) {
 // convergence criterion of the substep: test1 / nmodes * nfft * fac -- 0.8 in
 // poiss_z_ft.f90:179 (test1 itself in 2-D), 0.9 in poiss_x_ft.f90:158
 __global__ void k_mg_begin(DScal *S, int slot, int nfft, int nmodes, double fac) {
+    chained();
     S->poisson_iters[slot] = 0;
     S->mg_test = nfft == 1 ? S->test1 : S->test1 / (double)nmodes * (double)nfft * fac;
 }
@@ -1819,13 +1820,13 @@ static void mg2d_pre(lesgpu_case *c, int slot) {
     const DGrid &g = c->kp.g;
     DPois &P = c->pois;
     if (P.mg->xft) {
-        k_mg_begin<<<1, 1, 0, c->stream>>>(c->S, slot, g.n1m, g.n1mh, 0.9);
+        chain(k_mg_begin, 1, 1, 0, c->stream)(c->S, slot, g.n1m, g.n1mh, 0.9);
         const DevPlan px = devplan(P.fx);
         const int Lx = fft_lx(c);
-        k_fft_xr_fwd<<<dim3((g.n3m + Lx - 1) / Lx, g.n2m), kThreads, (size_t)2 * g.n1m * Lx * sizeof(double2),
-                       c->stream>>>(c->kp, P.ccap, px, Lx);
+        chain(k_fft_xr_fwd, dim3((g.n3m + Lx - 1) / Lx, g.n2m), kThreads, (size_t)2 * g.n1m * Lx * sizeof(double2),
+                       c->stream)(c->kp, P.ccap, px, Lx);
     } else {
-        k_mg_begin<<<1, 1, 0, c->stream>>>(c->S, slot, g.n3m, g.n3mh, 0.8);
+        chain(k_mg_begin, 1, 1, 0, c->stream)(c->S, slot, g.n3m, g.n3mh, 0.8);
         const DevPlan pz = devplan(P.fz);
         const int Lz = fft_lz(c);
         const size_t smz = (size_t)2 * (g.n3m > 1 ? g.n3m : 1) * Lz * sizeof(double2);
@@ -1842,8 +1843,8 @@ static void mg2d_post(lesgpu_case *c) {
         const DevPlan px = devplan(P.fx);
         const int Lx = fft_lx(c), pin = c->cfg.ich == 1 ? 1 : 0;
         const int Li = fft_xr_inv_lines(g.n1m, Lx, pin);
-        k_fft_xr_inv<<<dim3((g.n3m + Li - 1) / Li, g.n2m), kThreads, (size_t)2 * g.n1m * (Li + pin) * sizeof(double2),
-                       c->stream>>>(c->kp, P.ccap, px, Li, pin);
+        chain(k_fft_xr_inv, dim3((g.n3m + Li - 1) / Li, g.n2m), kThreads, (size_t)2 * g.n1m * (Li + pin) * sizeof(double2),
+                       c->stream)(c->kp, P.ccap, px, Li, pin);
     } else {
         const DevPlan pz = devplan(P.fz);
         const int Lz = fft_lz(c);
@@ -1914,6 +1915,7 @@ static std::mutex g_zft_mu;
 
 // A seeded noise right-hand side of every mode for the timing runs.
 __global__ void k_mgl_noise(double2 *ccap, long long n) {
+    chained();
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         unsigned long long z = ((unsigned long long)t + 1ULL) * 0x9E3779B97F4A7C15ULL;
         z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
@@ -1939,7 +1941,7 @@ static int mgl_autotune(lesgpu_case *c) {
         any = true;
         if (mgl_set_cluster(c, cs)) break;
         for (int r = 0; r < 3; r++) {           // the first is the warm-up
-            k_mgl_noise<<<blocks_for(n), kThreads, 0, c->stream>>>(c->pois.ccap, n);
+            chain(k_mgl_noise, blocks_for(n), kThreads, 0, c->stream)(c->pois.ccap, n);
             cudaEventRecord(e0, c->stream);
             mgl_launch(c, 3);
             cudaEventRecord(e1, c->stream);

@@ -85,6 +85,7 @@ struct OutletOutFinal {
 };
 
 __global__ void k_outlet_scale(KP p, int thermal) {
+    chained();
     const DGrid &g = p.g;
     const DFields &f = p.f;
     const double qr = p.S->cb[3];
@@ -107,6 +108,7 @@ __global__ void k_outlet_scale(KP p, int thermal) {
 
 // periodic copies of the outlet increments: dir 1 (y, all k), then dir 2 (z, all j)
 __global__ void k_outlet_ghost(KP p, int thermal, int dir) {
+    chained();
     const DGrid &g = p.g;
     const DFields &f = p.f;
     double *a[3] = {thermal ? f.dtout : f.duout, f.dvout, f.dwout};
@@ -126,6 +128,7 @@ __global__ void k_outlet_ghost(KP p, int thermal, int dir) {
 }
 
 __global__ void k_rhsincorpbc(KP p) {
+    chained();
     const DGrid &g = p.g;
     const DFields &f = p.f;
     const double acoef = p.S->acoef;
@@ -142,6 +145,7 @@ __global__ void k_rhsincorpbc(KP p) {
 }
 
 __global__ void k_rhsincorpbc_t(KP p) {
+    chained();
     const DGrid &g = p.g;
     const DFields &f = p.f;
     const DCfg &c = p.c;
@@ -171,16 +175,16 @@ static void outlet(lesgpu_case *c, int thermal) {
     reduce<2, 0u>(c, Box{0, 0, 0, (int)(nplane + (long long)g.n1m * g.n3m + (long long)g.n1m * g.n2m), 1, 1},
                      OutletQTerm{}, OutletQFinal{});
     reduce<1, 0u>(c, Box{0, 0, 0, (int)nplane, 1, 1}, OutletOutTerm{thermal}, OutletOutFinal{thermal});
-    k_outlet_scale<<<blocks_for(nplane), kThreads, 0, c->stream>>>(c->kp, thermal);
-    if (cf.yprdic == 1) k_outlet_ghost<<<blocks_for(g.n3 + 1), kThreads, 0, c->stream>>>(c->kp, thermal, 1);
-    if (cf.zprdic == 1) k_outlet_ghost<<<blocks_for(g.n2 + 1), kThreads, 0, c->stream>>>(c->kp, thermal, 2);
+    chain(k_outlet_scale, blocks_for(nplane), kThreads, 0, c->stream)(c->kp, thermal);
+    if (cf.yprdic == 1) chain(k_outlet_ghost, blocks_for(g.n3 + 1), kThreads, 0, c->stream)(c->kp, thermal, 1);
+    if (cf.zprdic == 1) chain(k_outlet_ghost, blocks_for(g.n2 + 1), kThreads, 0, c->stream)(c->kp, thermal, 2);
 }
 
 // convbc + rhsincorpbc (momentum), called between rhs(_ibm) and the ADI sweeps
 void launch_convbc(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     outlet(c, 0);
-    if (c->kp.c.ich != 1) k_rhsincorpbc<<<blocks_for((long long)g.n2m * g.n3m), kThreads, 0, c->stream>>>(c->kp);
+    if (c->kp.c.ich != 1) chain(k_rhsincorpbc, blocks_for((long long)g.n2m * g.n3m), kThreads, 0, c->stream)(c->kp);
 }
 
 // convbc_t + rhsincorpbc_t, only for flows not periodic in x
@@ -188,7 +192,7 @@ void launch_convbc_t(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     if (c->kp.c.xprdic != 0) return;
     outlet(c, 1);
-    if (c->kp.c.ich != 1) k_rhsincorpbc_t<<<blocks_for((long long)g.n2m * g.n3m), kThreads, 0, c->stream>>>(c->kp);
+    if (c->kp.c.ich != 1) chain(k_rhsincorpbc_t, blocks_for((long long)g.n2m * g.n3m), kThreads, 0, c->stream)(c->kp);
 }
 
 }  // namespace lg

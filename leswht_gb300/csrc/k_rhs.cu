@@ -14,6 +14,7 @@ namespace lg {
 // FP64 form is k_rhs64 (and k_rhs_t64).
 template <class R>
 __global__ void __launch_bounds__(kThreads, 3) k_rhs(KP p, Box b, R gam, R ro) {
+    chained();
     const Mir<R> &M = mir<R>(p);
     const DGrid &g = p.g;
     const DCfg &c = p.c;
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_rhs(KP p, Box b, R gam, R ro) {
 // 405, each 64 clocks a warp (k_grad64.cuh).  64^3: 175 us -> 100; 90x81x96:
 // 451 us -> 254.
 __global__ void __launch_bounds__(kThreads, 2) k_rhs64(KP p, Box b, double gam, double ro) {
+    chained();
     const DGrid &g = p.g;
     const DCfg &c = p.c;
     const Stn &T = p.st;
@@ -271,14 +273,15 @@ void launch_rhs(lesgpu_case *c, int msub) {
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     inst_begin(c, LESGPU_K_RHS);
     if (c->cfg.precision == LESGPU_PREC_MIXED)
-        k_rhs<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, (float)gam[msub], (float)ro[msub]);
+        chain(k_rhs<float>, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, (float)gam[msub], (float)ro[msub]);
     else
-        k_rhs64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, gam[msub], ro[msub]);
+        chain(k_rhs64, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, gam[msub], ro[msub]);
     inst_end(c, LESGPU_K_RHS);
 }
 
 // ------------------------------------------------------------------- divgs
 __global__ void __launch_bounds__(kThreads) k_divgs(KP p, Box b, int scale) {
+    chained();
     const DGrid &g = p.g;
     double dti = p.S->dtconsti;
     long long n = b.count();
@@ -295,6 +298,7 @@ __global__ void __launch_bounds__(kThreads) k_divgs(KP p, Box b, int scale) {
 }
 
 __global__ void k_scale_div(KP p, Box b) {
+    chained();
     double dti = p.S->dtconsti;
     long long n = b.count();
     for (long long tt = (long long)blockIdx.x * blockDim.x + threadIdx.x; tt < n; tt += (long long)gridDim.x * blockDim.x) {
@@ -309,11 +313,11 @@ void launch_divgs(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     bool ibm = c->kp.c.masson == 1 && c->kp.c.imovingon == 0 && c->kp.c.ibmon == 1;
-    k_divgs<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, ibm ? 0 : 1);
+    chain(k_divgs, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, ibm ? 0 : 1);
     if (ibm) {
         cudaMemsetAsync(c->kp.f.qmass, 0, sizeof(double) * g.nt, c->stream);
         launch_divgs_ibm(c);       // slv_cont.f90:48-113
-        k_scale_div<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+        chain(k_scale_div, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b);
     }
 }
 
@@ -325,6 +329,7 @@ struct UbulkTTerm;   // defined in k_energy via reduce; see launch_rhs_t there
 // and the terms reduce to the plain ones
 template <class R>
 __global__ void __launch_bounds__(kThreads) k_rhs_t(KP p, Box b, R gam, R ro, int conj) {
+    chained();
     const Mir<R> &M = mir<R>(p);
     const DGrid &g = p.g;
     const DCfg &c = p.c;
@@ -398,6 +403,7 @@ __global__ void __launch_bounds__(kThreads) k_rhs_t(KP p, Box b, R gam, R ro, in
 // the eddy diffusivity, the bulk velocity's reciprocal formed once: 55 FP64
 // operations a cell for 127.  64^3: 57 us -> 31.
 __global__ void __launch_bounds__(kThreads) k_rhs_t64(KP p, Box b, double gam, double ro, int conj) {
+    chained();
     const DGrid &g = p.g;
     const DCfg &c = p.c;
     const Stn &T = p.st;
@@ -467,9 +473,9 @@ void launch_rhs_t_kernel(lesgpu_case *c, int msub) {
     inst_begin(c, LESGPU_K_RHS_T);
     const int conj = c->kp.c.iconjg == 1 && c->conj_general;
     if (c->cfg.precision == LESGPU_PREC_MIXED)
-        k_rhs_t<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, (float)gam[msub], (float)ro[msub], conj);
+        chain(k_rhs_t<float>, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, (float)gam[msub], (float)ro[msub], conj);
     else
-        k_rhs_t64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, gam[msub], ro[msub], conj);
+        chain(k_rhs_t64, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, gam[msub], ro[msub], conj);
     inst_end(c, LESGPU_K_RHS_T);
 }
 

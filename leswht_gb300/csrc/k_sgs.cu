@@ -146,6 +146,7 @@ __device__ __forceinline__ R *scr(const KP &p, int s) { return reinterpret_cast<
 // pass 1 of sgs_dvmg (:434-491) and the constant model sgs_cvm
 template <class R>
 __global__ void __launch_bounds__(kThreads) k_vreman1(KP p, Box b, int dynamic) {
+    chained();
     const Mir<R> &M = mir<R>(p);
     const DGrid &g = p.g;
     GRID_LOOP(b) {      // mm[0..5] in scr[3..8], alp[0..8] in scr[9..17]
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(kThreads) k_vreman1(KP p, Box b, int dynamic) 
 
 // The FP64 form (k_grad64.cuh): 64^3 104 us -> 55.
 __global__ void __launch_bounds__(kThreads) k_vreman1_64(KP p, Box b, int dynamic) {
+    chained();
     const Stn &T = p.st;
     GRID_LOOP(b) {
         int i, j, k;
@@ -215,6 +217,7 @@ constexpr int kFiltA = 3;
 
 template <class R>
 __global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F, int run) {
+    chained();
     const DGrid &g = p.g;
     const bool xf = p.c.filter == 1 || p.c.filter == 3, zf = p.c.filter == 2 || p.c.filter == 3;
     const int a0 = blockIdx.y * kFiltA, na = F.na - a0 < kFiltA ? F.na - a0 : kFiltA;
@@ -286,8 +289,8 @@ static void filter_batch(lesgpu_case *c, FiltBatch &F) {
     Box b{1, 1, 1, g.n1m, g.n2m, (g.n3m + run - 1) / run};
     const dim3 grid((unsigned)blocks_for(b.count()), (unsigned)groups);
     inst_begin(c, LESGPU_K_SGS);
-    if (mixed(c)) k_filter<float><<<grid, kThreads, 0, c->stream>>>(c->kp, b, F, run);
-    else k_filter<double><<<grid, kThreads, 0, c->stream>>>(c->kp, b, F, run);
+    if (mixed(c)) chain(k_filter<float>, grid, kThreads, 0, c->stream)(c->kp, b, F, run);
+    else chain(k_filter<double>, grid, kThreads, 0, c->stream)(c->kp, b, F, run);
     inst_end(c, LESGPU_K_SGS);
 }
 
@@ -297,6 +300,7 @@ static void filter_batch(lesgpu_case *c, FiltBatch &F) {
 // scr[24..32]; out: uui[0..2], llij[0..5] in scr[3..11]
 template <class R>
 __global__ void __launch_bounds__(kThreads) k_vreman2(KP p, Box b) {
+    chained();
     const Mir<R> &M = mir<R>(p);
     const DGrid &g = p.g;
     GRID_LOOP(b) {
@@ -325,6 +329,7 @@ __global__ void __launch_bounds__(kThreads) k_vreman2(KP p, Box b) {
 }
 
 __global__ void __launch_bounds__(kThreads) k_vreman2_64(KP p, Box b) {
+    chained();
     const Stn &T = p.st;
     GRID_LOOP(b) {
         int i, j, k;
@@ -375,6 +380,7 @@ struct CsgstsFinal {
 };
 
 __global__ void k_zero_list(KP p, double *f) {
+    chained();
     for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < p.c.nzero; l += gridDim.x * blockDim.x)
         f[p.g.ix(p.f.inz[l + 1], p.f.jnz[l + 1], p.f.knz[l + 1])] = 0.0;
 }
@@ -417,6 +423,7 @@ struct ZeroFinal {
 // operations instead of nine -- the pass is FP64-pipe bound on GB300.
 __global__ void __launch_bounds__(kThreads) k_edge_interp(KP p, Box b, const double *f, double *f1, double *f2,
                                                            double *f3, int ib, int jb, int kb) {
+    chained();
     const DGrid &g = p.g;
     const long long n2 = g.n2 + 1, n3 = g.n3 + 1;
     GRID_LOOP(b) {
@@ -443,6 +450,7 @@ __global__ void __launch_bounds__(kThreads) k_edge_interp(KP p, Box b, const dou
 // the reference's order (x, then y, then z)
 __global__ void k_edge_bc(KP p, int dir, const double *f, double *f1, double *f2, double *f3,
                           int lo0, int hi0, int lo1, int hi1, int full) {
+    chained();
     const DGrid &g = p.g;
     const DCfg &c = p.c;
     const double *f2fx = g.f2fx, *f2fy = g.f2fy, *f2fz = g.f2fz;
@@ -514,19 +522,19 @@ static void edge_interpol(lesgpu_case *c, double *f, double **f1, int full) {
     if (cf.zprdic == 1) { GhostSpec s[1] = {{f, 0, g.n1, 0, g.n2}}; ghost(c, 2, s, 1); }
     int ib = full ? 1 : g.i_bgpx, jb = full ? 1 : g.j_bgpy, kb = full ? 1 : g.k_bgpz;
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
-    k_edge_interp<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, f, f1[0], f1[1], f1[2], ib, jb, kb);
+    chain(k_edge_interp, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, f, f1[0], f1[1], f1[2], ib, jb, kb);
     long long nx = (long long)(g.n2m - jb + 1) * (g.n3m - kb + 1);
     long long ny = (long long)(g.n1m - ib + 1) * (g.n3m - kb + 1);
     long long nz = (long long)(g.n1m - ib + 1) * (g.n2m - jb + 1);
-    k_edge_bc<<<blocks_for(nx), kThreads, 0, c->stream>>>(c->kp, 0, f, f1[0], f1[1], f1[2], jb, g.n2m, kb, g.n3m, full);
-    k_edge_bc<<<blocks_for(ny), kThreads, 0, c->stream>>>(c->kp, 1, f, f1[0], f1[1], f1[2], ib, g.n1m, kb, g.n3m, full);
-    k_edge_bc<<<blocks_for(nz), kThreads, 0, c->stream>>>(c->kp, 2, f, f1[0], f1[1], f1[2], ib, g.n1m, jb, g.n2m, full);
+    chain(k_edge_bc, blocks_for(nx), kThreads, 0, c->stream)(c->kp, 0, f, f1[0], f1[1], f1[2], jb, g.n2m, kb, g.n3m, full);
+    chain(k_edge_bc, blocks_for(ny), kThreads, 0, c->stream)(c->kp, 1, f, f1[0], f1[1], f1[2], ib, g.n1m, kb, g.n3m, full);
+    chain(k_edge_bc, blocks_for(nz), kThreads, 0, c->stream)(c->kp, 2, f, f1[0], f1[1], f1[2], ib, g.n1m, jb, g.n2m, full);
 }
 
 static void zero_in_body(lesgpu_case *c, double *f, int thermal, bool scale) {
     const DGrid &g = c->kp.g;
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
-    if (c->kp.c.nzero > 0) k_zero_list<<<blocks_for(c->kp.c.nzero), kThreads, 0, c->stream>>>(c->kp, f);
+    if (c->kp.c.nzero > 0) chain(k_zero_list, blocks_for(c->kp.c.nzero), kThreads, 0, c->stream)(c->kp, f);
     if (scale) reduce<2, 2u>(c, b, ZeroTerm<true>{f, thermal}, ZeroFinal{thermal});
     else reduce<2, 2u>(c, b, ZeroTerm<false>{f, thermal}, ZeroFinal{thermal});
 }
@@ -542,15 +550,15 @@ void launch_sgs(lesgpu_case *c) {
     DFields &f = c->kp.f;
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     if (c->kp.c.idvmon == 1) {
-        if (mixed(c)) k_vreman1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
-        else k_vreman1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
+        if (mixed(c)) chain(k_vreman1<float>, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, 1);
+        else chain(k_vreman1_64, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, 1);
         FiltBatch F{};
         F.na = 15;
         for (int m = 0; m < 6; m++) { F.src[m] = f.scr[3 + m]; F.dst[m] = f.scr[18 + m]; }
         for (int m = 0; m < 9; m++) { F.src[6 + m] = f.scr[9 + m]; F.dst[6 + m] = f.scr[24 + m]; }
         filter_batch(c, F);
-        if (mixed(c)) k_vreman2<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
-        else k_vreman2_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+        if (mixed(c)) chain(k_vreman2<float>, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b);
+        else chain(k_vreman2_64, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b);
         FiltBatch G{};
         G.na = 9;
         for (int m = 0; m < 9; m++) { G.src[m] = f.scr[3 + m]; G.dst[m] = f.scr[24 + m]; }
@@ -558,8 +566,8 @@ void launch_sgs(lesgpu_case *c) {
         if (mixed(c)) reduce<2, 0u>(c, b, LmMmTerm<float>{}, CsgstsFinal{});
         else reduce<2, 0u>(c, b, LmMmTerm<double>{}, CsgstsFinal{});
     } else {
-        if (mixed(c)) k_vreman1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
-        else k_vreman1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
+        if (mixed(c)) chain(k_vreman1<float>, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, 0);
+        else chain(k_vreman1_64, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, 0);
     }
 }
 
@@ -572,6 +580,7 @@ void launch_sgs_post(lesgpu_case *c, bool scale) {
 // pass 1 of sgs_edm: mm[0..2] scr[3..5]; s[0..5] scr[6..11]; tgrad[0..2] scr[12..14]
 template <class R>
 __global__ void __launch_bounds__(kThreads) k_edm1(KP p, Box b, int dynamic) {
+    chained();
     const Mir<R> &M = mir<R>(p);
     const DGrid &g = p.g;
     GRID_LOOP(b) {
@@ -604,6 +613,7 @@ __global__ void __launch_bounds__(kThreads) k_edm1(KP p, Box b, int dynamic) {
 // The FP64 form (k_grad64.cuh): 64^3 150 us -> 43 (the pow of the filter width
 // alone was some 150 operations).
 __global__ void __launch_bounds__(kThreads) k_edm1_64(KP p, Box b, int dynamic) {
+    chained();
     const DGrid &g = p.g;
     const Stn &T = p.st;
     GRID_LOOP(b) {
@@ -645,6 +655,7 @@ __global__ void __launch_bounds__(kThreads) k_edm1_64(KP p, Box b, int dynamic) 
 // llij[0..2] scr[7..9]
 template <class R>
 __global__ void __launch_bounds__(kThreads) k_edm2(KP p, Box b) {
+    chained();
     const Mir<R> &M = mir<R>(p);
     const DGrid &g = p.g;
     GRID_LOOP(b) {
@@ -670,6 +681,7 @@ __global__ void __launch_bounds__(kThreads) k_edm2(KP p, Box b) {
 }
 
 __global__ void __launch_bounds__(kThreads) k_edm2_64(KP p, Box b) {
+    chained();
     const Stn &T = p.st;
     GRID_LOOP(b) {
         int i, j, k;
@@ -722,15 +734,15 @@ void launch_sgs_t(lesgpu_case *c) {
     DFields &f = c->kp.f;
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
     if (c->kp.c.idvmon == 1) {
-        if (mixed(c)) k_edm1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
-        else k_edm1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 1);
+        if (mixed(c)) chain(k_edm1<float>, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, 1);
+        else chain(k_edm1_64, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, 1);
         FiltBatch F{};
         F.na = 12;
         for (int m = 0; m < 3; m++) { F.src[m] = f.scr[3 + m]; F.dst[m] = f.scr[18 + m]; }
         for (int m = 0; m < 9; m++) { F.src[3 + m] = f.scr[6 + m]; F.dst[3 + m] = f.scr[21 + m]; }
         filter_batch(c, F);
-        if (mixed(c)) k_edm2<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
-        else k_edm2_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b);
+        if (mixed(c)) chain(k_edm2<float>, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b);
+        else chain(k_edm2_64, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b);
         FiltBatch G{};
         G.na = 7;
         for (int m = 0; m < 7; m++) { G.src[m] = f.scr[3 + m]; G.dst[m] = f.scr[24 + m]; }
@@ -738,8 +750,8 @@ void launch_sgs_t(lesgpu_case *c) {
         if (mixed(c)) reduce<2, 0u>(c, b, LmMmTTerm<float>{}, CsgshfFinal{});
         else reduce<2, 0u>(c, b, LmMmTTerm<double>{}, CsgshfFinal{});
     } else {
-        if (mixed(c)) k_edm1<float><<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
-        else k_edm1_64<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, 0);
+        if (mixed(c)) chain(k_edm1<float>, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, 0);
+        else chain(k_edm1_64, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, 0);
     }
 }
 

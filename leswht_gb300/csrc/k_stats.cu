@@ -10,6 +10,7 @@
 namespace lg {
 
 __global__ void __launch_bounds__(kThreads) k_field_avg(KP p, Box b, double *avg) {
+    chained();
     const DGrid &g = p.g;
     const DScal *S = p.S;
     if (!(S->time > p.c.avg_tst)) return;          // field_avg returns while time <= AVG_TST
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(kThreads) k_field_avg(KP p, Box b, double *avg
 void launch_field_avg(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     Box b{1, 1, 1, g.n1m, g.n2m, g.n3m};
-    k_field_avg<<<blocks_for(b.count()), kThreads, 0, c->stream>>>(c->kp, b, c->kp.f.avg);
+    chain(k_field_avg, blocks_for(b.count()), kThreads, 0, c->stream)(c->kp, b, c->kp.f.avg);
 }
 
 }  // namespace lg

@@ -176,6 +176,7 @@ struct MirBatch {
 
 // FP64 -> FP32 (round to nearest, as the per-load conversions it replaces)
 __global__ void __launch_bounds__(kThreads) k_mirror(MirBatch b, long long nt) {
+    chained();
     const long long npair = nt >> 1;
     const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, st = (long long)gridDim.x * blockDim.x;
     for (int a = 0; a < b.n; a++) {
@@ -212,7 +213,7 @@ void launch_mirror(lesgpu_case *c, unsigned sets) {
     const long long nt = c->kp.g.nt;
     int nb = blocks_for(nt / 2 + 1);
     if (nb > 4 * 152) nb = 4 * 152;
-    k_mirror<<<nb, kThreads, 0, c->stream>>>(b, nt);
+    chain(k_mirror, nb, kThreads, 0, c->stream)(b, nt);
 }
 }  // namespace lg
 
@@ -714,6 +715,7 @@ extern "C" int lesgpu_set_fields(lesgpu_case *c, const double *u, const double *
 
 // ------------------------------------------------------------------ start
 __global__ void k_start(KP p) {
+    chained();
     DScal *S = p.S;
     S->ntime = 0;
     S->cflmax = p.c.cflfac;
@@ -732,7 +734,7 @@ extern "C" int lesgpu_start(lesgpu_case *c) {
     if (g.idtopt != 0 && g.iread == 0) s.dt = g.dt_size;
     if (g.ireset == 1) { s.ihist = 0; s.time = 0.0; }
     cudaMemcpyAsync(c->S, &s, sizeof(DScal), cudaMemcpyHostToDevice, c->stream);
-    k_start<<<1, 1, 0, c->stream>>>(c->kp);
+    chain(k_start, 1, 1, 0, c->stream)(c->kp);
     launch_mirror(c, kMirConj | kMirNu | kMirAl);
     if (g.ich != 0) launch_meanpg(c);
     if (g.ihtrans == 1 && g.ich == 1) launch_cvol(c);
@@ -761,6 +763,7 @@ extern "C" int lesgpu_start(lesgpu_case *c) {
 
 // ------------------------------------------------------------------- step
 __global__ void k_retrv_uvw(KP p) {   // retrv_uvw, slv_mmtm.f90:1710-1743
+    chained();
     const DGrid &g = p.g;
     long long n = (long long)g.n2m * g.n3m;
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (long long)gridDim.x * blockDim.x) {
@@ -796,7 +799,7 @@ static void enqueue_rhsnlhs(lesgpu_case *c, int msub) {
     if (c->cfg.ibmon != 0) launch_rhs_ibm(c);
     launch_convbc(c);
     launch_adi_uvw(c);
-    k_retrv_uvw<<<blocks_for((long long)c->kp.g.n2m * c->kp.g.n3m), kThreads, 0, c->stream>>>(c->kp);
+    chain(k_retrv_uvw, blocks_for((long long)c->kp.g.n2m * c->kp.g.n3m), kThreads, 0, c->stream)(c->kp);
     launch_ghost_uvw(c);
     mark_mirror(c, kMirVel);
 }
@@ -1268,7 +1271,10 @@ extern "C" int lesgpu_run_phase(lesgpu_case *c, int64_t phase, int64_t msub) {
 }
 
 // ----------------------------------------------------------- field_avg
-__global__ void k_avg_reset_count(KP p) { p.S->avg_count = 0; }
+__global__ void k_avg_reset_count(KP p) {
+    chained();
+    p.S->avg_count = 0;
+}
 
 // The interior cells of the sums, packed array by array into the step's
 // scratch (free between steps).  A strided device-to-host copy straight from
@@ -1279,6 +1285,7 @@ struct PackArgs {
     double *dst[LESGPU_NAVG];
 };
 __global__ void __launch_bounds__(kThreads) k_pack(PackArgs a, DGrid g, Box b) {
+    chained();
     const long long n = b.count();
     const double *src = a.src[blockIdx.y];
     double *dst = a.dst[blockIdx.y];
@@ -1307,7 +1314,7 @@ extern "C" int lesgpu_get_averages(lesgpu_case *c, double *out, int64_t *nsample
                 PackArgs p;
                 for (int a = 0; a < n; a++) { p.src[a] = avg + nt * (a0 + a); p.dst[a] = c->kp.f.scr[a]; }
                 const int nb = blocks_for(b.count());
-                k_pack<<<dim3(nb > 65535 ? 65535 : nb, n), kThreads, 0, c->stream>>>(p, g, b);
+                chain(k_pack, dim3(nb > 65535 ? 65535 : nb, n), kThreads, 0, c->stream)(p, g, b);
                 const int rc = to_host((CaseExtra *)c->dmem_pool, c->stream, out + nc * a0, p.dst, n, nc);
                 if (rc) return rc;
             }
@@ -1319,7 +1326,7 @@ extern "C" int lesgpu_get_averages(lesgpu_case *c, double *out, int64_t *nsample
     if (nsamples) *nsamples = s.avg_count;
     if (reset) {
         if (avg) cudaMemsetAsync(avg, 0, sizeof(double) * nt * LESGPU_NAVG, c->stream);
-        k_avg_reset_count<<<1, 1, 0, c->stream>>>(c->kp);
+        chain(k_avg_reset_count, 1, 1, 0, c->stream)(c->kp);
         if (cudaStreamSynchronize(c->stream) != cudaSuccess) return LESGPU_ERR_CUDA;
     }
     return 0;

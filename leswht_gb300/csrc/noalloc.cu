@@ -114,6 +114,7 @@ struct TableDst {
 // A block row per table (the transcendental functions are FP64-pipe bound, 64
 // clocks an operation of a warp: one warp should not walk through all four).
 __global__ void __launch_bounds__(64) k_noalloc_tables(YTables y, TableDst d, int n1m, int n2m, int n3m, double sdxis, double sdzis) {
+    lg::chained();
     const int n1mh = n1m / 2 + 1, n3mh = n3m / 2 + 1;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     double s, c;
@@ -227,7 +228,7 @@ extern "C" int lesgpu_poisson_ftft_noalloc(const lesgpu_grid *g, const double *d
     d.rows = (double4 *)(base + o_rows);
     d.twx = (double2 *)(base + o_twx);
     d.twz = (double2 *)(base + o_twz);
-    k_noalloc_tables<<<dim3((std::max(n1m, std::max(n2m, n3m)) + 3 + 63) / 64, 5), 64, 0, st>>>(y, d, n1m, n2m, n3m, g->f2fxi[1], g->f2fzi[1]);
+    lg::chain(k_noalloc_tables, dim3((std::max(n1m, std::max(n2m, n3m)) + 3 + 63) / 64, 5), 64, 0, st)(y, d, n1m, n2m, n3m, g->f2fxi[1], g->f2fzi[1]);
 
     lg::KP p;
     memset(&p, 0, sizeof(p));
@@ -257,7 +258,7 @@ extern "C" int lesgpu_poisson_ftft_noalloc(const lesgpu_grid *g, const double *d
     lg::fft_z_fwd64(gz, smz, st, p, p.f.divgsum, ccap, pz, Lz, sk, sj);
     lg::fft_x64((nxl + Lx - 1) / Lx, smx, st, ccap, nxl, px, Lx, 0);
     long long nl = (long long)n1m * n3mh;
-    lg::k_ytri_elim<<<lg::blocks_for((nl + 15) / 16 * 32, 64), 64, 0, st>>>(n1m, n2m, n3mh, ccap, d.ak1, d.ak3, d.rows, gam);
+    lg::chain(lg::k_ytri_elim, lg::blocks_for((nl + 15) / 16 * 32, 64), 64, 0, st)(n1m, n2m, n3mh, ccap, d.ak1, d.ak3, d.rows, gam);
     lg::fft_x64((nxl + Lx - 1) / Lx, smx, st, ccap, nxl, px, Lx, 1);
     lg::fft_z_inv64(gz, smz, st, p, ccap, pz, Lz, sk, sj);
     // a launch that failed leaves its error pending; report it, leave it for the caller to see
