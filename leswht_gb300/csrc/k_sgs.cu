@@ -213,6 +213,9 @@ struct FiltBatch {
 // most of the instructions.  The mean of a step's four
 // launches, us: 64^3 FP64 63 -> 43, FP32 12.9 -> 9.5; 384x256x384 FP32
 // 1479 -> 860.
+// The fused sums' order is what the compiler makes of c0 l + c1 m + c2 r, so
+// the mixed form's coefficient keeps its bits (another order moves it by up to 5e-5,
+// and every eddy viscosity with it).
 constexpr int kFiltA = 3;
 
 template <class R>
@@ -244,7 +247,7 @@ __global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F, i
         const R *cfx = mir<R>(p).cfx1 + 3 * i;
         const R c0 = cfx[0], c1 = cfx[1], c2 = cfx[2];
         auto xval = [&](const R *__restrict__ r) {
-            const R x = r[0], y = fma(c2, r[op], fma(c1, x, c0 * r[om]));
+            const R x = r[0], y = fma(c2, r[op], fma(c0, r[om], c1 * x));
             return filt ? y : x;
         };
         R xm[kFiltA], x0[kFiltA];
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F, i
             for (int a = 0; a < kFiltA; a++) xp[a] = xval(s[a] + qp);
 #pragma unroll
             for (int a = 0; a < kFiltA; a++) {
-                const R y = fma(z2, xp[a], fma(z1, x0[a], z0 * xm[a]));
+                const R y = fma(z2, xp[a], fma(z0, xm[a], z1 * x0[a]));
                 if (a < na) d[a][q] = zin ? y : x0[a];
                 xm[a] = x0[a];
                 x0[a] = xp[a];
