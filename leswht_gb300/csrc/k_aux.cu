@@ -24,7 +24,8 @@ struct CflTerm {
         const long long q = g.ix(i, j, k);
         const double c1 = abs_bits(p.f.u[q] + p.f.u[q + 1]), c2 = abs_bits(p.f.v[q] + p.f.v[q + g.sx]);
         const double c3 = abs_bits(p.f.w[q] + p.f.w[q + g.sxy]);
-        x[0] = fma(c3, p.st.hz[k], fma(c2, p.st.hy[j], c1 * p.st.hx[i]));
+        // in the order c1 + c2 + c3 has always been contracted: the time step's bits
+        x[0] = fma(c3, p.st.hz[k], fma(c1, p.st.hx[i], c2 * p.st.hy[j]));
     }
     __device__ void add(const KP &, int, int, int, const double *x, double *v) const {
         take_max(v[0], x[0]);
@@ -93,8 +94,8 @@ __global__ void k_substepinit(KP p, int s, int carry) {
     const double gam[4] = {0.0, 8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
     const double ro[4] = {0.0, 0.0, -17.0 / 60.0, -5.0 / 12.0};
     DScal *S = p.S;
-    // the projection's metric factors (k_ucalc), a multiplication per line
-    // and not one per cell
+    // the metric factors of the projection with flow rates (UcalcQvolTerm), a
+    // multiplication per line and not one per cell
     const double dtc = S->dt * (gam[s] + ro[s]);
     const DGrid &g = p.g;
     for (int i = threadIdx.x; i <= g.n1; i += blockDim.x) p.st.px[i] = dtc * g.c2cxi[i];
@@ -346,15 +347,16 @@ __global__ void __launch_bounds__(kThreads) k_ucalc(KP p, Box b) {
     chained();
     long long n = b.count();
     const DGrid &g = p.g;
+    const double dtc = p.S->dtconst;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         b.at(t, i, j, k);
         long long q = g.ix(i, j, k);
         const double *phi = p.f.phi;
         double ph = phi[q];
-        if (i >= g.i_bgpx) p.f.u[q] = fma(phi[g.ix(g.imv[i], j, k)] - ph, p.st.px[i], p.f.u[q]);
-        if (j >= 2) p.f.v[q] = fma(phi[q - g.sx] - ph, p.st.py[j], p.f.v[q]);
-        if (k >= g.k_bgpz) p.f.w[q] = fma(phi[g.ix(i, j, g.kmv[k])] - ph, p.st.pz[k], p.f.w[q]);
+        if (i >= g.i_bgpx) p.f.u[q] = p.f.u[q] - dtc * (ph - phi[g.ix(g.imv[i], j, k)]) * g.c2cxi[i];
+        if (j >= 2) p.f.v[q] = p.f.v[q] - dtc * (ph - phi[q - g.sx]) * g.c2cyi[j];
+        if (k >= g.k_bgpz) p.f.w[q] = p.f.w[q] - dtc * (ph - phi[g.ix(i, j, g.kmv[k])]) * g.c2czi[k];
     }
 }
 
@@ -477,14 +479,16 @@ __global__ void __launch_bounds__(kThreads) k_pcalc(KP p, Box b) {
     chained();
     long long n = b.count();
     const DGrid &g = p.g;
-    // three FP64 operations a cell, the factor formed once for a thread's cells
-    // (384x256x384 368 us with one cell a thread -> 240)
-    const double phiref = p.S->phiref, h = 0.5 * p.S->dtconst * p.c.rei_d;
+    // four FP64 operations a cell, in the order the pressure has always been
+    // summed: the mixed form's momentum kernel differences p in FP32, so its
+    // last bits show in w (k_mg.cu, kMgFineSpan)
+    const double dtc = p.S->dtconst, phiref = p.S->phiref, rei = p.c.rei_d;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         b.at(t, i, j, k);
         long long q = g.ix(i, j, k);
-        p.f.p[q] = fma(-h, p.f.divgsum[q], p.f.p[q] + (p.f.phi[q] - phiref));
+        const double pn = p.f.p[q] + p.f.phi[q] - 0.5 * dtc * p.f.divgsum[q] * rei;
+        p.f.p[q] = pn - phiref;
     }
 }
 

@@ -1632,6 +1632,16 @@ static int mgl_init(lesgpu_case *c) {
     return mgl_set_cluster(c, pick);
 }
 
+// Cells a unit length in z from which the mixed form keeps the cycle in global
+// memory.  The two cycles round their FP32 corrections differently, which
+// leaves p 1e-10 apart; the momentum kernel differences p in FP32, and where
+// that turns one rounding of p, w jumps by ulp(p) dt / dz.  Beside a body set
+// off from rest p is 100 to 200: at 64 cells over pi (dz = 1/20) a jump is up
+// to 1.2e-3 of w's rms, past the 8e-4 its results are held to, at 48 cells
+// (1/15) 5e-4, at 16 cells 3e-4.  A 256x192x64 solve takes 10.0 ms so and
+// 2.3 ms resident.
+constexpr double kMgFineSpan = 16.0;
+
 int mg2d_init(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     const lesgpu_config &cf = c->cfg;
@@ -1661,7 +1671,8 @@ int mg2d_init(lesgpu_case *c) {
     {   // resident cycles wherever some cluster holds a mode (and no mode runs SOR)
         MgLineArgs a;
         size_t sm;
-        const bool ok = nmodes <= cf.imgsor && 4 * nlev + 2 * cf.nbli + 8 <= kMglMaxPhase;
+        const bool fine = T->mixed && !xft && c->h_grid->f2fzi[1] > kMgFineSpan;
+        const bool ok = !fine && nmodes <= cf.imgsor && 4 * nlev + 2 * cf.nbli + 8 <= kMglMaxPhase;
         for (int cs = 1; cs <= 16 && ok; cs <<= 1)
             if (mgl_plan(*T, g.n2m, cs, a, sm)) T->resident = 1;
     }

@@ -374,11 +374,14 @@ __device__ __forceinline__ void take_max(double &m, double x) {
 }
 
 // Deterministic block totals of NV doubles (the sum, or the maximum for the
-// values in MAXM); every thread gets them.  Warp q totals value q: eight
-// partials a lane, then a shuffle tree -- twelve dependent FP64 operations
-// whatever NV, where a tree of every value in every warp took fifteen NV.
+// values in MAXM); every thread gets them.  The order is that of a shuffle
+// tree in every warp (lanes 16, 8, 4, 2, 1 apart) and one over the warps'
+// totals (4, 2, 1 apart), but warp q runs all of value q's trees, level by
+// level with its lanes full: twelve dependent FP64 operations whatever NV,
+// where every warp running a tree of every value took fifteen NV.
 template <int NV, unsigned MAXM>
 __device__ __forceinline__ void block_totals(double (&v)[NV]) {
+    static_assert(kThreads == 256, "eight warps");
     __shared__ double sh[NV][kThreads];
     __shared__ double tot[NV];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -387,17 +390,25 @@ __device__ __forceinline__ void block_totals(double (&v)[NV]) {
     __syncthreads();
     if (wid < NV) {
         const bool mx = (MAXM >> wid) & 1u;
-        double x = sh[wid][lane];
+        auto op = [&](double a, double b) { return mx ? max_bits(a, b) : a + b; };
+        // the half of a pair of lists this lane keeps gets its partner's part of it
+        auto fold = [&](double a, double b, int o) {
+            const bool up = lane & o;
+            const double got = __shfl_xor_sync(0xffffffffu, up ? a : b, o);
+            return op(up ? b : a, got);
+        };
+        double a[4];
 #pragma unroll
-        for (int w = 1; w < kThreads / 32; w++) {
-            const double y = sh[wid][lane + 32 * w];
-            if (mx) x = max_bits(x, y);
-            else x = x + y;
+        for (int s = 0; s < 4; s++) {            // lanes 16 apart of warps 2s and 2s + 1
+            const double *w = sh[wid] + 64 * s + 32 * (lane >> 4) + (lane & 15);
+            a[s] = op(w[0], w[16]);
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double y = __shfl_down_sync(0xffffffffu, x, o);
-            if (mx) x = max_bits(x, y);
-            else x = x + y;
+        double x = fold(fold(a[0], a[1], 8), fold(a[2], a[3], 8), 4);
+        // lane bits 4, 3, 2 now name the warp (bits 0, 1, 2), bits 1, 0 the rest of its list
+#pragma unroll
+        for (int s = 0; s < 5; s++) {
+            const int o = s < 2 ? 2 >> s : 4 << (s - 2);
+            x = op(x, __shfl_xor_sync(0xffffffffu, x, o));
         }
         if (lane == 0) tot[wid] = x;
     }
