@@ -1921,7 +1921,10 @@ long long mg2d_batch_key(const lesgpu_case *c) {
 // the others finish early -- and its cycle count depends on the data, so the
 // candidates are timed on that mode alone, three V-cycles with the
 // convergence test off (results go to scratch).
-static std::map<std::array<int, 7>, int> g_zft_cs;
+// The table's key holds all that decides which clusters hold a mode: the shape,
+// and the form and cycle with it (FP64 lines take twice the shared memory; the
+// cycle in global memory wants even ranges of lines instead).
+static std::map<std::array<int, 9>, int> g_zft_cs;
 static std::mutex g_zft_mu;
 
 // A seeded noise right-hand side of every mode for the timing runs.
@@ -1970,7 +1973,7 @@ int mg2d_autotune(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     MgTables *T = c->pois.mg;
     if (!T || (c->cfg.poisson != LESGPU_POISSON_Z_FT && c->cfg.poisson != LESGPU_POISSON_X_FT)) return 0;
-    const std::array<int, 7> key{T->xft, g.n1m, g.n2m, g.n3m, T->nlev, (int)c->cfg.imgsor, T->cap};
+    const std::array<int, 9> key{T->xft, g.n1m, g.n2m, g.n3m, T->nlev, (int)c->cfg.imgsor, T->cap, T->mixed, T->resident};
     {
         std::lock_guard<std::mutex> lk(g_zft_mu);
         auto it = g_zft_cs.find(key);
