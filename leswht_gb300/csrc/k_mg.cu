@@ -1593,6 +1593,15 @@ static void mgl_launch(lesgpu_case *c, int slot) {
     cudaLaunchKernelEx(&lc, mgl_kernel(T, c->kp.g.n2m), (const MgLineArgs *)T.dargs + slot, T.nmodes);
 }
 
+static bool mgl_attributes(const MgTables &T, int n2m) {
+    const MglKernel k = mgl_kernel(T, n2m);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMglSmem) == cudaSuccess &&
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
+        return true;
+    cudaGetLastError();
+    return false;
+}
+
 static int mgl_init(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     DPois &P = c->pois;
@@ -1610,10 +1619,6 @@ static int mgl_init(lesgpu_case *c) {
     } else {
         if (fft_smem64(kFftSmemMax)) return LESGPU_ERR_CUDA;
     }
-    const MglKernel k = mgl_kernel(*T, g.n2m);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMglSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        return LESGPU_ERR_CUDA;
     int cap = mg_cluster_cap();
     const char *env = getenv("LESGPU_MG_CLUSTER_MAX");
     if (env && atoi(env) >= 1) cap = atoi(env);
@@ -1673,8 +1678,12 @@ int mg2d_init(lesgpu_case *c) {
         size_t sm;
         const bool fine = T->mixed && !xft && c->h_grid->f2fzi[1] > kMgFineSpan;
         const bool ok = !fine && nmodes <= cf.imgsor && 4 * nlev + 2 * cf.nbli + 8 <= kMglMaxPhase;
-        for (int cs = 1; cs <= 16 && ok; cs <<= 1)
-            if (mgl_plan(*T, g.n2m, cs, a, sm)) T->resident = 1;
+        bool fits = false;
+        for (int cs = 1; cs <= 16 && ok; cs <<= 1) fits = fits || mgl_plan(*T, g.n2m, cs, a, sm);
+        // and the device takes one of them: 16 blocks, or a block of all the
+        // shared memory, are more than every device gives
+        if (fits && mgl_attributes(*T, g.n2m))
+            for (int cs = 1; cs <= 16 && !T->resident; cs <<= 1) T->resident = mgl_active(c, cs) >= 1;
     }
     rc = set_up_tables(c, *T);
     if (rc) return rc;
