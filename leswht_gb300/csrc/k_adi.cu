@@ -1767,23 +1767,38 @@ int adi_tuned(const lesgpu_case *c, int *out, int maxn) {
 // Self-check of the FP64 pivot reciprocal (no reference counterpart): r[q] =
 // rcp_pivot(x[q]) for n host values, so a test can bound its error.
 namespace lg {
-__global__ void k_rcp_check(const double *x, double *r, long long n) {
+__global__ void k_rcp_check(const double *x, double *r, double *fast, double *ok, long long n) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n) r[q] = rcp_pivot<double>(x[q]);
+    if (q >= n) return;
+    r[q] = rcp_pivot<double>(x[q]);
+    bool in = true;
+    fast[q] = rcp_fp64_fast(x[q], in);
+    ok[q] = in ? 1.0 : 0.0;
+}
+// both reciprocals of n values, and where the branch-free one holds
+static int check_rcp(const double *x, double *r, double *fast, double *ok, int64_t n) {
+    const size_t bytes = sizeof(double) * (size_t)n;
+    double *d = nullptr;
+    if (cudaMalloc(&d, 4 * bytes) != cudaSuccess) return LESGPU_ERR_OOM;
+    int rc = 0;
+    if (cudaMemcpy(d, x, bytes, cudaMemcpyHostToDevice) != cudaSuccess) rc = LESGPU_ERR_CUDA;
+    if (!rc) {
+        k_rcp_check<<<(unsigned)((n + 255) / 256), 256>>>(d, d + n, d + 2 * n, d + 3 * n, (long long)n);
+        double *const to[3] = {r, fast, ok};
+        for (int q = 0; q < 3; q++)
+            if (to[q] && cudaMemcpy(to[q], d + (q + 1) * n, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) rc = LESGPU_ERR_CUDA;
+    }
+    cudaFree(d);
+    return rc;
 }
 }  // namespace lg
 
 extern "C" int lesgpu_check_rcp(const double *x, double *r, int64_t n) {
     if (n < 0 || (n > 0 && (!x || !r))) return LESGPU_ERR_ARG;
-    if (n == 0) return 0;
-    double *d = nullptr;
-    if (cudaMalloc(&d, sizeof(double) * 2 * (size_t)n) != cudaSuccess) return LESGPU_ERR_OOM;
-    int rc = 0;
-    if (cudaMemcpy(d, x, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice) != cudaSuccess) rc = LESGPU_ERR_CUDA;
-    if (!rc) {
-        lg::k_rcp_check<<<(unsigned)((n + 255) / 256), 256>>>(d, d + n, (long long)n);
-        if (cudaMemcpy(r, d + n, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost) != cudaSuccess) rc = LESGPU_ERR_CUDA;
-    }
-    cudaFree(d);
-    return rc;
+    return n == 0 ? 0 : lg::check_rcp(x, r, nullptr, nullptr, n);
+}
+
+extern "C" int lesgpu_check_rcp_fast(const double *x, double *r, double *ok, int64_t n) {
+    if (n < 0 || (n > 0 && (!x || !r || !ok))) return LESGPU_ERR_ARG;
+    return n == 0 ? 0 : lg::check_rcp(x, nullptr, r, ok, n);
 }
