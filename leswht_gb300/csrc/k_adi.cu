@@ -1578,11 +1578,16 @@ static void adi_launch(lesgpu_case *c, const AdiBatch &B, int ncomp) {
     if (c->autotune) {
         std::lock_guard<std::mutex> lk(g_adi_mu);
         auto it = g_adi_w.find(adi_key(c, B, h));
-        if (it != g_adi_w.end()) w = it->second;
+        // a shape's entry may be of a case without general conjugate tables:
+        // its temperature sweeps then keep the untuned form
+        if (it != g_adi_w.end() && (it->second != kEnds || adi_factored(c, B))) w = it->second;
     }
     if (h.f32 && c->adi_force_f32) w = c->adi_force_f32;
     inst_begin(c, LESGPU_K_ADI);
-    if (!adi_run(c, B, h, w)) adi_run(c, B, h, 1);
+    if (!adi_run(c, B, h, w)) {
+        c->adi_other++;
+        adi_run(c, B, h, 1);
+    }
     inst_end(c, LESGPU_K_ADI);
 }
 
@@ -1801,4 +1806,11 @@ extern "C" int lesgpu_check_rcp(const double *x, double *r, int64_t n) {
 extern "C" int lesgpu_check_rcp_fast(const double *x, double *r, double *ok, int64_t n) {
     if (n < 0 || (n > 0 && (!x || !r || !ok))) return LESGPU_ERR_ARG;
     return n == 0 ? 0 : lg::check_rcp(x, nullptr, r, ok, n);
+}
+
+// sweeps of a case that could not take the form chosen for them, for tests
+extern "C" int lesgpu_check_adi_other(const lesgpu_case *c, int64_t *n) {
+    if (!c || !n) return LESGPU_ERR_ARG;
+    *n = c->adi_other;
+    return 0;
 }

@@ -441,6 +441,7 @@ struct lesgpu_case {
     // LESGPU_ADI_FP32_FORM at start: the form every FP32 sweep uses (lanes
     // per line, + 64 register-capped, 128 tiled; 0 = the autotuner's)
     int adi_force_f32;
+    long long adi_other;        // sweeps enqueued in another form than the one chosen
     // FP32 mirror sets (kMir*) whose FP64 arrays changed since their last
     // refresh, as the enqueued work stands (host-side bookkeeping of the
     // mixed form; launch_mirror converts only these)
