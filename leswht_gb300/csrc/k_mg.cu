@@ -2026,3 +2026,12 @@ int mg2d_autotune(lesgpu_case *c) {
 int mg2d_cluster(const lesgpu_case *c) { return c->pois.mg ? c->pois.mg->cs : 0; }
 
 }  // namespace lg
+
+// what the multigrid of a case runs as, for tests: resident 1 = a mode's lines
+// in its cluster's shared memory; blocks per mode
+extern "C" int lesgpu_check_mg(const lesgpu_case *c, int64_t *resident, int64_t *blocks) {
+    if (!c || !resident || !blocks || !c->pois.mg) return LESGPU_ERR_ARG;
+    *resident = c->pois.mg->resident;
+    *blocks = c->pois.mg->cs;
+    return 0;
+}
