@@ -378,11 +378,11 @@ __device__ __forceinline__ void ycoef(const DGrid &g, const double *ak1, const d
 // at once, by lane l of a half-warp upwards and lane l + 16 downwards, which
 // meet in a 2x2 system: half the dependent rows and twice the warps of the
 // one-ended sweep, which ran 128x125x120's 7808 modes as 244 warps of the
-// GPU's 608 sub-partitions.  A row costs 11 FP64 operations (64 clocks each
+// GPU's 608 sub-partitions.  A row costs 10 FP64 operations (64 clocks each
 // of a warp), 12 with the back substitution's two, from precomputed rows.
 // 128x125x120: 194 us one-ended, 55 this way.
 __global__ void __launch_bounds__(64) k_ytri_elim(int n1m, int n2m, int n3mh, double2 *ccap, const double *ak1, const double *ak3,
-                                                  const double4 *rows, double *gam) {
+                                                  YRows rows, double *gam) {
     chained();
     const long long nl = (long long)n1m * n3mh, sj = nl;
     const int lane = threadIdx.x & 31, up = lane >> 4;      // up: the half that comes down from row n2m
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(64) k_ytri_elim(int n1m, int n2m, int n3mh, do
          w += ((long long)gridDim.x * blockDim.x) >> 5) {
         const long long t0 = w * 16 + (lane & 15), t = t0 < nl ? t0 : nl - 1;
         const bool on = t0 < nl;
-        const double akk = ak1[1 + (int)(t % n1m)] + ak3[1 + (int)(t / n1m)];
+        const double akk = ak1[1 + (int)(t % n1m)] + ak3[1 + (int)(t / n1m)], akk2 = 2.0 * akk;
         double2 *r = ccap + t;
         double *gm = gam + t;
         const bool pin = t == 0;
@@ -403,20 +403,23 @@ __global__ void __launch_bounds__(64) k_ytri_elim(int n1m, int n2m, int n3mh, do
         double bet = 0.0, cprev = 0.0;
         double2 x = make_double2(0.0, 0.0);
         for (int q0 = 0; q0 < n; q0 += U) {
-            double2 rv[U];
-            double4 cf[U];
+            double2 rv[U], cf[U];
+            double cd[U];
+            int cb[U];
 #pragma unroll
             for (int u = 0; u < U; u++)
                 if (q0 + u < n) {
                     const int j = j0 + dj * (q0 + u);
                     rv[u] = r[(long long)(j - 1) * sj];
-                    cf[u] = rows[j];
+                    cf[u] = rows.a[j];
+                    cd[u] = rows.c[j];
+                    cb[u] = rows.both[j];
                 }
 #pragma unroll
             for (int u = 0; u < U; u++)
                 if (q0 + u < n) {
                     const int j = j0 + dj * (q0 + u);
-                    double lo = up ? cf[u].y : cf[u].x, hi = up ? cf[u].x : cf[u].y, ac = cf[u].z - cf[u].w * akk;
+                    double lo = up ? cf[u].y : cf[u].x, hi = up ? cf[u].x : cf[u].y, ac = cd[u] - (cb[u] ? akk2 : akk);
                     double2 rj = rv[u];
                     if (pin && j == n2m) { ac = 1.0; lo = hi = 0.0; rj = make_double2(0.0, 0.0); }
                     const double g = cprev * bet;
@@ -460,10 +463,9 @@ __global__ void __launch_bounds__(64) k_ytri_elim(int n1m, int n2m, int n3mh, do
         if (w == 0) {
             __syncwarp();
             if (pin && on) {
-                const double4 last = rows[n2m];
+                const double am = rows.a[n2m].x, ajc = rows.c[n2m] - (rows.both[n2m] ? akk2 : akk);
                 const double2 cm = r[(long long)(n2m - 2) * sj];
-                const double ajc = last.z - last.w * akk;
-                const double2 ph = make_double2((-last.x * cm.x + crhsref.x) / ajc, (-last.x * cm.y + crhsref.y) / ajc);
+                const double2 ph = make_double2((-am * cm.x + crhsref.x) / ajc, (-am * cm.y + crhsref.y) / ajc);
                 __syncwarp(0x00010001u);            // both halves have read row n2m - 1
                 for (int q = 0; q < n; q++) {
                     const long long at = (long long)(j0 + dj * q - 1) * sj;

@@ -36,8 +36,14 @@ int fft_smem64(int bytes);
 __global__ void k_fft_xr_fwd(KP p, double2 *ccap, DevPlan P, int L);
 __global__ void k_fft_xr_inv(KP p, const double2 *ccap, DevPlan P, int L, int pin);
 int fft_xr_inv_lines(int n, int L, int pin);
-// rows[j] = (am, ap, c0, w) of row j, the diagonal c0 - w (ak1 + ak3)
-__global__ void k_ytri_elim(int n1m, int n2m, int n3mh, double2 *ccap, const double *ak1, const double *ak3, const double4 *rows,
+// row j of the y systems: a[j] = (am, ap), the diagonal c[j] less ak1 + ak3,
+// twice of it where both[j] (walls above and below the row)
+struct YRows {
+    double2 *a;
+    double *c;
+    int *both;
+};
+__global__ void k_ytri_elim(int n1m, int n2m, int n3mh, double2 *ccap, const double *ak1, const double *ak3, YRows rows,
                             double *gam);
 __global__ void k_ytri_lu(KP p, const double *ak1, const double *ak3, double *ybet, double *ygam, double *yam,
                           double *pinref);

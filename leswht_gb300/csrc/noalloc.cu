@@ -103,7 +103,7 @@ struct YTables {
 
 struct TableDst {
     double *ak1, *ak3;
-    double4 *rows;              // (am, ap, c0, w) of row j (k_ytri_elim)
+    lg::YRows rows;             // of the y systems (k_ytri_elim)
     double2 *twx, *twz;
 };
 
@@ -141,8 +141,9 @@ __global__ void __launch_bounds__(64) k_noalloc_tables(YTables y, TableDst d, in
         if (t >= 1 && t <= n2m) {
             const double fl = y.fixjl[t], fu = y.fixju[t], in = (1.0 - fl) * (1.0 - fu);
             const double am = y.f2fyi[t] * y.c2cyi[t] * (1.0 - fl), ap = y.f2fyi[t] * y.c2cyi[y.jpv[t]] * (1.0 - fu);
-            d.rows[t] = make_double4(am, ap, -((am + ap) * in + y.f2fyi[1] * y.c2cyi[2] * fl + y.f2fyi[n2m] * y.c2cyi[n2m] * fu),
-                                     in + fl + fu);
+            d.rows.a[t] = make_double2(am, ap);
+            d.rows.c[t] = -((am + ap) * in + y.f2fyi[1] * y.c2cyi[2] * fl + y.f2fyi[n2m] * y.c2cyi[n2m] * fu);
+            d.rows.both[t] = y.fixjl[t] && y.fixju[t];
         }
     }
 }
@@ -192,7 +193,12 @@ extern "C" int lesgpu_poisson_ftft_noalloc(const lesgpu_grid *g, const double *d
     size_t off = 0;
     const size_t o_ak1 = off; off = align256(off + sizeof(double) * (n1 + 2));
     const size_t o_ak3 = off; off = align256(off + sizeof(double) * (n3mh + 2));
-    const size_t o_rows = off; off = align256(off + sizeof(double4) * (n2m + 1));
+    // the rows take the room of the five wall-normal tables they are formed
+    // from (two of doubles, three of ints), so the limit accepts the sizes it
+    // would with those
+    const size_t o_rows_a = off; off += 2 * align256(sizeof(double) * (n2 + 2));
+    const size_t o_rows_c = off; off += 2 * align256(sizeof(int) * (n2m + 2));
+    const size_t o_rows_b = off; off += align256(sizeof(int) * (n2m + 2));
     const size_t o_twx = off; off = align256(off + sizeof(double2) * n1m);
     const size_t o_twz = off; off = align256(off + sizeof(double2) * n3m);
     const size_t o_ccap = off; off = align256(off + sizeof(double2) * nspec);
@@ -225,7 +231,7 @@ extern "C" int lesgpu_poisson_ftft_noalloc(const lesgpu_grid *g, const double *d
     TableDst d;
     d.ak1 = (double *)(base + o_ak1);
     d.ak3 = (double *)(base + o_ak3);
-    d.rows = (double4 *)(base + o_rows);
+    d.rows = lg::YRows{(double2 *)(base + o_rows_a), (double *)(base + o_rows_c), (int *)(base + o_rows_b)};
     d.twx = (double2 *)(base + o_twx);
     d.twz = (double2 *)(base + o_twz);
     lg::chain(k_noalloc_tables, dim3((std::max(n1m, std::max(n2m, n3m)) + 3 + 63) / 64, 5), 64, 0, st)(y, d, n1m, n2m, n3m, g->f2fxi[1], g->f2fzi[1]);
