@@ -927,8 +927,8 @@ __global__ void __launch_bounds__(kMglThreads, 1) k_mgl_modes(const MgLineArgs *
         // sqrt(n) < test as an integer test of n: the least n whose root is
         // not below the criterion
         const double test = a.S->mg_test;
-        double t2 = test > 0.0 ? test * test : 0.0;
-        if (t2 > 0.0 && t2 <= 1.0e300) {
+        double t2 = test > 0.0 ? test * test : 0.0;     // 0 too where the square underflows: a zero residual passes
+        if (test > 0.0 && t2 <= 1.0e300) {
             while (t2 > 0.0 && sqrt(t2) >= test) t2 = __longlong_as_double(__double_as_longlong(t2) - 1);
             while (sqrt(t2) < test) t2 = __longlong_as_double(__double_as_longlong(t2) + 1);
         }
