@@ -1497,6 +1497,10 @@ static bool adi_factored(const lesgpu_case *c, const AdiBatch &B) {
     return !(B.a[0].comp == CT && c->kp.c.iconjg == 1 && c->conj_general);
 }
 
+// the two-ended form: factored coefficients, and no fine span's mixed form
+// (kFineSpan), which keeps the roundings of the other forms
+static bool adi_ends(const lesgpu_case *c, const AdiBatch &B) { return adi_factored(c, B) && !c->fine_span; }
+
 // launch with W = w & 63 lanes per line (w & 64: the register-capped warp-scan
 // kernel; w == kTiled: the tiled FP32 sweep); false if that form cannot take
 // the batch (W cannot hold the line, MC <= 12; the tiled form needs FP32
@@ -1510,7 +1514,7 @@ static bool adi_run(lesgpu_case *c, const AdiBatch &B, const AdiShape &h, int wc
         return adit_launch(c, B, h.ncomp, h.nmax);
     }
     if (wcode == kEnds) {
-        if (h.f32 || !fac) return false;
+        if (h.f32 || !adi_ends(c, B)) return false;
         return ends_launch(c, B, h.ncomp, h.mx, h.nmax);
     }
     const int w = wcode & 63;
@@ -1543,7 +1547,7 @@ static bool adi_run(lesgpu_case *c, const AdiBatch &B, const AdiShape &h, int wc
 }
 
 struct AdiTuneKey {
-    int n1m, n2m, n3m, dir, ncomp, f32, periodic, nmax;
+    int n1m, n2m, n3m, dir, ncomp, f32, periodic, nmax;      // f32: 2 for FP64 sweeps of a mixed case past kFineSpan
     bool operator<(const AdiTuneKey &o) const {
         const int a[8] = {n1m, n2m, n3m, dir, ncomp, f32, periodic, nmax};
         const int b[8] = {o.n1m, o.n2m, o.n3m, o.dir, o.ncomp, o.f32, o.periodic, o.nmax};
@@ -1555,7 +1559,7 @@ static std::mutex g_adi_mu;
 
 static AdiTuneKey adi_key(const lesgpu_case *c, const AdiBatch &B, const AdiShape &h) {
     const DGrid &g = c->kp.g;
-    return AdiTuneKey{g.n1m, g.n2m, g.n3m, B.a[0].dir, h.ncomp, h.f32 ? 1 : 0, B.a[0].periodic, h.nmax};
+    return AdiTuneKey{g.n1m, g.n2m, g.n3m, B.a[0].dir, h.ncomp, h.f32 ? 1 : c->fine_span ? 2 : 0, B.a[0].periodic, h.nmax};
 }
 
 // W used until a shape is tuned: the FP32 form 32 lanes; FP64 the two-ended
@@ -1565,7 +1569,7 @@ static AdiTuneKey adi_key(const lesgpu_case *c, const AdiBatch &B, const AdiShap
 static int adi_default_w(const lesgpu_case *c, const AdiBatch &B, const AdiShape &h) {
     if (h.f32) return 32;
     const long long lines = h.mx * h.ncomp;
-    if (lines >= 3000 && h.nmax <= 128 && adi_factored(c, B) && (!B.a[0].periodic || h.nmax >= 4)) return kEnds;
+    if (lines >= 3000 && h.nmax <= 128 && adi_ends(c, B) && (!B.a[0].periodic || h.nmax >= 4)) return kEnds;
     int w = 1;
     while (w < 32 && lines * w < 65536) w <<= 1;
     return w < 8 ? 1 : w;
@@ -1580,7 +1584,7 @@ static void adi_launch(lesgpu_case *c, const AdiBatch &B, int ncomp) {
         auto it = g_adi_w.find(adi_key(c, B, h));
         // a shape's entry may be of a case without general conjugate tables:
         // its temperature sweeps then keep the untuned form
-        if (it != g_adi_w.end() && (it->second != kEnds || adi_factored(c, B))) w = it->second;
+        if (it != g_adi_w.end() && (it->second != kEnds || adi_ends(c, B))) w = it->second;
     }
     if (h.f32 && c->adi_force_f32) w = c->adi_force_f32;
     inst_begin(c, LESGPU_K_ADI);
@@ -1762,7 +1766,8 @@ int adi_tuned(const lesgpu_case *c, int *out, int maxn) {
     for (const auto &kv : g_adi_w) {
         const AdiTuneKey &k = kv.first;
         if (k.n1m != g.n1m || k.n2m != g.n2m || k.n3m != g.n3m || n + 4 > maxn) continue;
-        out[n++] = k.dir; out[n++] = k.ncomp; out[n++] = k.f32; out[n++] = kv.second;
+        if (k.f32 == (c->fine_span ? 0 : 2)) continue;
+        out[n++] = k.dir; out[n++] = k.ncomp; out[n++] = k.f32 == 1; out[n++] = kv.second;
     }
     return n / 4;
 }

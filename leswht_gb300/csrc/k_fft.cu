@@ -50,8 +50,9 @@ struct FastDiv {
 // One radix-R stage of block_fft on L interleaved lines, R a compile-time
 // constant (the plans hold radices 4, 2, 3 and 5 only), so the butterfly and
 // its loads, twiddles and stores unroll.  Twiddle index jm r twstep < Ns R
-// N / (Ns R) = N: inside the table.
-template <class V, int R>
+// N / (Ns R) = N: inside the table.  PLAIN: radices 3 and 5 by plain sums, whose
+// roundings the mixed form of a fine span keeps (kFineSpan).
+template <class V, int R, bool PLAIN>
 __device__ __forceinline__ void fft_stage(const V *in, V *out, int L, const FastDiv &dL, int N, int Ns,
                                           const V *tw, int inv) {
     const int NR = N / R;
@@ -85,6 +86,18 @@ __device__ __forceinline__ void fft_stage(const V *in, V *out, int L, const Fast
             y[2] = csub(s02, s13);
             y[1] = cadd(d02, jd13);
             y[3] = csub(d02, jd13);
+        } else if constexpr (PLAIN) {
+#pragma unroll
+            for (int m = 0; m < R; m++) {
+                V acc = v[0];
+#pragma unroll
+                for (int r = 1; r < R; r++) {
+                    V t = tw[((m * r) % R) * NR];
+                    if (inv) t.y = -t.y;
+                    acc = cadd(acc, cmul(v[r], t));
+                }
+                y[m] = acc;
+            }
         } else if constexpr (R == 3) {
             // 12 operations instead of the 24 of the plain sums (Winograd,
             // "On computing the discrete Fourier transform", Math. Comp. 32
@@ -119,7 +132,7 @@ __device__ __forceinline__ void fft_stage(const V *in, V *out, int L, const Fast
 }
 
 // Run all stages on L interleaved lines; returns the buffer holding the result.
-template <class V>
+template <class V, bool PLAIN = false>
 __device__ V *block_fft(V *b0, V *b1, int L, const DevPlan &P, int inv) {
     const int N = P.n;
     const V *tw = twid<V>(P);
@@ -130,10 +143,10 @@ __device__ V *block_fft(V *b0, V *b1, int L, const DevPlan &P, int inv) {
         const int code = (int)(P.radc >> (2 * st)) & 3;
         const int R = code == 0 ? 4 : code == 1 ? 2 : code == 2 ? 3 : 5;
         switch (R) {
-        case 4: fft_stage<V, 4>(in, out, L, dL, N, Ns, tw, inv); break;
-        case 2: fft_stage<V, 2>(in, out, L, dL, N, Ns, tw, inv); break;
-        case 3: fft_stage<V, 3>(in, out, L, dL, N, Ns, tw, inv); break;
-        default: fft_stage<V, 5>(in, out, L, dL, N, Ns, tw, inv); break;
+        case 4: fft_stage<V, 4, PLAIN>(in, out, L, dL, N, Ns, tw, inv); break;
+        case 2: fft_stage<V, 2, PLAIN>(in, out, L, dL, N, Ns, tw, inv); break;
+        case 3: fft_stage<V, 3, PLAIN>(in, out, L, dL, N, Ns, tw, inv); break;
+        default: fft_stage<V, 5, PLAIN>(in, out, L, dL, N, Ns, tw, inv); break;
         }
         __syncthreads();
         V *tmp = in; in = out; out = tmp;
@@ -168,7 +181,7 @@ DevPlan devplan(const FftPlan &p) {
 // conjugate-symmetric spectra and takes x = Re, y = Im.  Half the transforms
 // of the real z lines, each exact up to rounding (on GB300 the FP64 pipe, not
 // memory, bounds these passes).  Line pair l holds i = i0 + 2l and i0 + 2l + 1.
-template <class V>
+template <class V, bool PLAIN = false>
 __global__ void k_fft_z_fwd(KP p, const double *src, V *ccap, DevPlan P, int L, long long sk, long long sj) {
     chained();
     using T = decltype(V{}.x);
@@ -187,7 +200,7 @@ __global__ void k_fft_z_fwd(KP p, const double *src, V *ccap, DevPlan P, int L, 
         slot[l2 & 1] = val;
     }
     __syncthreads();
-    const V *res = block_fft(b0, b1, L, P, 0);
+    const V *res = block_fft<V, PLAIN>(b0, b1, L, P, 0);
     const int n3mh = g.n3mh;
     for (int w = threadIdx.x; w < n3mh * 2 * L; w += blockDim.x) {
         const int kk = d2L.div(w), l2 = w - kk * 2 * L;
@@ -202,7 +215,7 @@ __global__ void k_fft_z_fwd(KP p, const double *src, V *ccap, DevPlan P, int L, 
 }
 
 // ADD: phi += the result (the correction pass of the mixed form), else phi =
-template <class V, bool ADD>
+template <class V, bool ADD, bool PLAIN = false>
 __global__ void k_fft_z_inv(KP p, const V *ccap, DevPlan P, int L, long long sk, long long sj) {
     chained();
     using T = decltype(V{}.x);
@@ -233,7 +246,7 @@ __global__ void k_fft_z_inv(KP p, const V *ccap, DevPlan P, int L, long long sk,
         b0[e * L + l] = V{x.x - y.y, x.y + y.x};     // Z = X + i Y
     }
     __syncthreads();
-    const V *res = block_fft(b0, b1, L, P, 1);
+    const V *res = block_fft<V, PLAIN>(b0, b1, L, P, 1);
     const double dn = 1.0 / (double)N;
     for (int w = threadIdx.x; w < N * 2 * L; w += blockDim.x) {
         const int e = d2L.div(w), l2 = w - e * 2 * L;
@@ -941,12 +954,12 @@ void launch_poisson(lesgpu_case *c, int msub) {
 
 // FP64 launches for the other translation units
 void fft_z_fwd64(dim3 grid, size_t smem, cudaStream_t st, KP p, const double *src, double2 *ccap, DevPlan P, int L,
-                 long long sk, long long sj) {
-    chain(k_fft_z_fwd<double2>, grid, kThreads, smem, st)(p, src, ccap, P, L, sk, sj);
+                 long long sk, long long sj, int plain) {
+    chain(plain ? k_fft_z_fwd<double2, true> : k_fft_z_fwd<double2>, grid, kThreads, smem, st)(p, src, ccap, P, L, sk, sj);
 }
 void fft_z_inv64(dim3 grid, size_t smem, cudaStream_t st, KP p, const double2 *ccap, DevPlan P, int L, long long sk,
-                 long long sj) {
-    chain(k_fft_z_inv<double2, false>, grid, kThreads, smem, st)(p, ccap, P, L, sk, sj);
+                 long long sj, int plain) {
+    chain(plain ? k_fft_z_inv<double2, false, true> : k_fft_z_inv<double2, false>, grid, kThreads, smem, st)(p, ccap, P, L, sk, sj);
 }
 void fft_x64(int nblocks, size_t smem, cudaStream_t st, double2 *ccap, int nlines, DevPlan P, int L, int inv) {
     chain(k_fft_x<double2>, nblocks, kThreads, smem, st)(ccap, nlines, P, L, inv);
@@ -954,6 +967,8 @@ void fft_x64(int nblocks, size_t smem, cudaStream_t st, double2 *ccap, int nline
 int fft_smem64(int bytes) {
     return (cudaFuncSetAttribute(k_fft_z_fwd<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
             cudaFuncSetAttribute(k_fft_z_inv<double2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
+            cudaFuncSetAttribute(k_fft_z_fwd<double2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
+            cudaFuncSetAttribute(k_fft_z_inv<double2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
             cudaFuncSetAttribute(k_fft_x<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
                ? 0 : LESGPU_ERR_CUDA;
 }

@@ -24,11 +24,12 @@ constexpr int kFftSmemMax = 200 * 1024;
 
 // z transforms; the spectrum element (i, k, j) sits at (i-1) + sk*(k-1) + sj*(j-1)
 // FP64 launches of the transforms (kernel templates of k_fft.cu, which other
-// translation units cannot launch directly): src is the real field transformed
+// translation units cannot launch directly): src is the real field transformed;
+// plain: radices 3 and 5 by plain sums (kFineSpan)
 void fft_z_fwd64(dim3 grid, size_t smem, cudaStream_t st, KP p, const double *src, double2 *ccap, DevPlan P, int L,
-                 long long sk, long long sj);
+                 long long sk, long long sj, int plain = 0);
 void fft_z_inv64(dim3 grid, size_t smem, cudaStream_t st, KP p, const double2 *ccap, DevPlan P, int L, long long sk,
-                 long long sj);
+                 long long sj, int plain = 0);
 void fft_x64(int nblocks, size_t smem, cudaStream_t st, double2 *ccap, int nlines, DevPlan P, int L, int inv);
 // opt the FP64 transform kernels into `bytes` of dynamic shared memory
 int fft_smem64(int bytes);

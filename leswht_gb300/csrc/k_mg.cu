@@ -1637,16 +1637,6 @@ static int mgl_init(lesgpu_case *c) {
     return mgl_set_cluster(c, pick);
 }
 
-// Cells a unit length in z from which the mixed form keeps the cycle in global
-// memory.  The two cycles round their FP32 corrections differently, which
-// leaves p 1e-10 apart; the momentum kernel differences p in FP32, and where
-// that turns one rounding of p, w jumps by ulp(p) dt / dz.  Beside a body set
-// off from rest p is 100 to 200: at 64 cells over pi (dz = 1/20) a jump is up
-// to 1.2e-3 of w's rms, past the 8e-4 its results are held to, at 48 cells
-// (1/15) 5e-4, at 16 cells 3e-4.  A 256x192x64 solve takes 10.0 ms so and
-// 2.3 ms resident.
-constexpr double kMgFineSpan = 16.0;
-
 int mg2d_init(lesgpu_case *c) {
     const DGrid &g = c->kp.g;
     const lesgpu_config &cf = c->cfg;
@@ -1676,8 +1666,7 @@ int mg2d_init(lesgpu_case *c) {
     {   // resident cycles wherever some cluster holds a mode (and no mode runs SOR)
         MgLineArgs a;
         size_t sm;
-        const bool fine = T->mixed && !xft && c->h_grid->f2fzi[1] > kMgFineSpan;
-        const bool ok = !fine && nmodes <= cf.imgsor && 4 * nlev + 2 * cf.nbli + 8 <= kMglMaxPhase;
+        const bool ok = !(T->mixed && c->fine_span) && nmodes <= cf.imgsor && 4 * nlev + 2 * cf.nbli + 8 <= kMglMaxPhase;
         bool fits = false;
         for (int cs = 1; cs <= 16 && ok; cs <<= 1) fits = fits || mgl_plan(*T, g.n2m, cs, a, sm);
         // and the device takes one of them: 16 blocks, or a block of all the
@@ -1852,7 +1841,7 @@ static void mg2d_pre(lesgpu_case *c, int slot) {
         const size_t smz = (size_t)2 * (g.n3m > 1 ? g.n3m : 1) * Lz * sizeof(double2);
         const dim3 gz((g.n1m + 2 * Lz - 1) / (2 * Lz), g.n2m);   // 2 Lz real lines per block
         const long long sk = (long long)g.n1m * g.n2m, sj = g.n1m;
-        fft_z_fwd64(gz, smz, c->stream, c->kp, c->kp.f.divgsum, P.ccap, pz, Lz, sk, sj);
+        fft_z_fwd64(gz, smz, c->stream, c->kp, c->kp.f.divgsum, P.ccap, pz, Lz, sk, sj, c->fine_span);
     }
 }
 
@@ -1871,7 +1860,7 @@ static void mg2d_post(lesgpu_case *c) {
         const size_t smz = (size_t)2 * (g.n3m > 1 ? g.n3m : 1) * Lz * sizeof(double2);
         const dim3 gz((g.n1m + 2 * Lz - 1) / (2 * Lz), g.n2m);
         const long long sk = (long long)g.n1m * g.n2m, sj = g.n1m;
-        fft_z_inv64(gz, smz, c->stream, c->kp, P.ccap, pz, Lz, sk, sj);
+        fft_z_inv64(gz, smz, c->stream, c->kp, P.ccap, pz, Lz, sk, sj, c->fine_span);
     }
 }
 

@@ -574,6 +574,7 @@ extern "C" int lesgpu_create(const lesgpu_config *cfg, const lesgpu_grid *g, les
     // only by this wait
     if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) { lesgpu_destroy(c); return LESGPU_ERR_CUDA; }
     launch_red_weights(c);
+    c->fine_span = cfg->precision == LESGPU_PREC_MIXED && cfg->poisson == LESGPU_POISSON_Z_FT && g->f2fzi[1] > kFineSpan;
     c->h_grid = g;
     rc = poisson_init(c);
     c->h_grid = nullptr;

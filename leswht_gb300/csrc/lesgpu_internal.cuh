@@ -417,6 +417,20 @@ __device__ __forceinline__ void block_totals(double (&v)[NV]) {
     for (int q = 0; q < NV; q++) v[q] = tot[q];
 }
 
+// Cells a unit length in z from which a mixed case under poiss_z_ft keeps the
+// roundings on the way to p: the multigrid cycle in global memory, the plain
+// radix-3 and radix-5 sums of its transforms, no two-ended sweeps.  The
+// momentum kernel differences an FP32 copy of p, which beside a body set off
+// from rest is 100 to 200; any change of a last bit before the multigrid's FP32
+// corrections leaves p 1e-10 apart, and where that turns one rounding of p, w
+// jumps by ulp(p) dt / dz.  With those three changed, w moved by more than
+// 2e-5 (rel-L2) or 8e-4 of its rms at a point in none of 87 cylinders and
+// squares of up to 18 cells over pi, in 3 of 76 of 19 to 32 cells (1/10), and
+// in 8 of 49 of 36 cells (1/11.5) and more.  The autotuner's choice among the
+// other sweeps alone does it in 0, 4 and 1 of them.  A 256x192x64 solve takes
+// 10.0 ms in global memory and 2.3 ms resident.
+constexpr double kFineSpan = 11.0;
+
 }  // namespace lg
 
 // --------------------------------------------------------------- the case
@@ -442,6 +456,7 @@ struct lesgpu_case {
     // per line, + 64 register-capped, 128 tiled; 0 = the autotuner's)
     int adi_force_f32;
     long long adi_other;        // sweeps enqueued in another form than the one chosen
+    int fine_span;              // a mixed case past kFineSpan
     // FP32 mirror sets (kMir*) whose FP64 arrays changed since their last
     // refresh, as the enqueued work stands (host-side bookkeeping of the
     // mixed form; launch_mirror converts only these)

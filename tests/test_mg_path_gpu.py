@@ -3,7 +3,7 @@ after a fixed number of cycles.
 
 A mode's lines live in its cluster's shared memory wherever a cluster of at
 most 16 blocks holds them; FITS gives the smallest that does, FP64 and mixed.
-Modes that none holds, SOR modes and mixed spans finer than 1/16 run the cycle
+Modes that none holds, SOR modes and mixed spans finer than 1/11 run the cycle
 in global memory.  Every mode takes CYCLES of them, the criterion being out of
 reach, on the GPU and in the oracle, so the iterates are those of the same
 cycle also in the mixed form, which at a criterion may stop one sooner or
@@ -76,10 +76,10 @@ def test_global_memory(oracle_lib, n, nbli):
 
 def test_global_memory_fine_span(oracle_lib):
     """dz = 1/20 in the mixed form; the FP64 form of the case, and the mixed
-    form at dz = 1/15, stay in the clusters."""
+    form at dz = 1/10, stay in the clusters."""
     c = fixed(cases.cylinder(32, 24, 64, precision=abi.PREC_MIXED))
     s = leswht_gb300.gpu_solver(c)
     assert path(s)[0] == 0
     check_phi(oracle_lib, c, 1e-5, s)
     assert path(leswht_gb300.gpu_solver(cases.cylinder(32, 24, 64)))[0] == 1
-    assert path(leswht_gb300.gpu_solver(cases.cylinder(32, 24, 48, precision=abi.PREC_MIXED)))[0] == 1
+    assert path(leswht_gb300.gpu_solver(cases.cylinder(32, 24, 32, precision=abi.PREC_MIXED)))[0] == 1
