@@ -212,10 +212,11 @@ struct FiltBatch {
 // 6 and 4).  The arrays share the addresses and weights, which in FP32 are
 // most of the instructions.  The mean of a step's four
 // launches, us: 64^3 FP64 63 -> 43, FP32 12.9 -> 9.5; 384x256x384 FP32
-// 1479 -> 860.
+// 1479 -> 887.
 // The fused sums' order is what the compiler makes of c0 l + c1 m + c2 r, so
 // the mixed form's coefficient keeps its bits (another order moves it by up to 5e-5,
-// and every eddy viscosity with it).
+// and every eddy viscosity with it); with the loads of the three arrays written
+// ahead of them, as in xvals, 384x256x384 FP32 takes 887 us, not 987.
 constexpr int kFiltA = 3;
 
 template <class R>
@@ -246,17 +247,25 @@ __global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F, i
         const bool filt = op != 0;
         const R *cfx = mir<R>(p).cfx1 + 3 * i;
         const R c0 = cfx[0], c1 = cfx[1], c2 = cfx[2];
-        auto xval = [&](const R *__restrict__ r) {
-            const R x = r[0], y = fma(c2, r[op], fma(c0, r[om], c1 * x));
-            return filt ? y : x;
+        // the x-filtered values of all arrays at offset q, their loads ahead of the sums
+        auto xvals = [&](long long q, R (&out)[kFiltA]) {
+            R l[kFiltA], x[kFiltA], r[kFiltA];
+#pragma unroll
+            for (int a = 0; a < kFiltA; a++) {
+                l[a] = s[a][q + om];
+                x[a] = s[a][q];
+                r[a] = s[a][q + op];
+            }
+#pragma unroll
+            for (int a = 0; a < kFiltA; a++) {
+                const R y = fma(c2, r[a], fma(c0, l[a], c1 * x[a]));
+                out[a] = filt ? y : x[a];
+            }
         };
         R xm[kFiltA], x0[kFiltA];
         const long long qa = g.ix(i, j, ka), qm = g.ix(i, j, ka == 1 ? g.n3m : ka - 1);
-#pragma unroll
-        for (int a = 0; a < kFiltA; a++) {
-            x0[a] = xval(s[a] + qa);
-            xm[a] = xval(s[a] + qm);
-        }
+        xvals(qa, x0);
+        xvals(qm, xm);
         const R *cfz = mir<R>(p).cfz1 + 3 * ka;
         long long q = qa;
         for (int k = ka; k <= kb; k++, q += g.sxy, cfz += 3) {
@@ -267,8 +276,7 @@ __global__ void __launch_bounds__(kThreads) k_filter(KP p, Box b, FiltBatch F, i
             const bool zin = zf && ((k >= 2 && k <= g.n3m - 1) || p.c.zprdic == 1);
             const R z0 = cfz[0], z1 = cfz[1], z2 = cfz[2];
             R xp[kFiltA];
-#pragma unroll
-            for (int a = 0; a < kFiltA; a++) xp[a] = xval(s[a] + qp);
+            xvals(qp, xp);
 #pragma unroll
             for (int a = 0; a < kFiltA; a++) {
                 const R y = fma(z2, xp[a], fma(z0, xm[a], z1 * x0[a]));
