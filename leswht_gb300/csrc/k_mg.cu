@@ -87,7 +87,7 @@ struct MgTables {
     long long *iters;           // per mode, last solve
     long long pc_plane, gg_plane;
     // the cycles with the modes resident in their clusters' shared memory
-    // (k_mgl.cuh), used wherever a mode fits
+    // (k_mgl.cuh), used wherever a mode fits, up to kFineSpan in the mixed form
     int resident, prd;
     MgLineArgs *dargs;          // device copies: one per substep, one for the autotuner's timing
     double *ltab_d, *llc_d, *lact, *lasl, *lanl;
@@ -1663,7 +1663,8 @@ int mg2d_init(lesgpu_case *c) {
     const char *mg64 = getenv("LESGPU_MG_FP64");
     T->mixed = cf.precision == LESGPU_PREC_MIXED && !(mg64 && mg64[0] == '1');
     T->prd = (xft ? cf.zprdic : cf.xprdic) == 1;
-    {   // resident cycles wherever some cluster holds a mode (and no mode runs SOR)
+    {   // resident cycles wherever some cluster holds a mode (and no mode runs SOR,
+        // nor the mixed form a span past kFineSpan)
         MgLineArgs a;
         size_t sm;
         const bool ok = !(T->mixed && c->fine_span) && nmodes <= cf.imgsor && 4 * nlev + 2 * cf.nbli + 8 <= kMglMaxPhase;

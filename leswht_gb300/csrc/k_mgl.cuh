@@ -177,15 +177,6 @@ struct MglCtx {
     MglPhase ph[kMglMaxPhase];
 };
 
-// line l (0-based) of a level in the store `area`
-template <int R, class T>
-__device__ __forceinline__ T *mgl_line(const MglCtx &c, T *area, const MgLevel &L, int l) {
-    const int q = l >> 1;
-    const int own = L.inv ? (int)__umulhi((unsigned)q, L.inv) : q;
-    const int home = L.solo ? 0 : own;
-    T *p = area + (L.off + (q - own * L.pp) * 2 + (l & 1)) * (R * 32);
-    return home == c.rank ? p : cooperative_groups::this_cluster().map_shared_rank(p, home);
-}
 // neighbours of line l, -1 outside the level
 __device__ __forceinline__ int mgl_im(const MglCtx &c, const MgLevel &L, int l) { return l > 0 ? l - 1 : c.a.prd ? L.n - 1 : -1; }
 __device__ __forceinline__ int mgl_ip(const MglCtx &c, const MgLevel &L, int l) { return l + 1 < L.n ? l + 1 : c.a.prd ? 0 : -1; }

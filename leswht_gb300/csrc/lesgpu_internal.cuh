@@ -313,9 +313,9 @@ struct Box {
 // may be launched while the one before it completes, and starts its work,
 // after chained(), once that one's writes are visible -- part of its launch is
 // off the path.  Every kernel launched this way calls chained() first; one
-// that did not would wait for nothing.  Ten 64^3 mixed steps of some 110
+// that did not would wait for nothing.  Ten 64^3 mixed steps of some 125
 // kernels each: 11.59 ms with plain launches, 11.22 so; a 30x33x24 solve of
-// five kernels 73 us, 64.  Letting the next kernel in earlier
+// six kernels 73 us, 64.  Letting the next kernel in earlier
 // (griddepcontrol.launch_dependents, before or after the wait) puts its
 // waiting blocks where SMs happen to be free first: 14.26 and 13.37 ms.
 template <class... P>
